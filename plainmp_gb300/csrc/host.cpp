@@ -518,7 +518,7 @@ static void check_rotation(const double* rot) {
 // Device image of one SDF tree (for SDF-level evaluate / is_outside calls).
 struct SdfDeviceImage {
   DevBuf prims, clouds;
-  int n_prims = 0;
+  int n_prims = 0, n_clouds = 0;
   int device = -1;
   std::vector<std::pair<const HostSdf*, uint64_t>> sig;
 };
@@ -988,7 +988,7 @@ void check_arr(const void* p, int64_t n, const char* what) {
 }
 
 // Device image of an SDF tree for SDF-level calls
-const PmPrim* sdf_image(pmgpu_sdf* h, int* n_prims, const PmGridDev** clouds) {
+const PmPrim* sdf_image(pmgpu_sdf* h, int* n_prims, const PmGridDev** clouds, int* n_clouds) {
   std::vector<std::shared_ptr<HostSdf>> f;
   flatten(h->s, f);
   std::vector<std::pair<const HostSdf*, uint64_t>> sig;
@@ -1015,9 +1015,11 @@ const PmPrim* sdf_image(pmgpu_sdf* h, int* n_prims, const PmGridDev** clouds) {
     h->img.clouds.ensure(std::max<size_t>(cl.size(), 1) * sizeof(PmGridDev));
     if (!cl.empty()) cuda_check(cudaMemcpy(h->img.clouds.p, cl.data(), cl.size() * sizeof(PmGridDev), cudaMemcpyHostToDevice), "sdf upload");
     h->img.n_prims = (int)prims.size();
+    h->img.n_clouds = (int)cl.size();
     h->img.sig = sig;
   }
   *n_prims = h->img.n_prims;
+  *n_clouds = h->img.n_clouds;
   *clouds = h->img.clouds.as<PmGridDev>();
   return h->img.prims.as<PmPrim>();
 }
@@ -1470,18 +1472,18 @@ int pmgpu_sdf_evaluate(pmgpu_sdf* s, const double* points, int64_t n, double* ou
     if (n < 0) throw std::invalid_argument("negative count");
     check_arr(points, n, "points");
     check_arr(out, n, "out");
-    int np;
+    int np, ncl;
     const PmGridDev* cl;
-    const PmPrim* pr = sdf_image(s, &np, &cl);
+    const PmPrim* pr = sdf_image(s, &np, &cl, &ncl);
     cudaStream_t st = as_stream(stream);
     if (mem == PMGPU_MEM_DEVICE) {
-      cuda_check(launch_sdf_points(pr, np, cl, s->s->kind == PM_SDF_UNION, points, nullptr, n, out, nullptr, st), "sdf evaluate");
+      cuda_check(launch_sdf_points(pr, np, cl, ncl, s->s->kind == PM_SDF_UNION, points, nullptr, n, out, nullptr, st), "sdf evaluate");
       return;
     }
     DevBuf a, b;
     const double* dp = stage_in(a, points, (size_t)n * 3, st);
     double* dout = (double*)b.ensure(std::max<size_t>((size_t)n * 8, 16));
-    cuda_check(launch_sdf_points(pr, np, cl, s->s->kind == PM_SDF_UNION, dp, nullptr, n, dout, nullptr, st), "sdf evaluate");
+    cuda_check(launch_sdf_points(pr, np, cl, ncl, s->s->kind == PM_SDF_UNION, dp, nullptr, n, dout, nullptr, st), "sdf evaluate");
     stage_out(out, dout, (size_t)n, st);
     cuda_check(cudaStreamSynchronize(st), "sdf evaluate");
   });
@@ -1494,19 +1496,19 @@ int pmgpu_sdf_is_outside(pmgpu_sdf* s, const double* points, const double* radii
     check_arr(points, n, "points");
     check_arr(radii, n, "radii");
     check_arr(out, n, "out");
-    int np;
+    int np, ncl;
     const PmGridDev* cl;
-    const PmPrim* pr = sdf_image(s, &np, &cl);
+    const PmPrim* pr = sdf_image(s, &np, &cl, &ncl);
     cudaStream_t st = as_stream(stream);
     if (mem == PMGPU_MEM_DEVICE) {
-      cuda_check(launch_sdf_points(pr, np, cl, 1, points, radii, n, nullptr, out, st), "sdf is_outside");
+      cuda_check(launch_sdf_points(pr, np, cl, ncl, 1, points, radii, n, nullptr, out, st), "sdf is_outside");
       return;
     }
     DevBuf a, b, c;
     const double* dp = stage_in(a, points, (size_t)n * 3, st);
     const double* dr = stage_in(b, radii, (size_t)n, st);
     uint8_t* dout = (uint8_t*)c.ensure(std::max<size_t>((size_t)n, 16));
-    cuda_check(launch_sdf_points(pr, np, cl, 1, dp, dr, n, nullptr, dout, st), "sdf is_outside");
+    cuda_check(launch_sdf_points(pr, np, cl, ncl, 1, dp, dr, n, nullptr, dout, st), "sdf is_outside");
     stage_out(out, dout, (size_t)n, st);
     cuda_check(cudaStreamSynchronize(st), "sdf is_outside");
   });
@@ -1518,9 +1520,9 @@ int pmgpu_cloud_nearest(pmgpu_sdf* cloud, const double* points, int64_t n, doubl
     if (cloud->s->kind != PM_SDF_CLOUD) throw std::invalid_argument("not a CloudSDF");
     if (n < 0) throw std::invalid_argument("negative count");
     check_arr(points, n, "points");
-    int np;
+    int np, ncl;
     const PmGridDev* cl;
-    sdf_image(cloud, &np, &cl);
+    sdf_image(cloud, &np, &cl, &ncl);
     cudaStream_t st = as_stream(stream);
     if (mem == PMGPU_MEM_DEVICE) {
       cuda_check(launch_cloud_nearest(cl, points, n, sqdist, nearest3, st), "cloud nearest");

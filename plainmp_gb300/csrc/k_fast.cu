@@ -29,6 +29,7 @@
 #include "pm_grad.cuh"
 #include "pm_launch.h"
 #include "pm_view.cuh"
+#include "pm_warp.cuh"
 
 using namespace pmd;
 
@@ -318,10 +319,6 @@ __device__ __forceinline__ void clearance(const PrimF& P, const PmGridDev* cloud
   }
   g = 3.0e38f;
   sd = 3.0e38f;
-}
-
-__device__ __forceinline__ unsigned long long nn_key(float d2, int idx) {
-  return ((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)idx;
 }
 
 // Block offsets (dx, dy, dz) with max |d| <= kOffR, sorted by the minimum distance between two
@@ -678,224 +675,6 @@ __device__ inline NNResult32 warp_nearest32(const PmGridDev& G, float qx, float 
   r.d2 = best;
   r.idx = bidx;
   return r;
-}
-
-// Warp-cooperative exact FP64 nearest neighbour below maxd2: the minimum over points of
-// fl(dx*dx + (dy*dy + dz*dz)) in FP64, as grid_nearest64.  The cube of blocks around q within
-// sqrt(maxd2), one block of slack per side, is split across lanes; a candidate block's occupied
-// cells are split across lanes and the warp minimum is shared after every block.
-// The pruning runs in FP32 and only the points it cannot rule out reach FP64 (the FP64 pipe
-// takes a whole warp instruction per operation, however few lanes are active): a block, cell or
-// point is skipped when its FP32 distance from q exceeds the current best by more than the FP32
-// error of both (t = 4e-7 (|q|_1 + |p|_1 max) + 4e-6 d, far above the rounding of the points,
-// of q and of the distance arithmetic), so no point below the best is ever skipped.  hint: a
-// point index whose distance starts the search (e.g. the FP32 nearest point), or -1.
-__device__ inline NNResult64 warp_nearest64(const PmGridDev& G, const D3& q, double maxd2, int hint = -1) {
-  const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  NNResult64 r{maxd2, -1};
-  if (G.n_points <= 0 || !(maxd2 > 0.0)) return r;
-  double best = maxd2;
-  int bidx = -1;
-  if (hint >= 0 && hint < G.n_points) {
-    const D3 d{G.px[hint] - q.x, G.py[hint] - q.y, G.pz[hint] - q.z};
-    const double d2 = d.x * d.x + (d.y * d.y + d.z * d.z);
-    if (d2 < best) {
-      best = d2;
-      bidx = hint;
-    }
-  }
-  const float qx = (float)q.x, qy = (float)q.y, qz = (float)q.z;
-  float pmax = 0.f;
-  for (int a = 0; a < 3; a++) pmax += fmaxf(fabsf(G.box_lo32[a]), fabsf(G.box_hi32[a]));
-  const float tabs = 4e-7f * (fabsf(qx) + fabsf(qy) + fabsf(qz) + pmax) + 1e-12f;
-  // FP32 threshold on squared distances: anything above it is farther than the best
-  auto thr = [&](double b) {
-    const float sb = sqrtf((float)b) * (1.0f + 4e-6f) + tabs;
-    return sb * sb * (1.0f + 1e-6f);
-  };
-  float t32 = thr(best);
-  // warp minimum of (best, bidx); best >= 0, so its bits order like its value
-  auto warp_min = [&]() {
-    long long bb = __double_as_longlong(best);
-    for (int o = 16; o > 0; o >>= 1) {
-      const long long ob = __shfl_xor_sync(FULL, bb, o);
-      const int oi = __shfl_xor_sync(FULL, bidx, o);
-      if (ob < bb || (ob == bb && oi >= 0 && (bidx < 0 || oi < bidx))) {
-        bb = ob;
-        bidx = oi;
-      }
-    }
-    best = __longlong_as_double(bb);
-    t32 = thr(best);
-  };
-  // Where q's fine cell has a cell list (every occupied cell that can hold q's nearest point, nearest
-  // first), the warp scans it 32 entries at a time: an entry whose stored lower bound reaches the
-  // FP32 threshold ends the scan, the others are tested by their box, and the points of each
-  // surviving cell are split over the lanes (FP32 prefilter, then the exact FP64 distance).
-  int2 rng;
-  if (cell_list_of(G, qx, qy, qz, rng)) {  // the same on every lane
-    const float unit = G.cell32 * (1.0f / (float)PM_CL_UNITS);
-    for (int base = rng.x; base < rng.y; base += 32) {  // warp-uniform
-      const int k = base + lane;
-      bool beyond = true;  // this entry, and (sorted) every later one, lies beyond the best
-      int2 pr = make_int2(0, 0);
-      if (k < rng.y) {
-        const uint32_t e = __ldg(G.cl_ent + k);
-        const float lbd = (float)(e >> 24) * unit;
-        beyond = lbd * lbd * (1.0f - 1e-5f) >= t32;
-        if (!beyond) {
-          const int o = (int)(e & 0xffffffu);
-          const float4 lo = __ldg(G.cell_rec + 2 * o), hi = __ldg(G.cell_rec + 2 * o + 1);
-          const float gx = gap32(qx, lo.x, hi.x), gy = gap32(qy, lo.y, hi.y), gz = gap32(qz, lo.z, hi.z);
-          if (!(fmaf(gx, gx, fmaf(gy, gy, gz * gz)) > t32)) pr = make_int2(__float_as_int(lo.w), __float_as_int(hi.w));
-        }
-      }
-      const bool stop = __shfl_sync(FULL, beyond ? 1 : 0, 31) != 0;
-      for (unsigned bal = __ballot_sync(FULL, pr.y > pr.x); bal != 0; bal &= bal - 1) {  // warp-uniform
-        const int src = __ffs(bal) - 1;
-        const int p0 = __shfl_sync(FULL, pr.x, src), p1 = __shfl_sync(FULL, pr.y, src);
-        for (int pi = p0 + lane; pi < p1; pi += 32) {
-          const float4 pt = __ldg(G.p32 + pi);
-          const float ex = pt.x - qx, ey = pt.y - qy, ez = pt.z - qz;
-          if (fmaf(ex, ex, fmaf(ey, ey, ez * ez)) > t32) continue;
-          const D3 d{G.px[pi] - q.x, G.py[pi] - q.y, G.pz[pi] - q.z};
-          const double d2 = d.x * d.x + (d.y * d.y + d.z * d.z);
-          if (d2 < best || (d2 == best && bidx >= 0 && pi < bidx)) {
-            best = d2;
-            bidx = pi;
-          }
-        }
-      }
-      warp_min();
-      if (stop) break;
-    }
-    r.d2 = best;
-    r.idx = bidx;
-    return r;
-  }
-  const float reach = sqrtf((float)maxd2) * (1.0f + 1e-6f);
-  const float qa[3] = {qx, qy, qz};
-  const int nb[3] = {G.nbx, G.nby, G.nbz};
-  int lo[3], hi[3];
-  for (int a = 0; a < 3; a++) {
-    const float f0 = floorf((qa[a] - reach - G.o32[a]) * G.inv_blk32) - 1.0f;
-    const float f1 = floorf((qa[a] + reach - G.o32[a]) * G.inv_blk32) + 1.0f;
-    if (!(f1 >= 0.f) || !(f0 <= (float)(nb[a] - 1))) {  // also rejects NaN
-      r.d2 = best;
-      r.idx = bidx;
-      return r;
-    }
-    lo[a] = f0 < 0.f ? 0 : (int)f0;
-    hi[a] = f1 > (float)(nb[a] - 1) ? nb[a] - 1 : (int)f1;
-  }
-  const int nx = hi[0] - lo[0] + 1, ny = hi[1] - lo[1] + 1, nz = hi[2] - lo[2] + 1;
-  const int nblk = nx * ny * nz;
-  for (int base = 0; base < nblk; base += 32) {
-    const int i = base + lane;
-    bool cand = false;
-    int2 occ = make_int2(0, 0);
-    if (i < nblk) {
-      const int bx = lo[0] + i % nx;
-      const int t = i / nx;
-      const int by = lo[1] + t % ny, bz = lo[2] + t / ny;
-      const int b = bx + nb[0] * (by + nb[1] * bz);
-      occ = __ldg(reinterpret_cast<const int2*>(G.blk_occ) + b);
-      cand = occ.x < occ.y && !(box_d2_32(G.blk_box + 6 * b, qx, qy, qz) > t32);
-    }
-    unsigned bal = __ballot_sync(FULL, cand);
-    while (bal) {
-      const int src = __ffs(bal) - 1;
-      bal &= bal - 1;
-      const int c0 = __shfl_sync(FULL, occ.x, src), c1 = __shfl_sync(FULL, occ.y, src);
-      for (int c = c0 + lane; c < c1; c += 32) {
-        if (box_d2_32(G.cell_box + 6 * c, qx, qy, qz) > t32) continue;
-        const int2 pr = __ldg(reinterpret_cast<const int2*>(G.cell_pts) + c);
-        for (int p = pr.x; p < pr.y; p++) {
-          const float4 pt = __ldg(G.p32 + p);
-          const float ex = pt.x - qx, ey = pt.y - qy, ez = pt.z - qz;
-          if (fmaf(ex, ex, fmaf(ey, ey, ez * ez)) > t32) continue;
-          const D3 d{G.px[p] - q.x, G.py[p] - q.y, G.pz[p] - q.z};
-          const double d2 = d.x * d.x + (d.y * d.y + d.z * d.z);
-          if (d2 < best || (d2 == best && bidx >= 0 && p < bidx)) {
-            best = d2;
-            bidx = p;
-            t32 = thr(best);
-          }
-        }
-      }
-      warp_min();
-    }
-  }
-  r.d2 = best;
-  r.idx = bidx;
-  return r;
-}
-
-// is_outside(p, r) of a point cloud (primitive_sdf.hpp:597-603) with the warp search: only
-// whether a point lies within r + radius matters (see prim_outside).  Warp-uniform arguments.
-__device__ __forceinline__ bool cloud_outside_warp(const PmPrim& P, const PmGridDev* clouds, const D3& p, double r, int* near,
-                                                   int hint = -1) {
-  const double reach = (r + P.a) * (1.0 + 1e-12) + 1e-12;
-  const NNResult64 nn = warp_nearest64(clouds[P.cloud], p, reach * reach, hint);
-  if (near) *near = nn.idx;
-  if (nn.idx < 0) return true;
-  return sqrt(nn.d2) - P.a > r;
-}
-
-// Starting candidate of a warp search, in two steps so that the loads can be issued early: the field
-// record (nearest point and index) of one of the 8 fine-cell centres around q on lanes 0-7 (index -1
-// elsewhere and outside the grid), and q's own cell-list range on lane 8 (int bits in x, y; -1 none);
-// then the best of the 8 shared by the warp ((INFINITY, -1) if none) and the list range.
-// sub: the lane's position in its query's group of lanes (the lane itself for a whole warp; 0-15 for
-// a half warp).
-__device__ __forceinline__ float4 field_corner_record(const PmGridDev& G, float qx, float qy, float qz, int sub) {
-  const int lane = sub;
-  float4 rec = make_float4(__int_as_float(-1), __int_as_float(-1), 0.f, __int_as_float(-1));
-  if (lane < 8 && G.n_points > 0) {
-    const float inv = G.inv_cell32;
-    const float qa[3] = {qx, qy, qz};
-    const int nc[3] = {G.nbx * PM_GRID_B, G.nby * PM_GRID_B, G.nbz * PM_GRID_B};
-    int cc[3];
-    bool ok = true;
-    for (int a = 0; a < 3; a++) {
-      const float t = floorf((qa[a] - G.o32[a]) * inv - 0.5f) + (float)((lane >> a) & 1);
-      ok = ok && t >= 0.f && t <= (float)(nc[a] - 1);
-      cc[a] = ok ? (int)t : 0;
-    }
-    if (ok) rec = __ldg(G.cell_np + cc[0] + nc[0] * (cc[1] + (int64_t)nc[1] * cc[2]));
-  } else if (lane == 8 && G.n_points > 0) {
-    int2 rng;
-    if (cell_list_of(G, qx, qy, qz, rng)) rec = make_float4(__int_as_float(rng.x), __int_as_float(rng.y), 0.f, __int_as_float(-1));
-  }
-  return rec;
-}
-struct FieldStart {
-  NNResult32 nn;  // the best of the 8 corner records
-  int2 rng;       // q's cell-list range (-1: none)
-};
-// width: 32 (one query per warp) or 16 (one per half warp; every lane calls it).
-__device__ __forceinline__ FieldStart field_corner_candidate(const float4& rec, float qx, float qy, float qz, int width = 32) {
-  const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & (width - 1);
-  const int idx = __float_as_int(rec.w);
-  unsigned long long key = ~0ull;
-  if (lane < 8 && idx >= 0) {  // the FP32 expression of every walk (point_d2_32)
-    const float dx = rec.x - qx, dy = rec.y - qy, dz = rec.z - qz;
-    key = nn_key(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), idx);
-  }
-  for (int o = 4; o > 0; o >>= 1) {
-    const unsigned long long k2 = __shfl_xor_sync(FULL, key, o);
-    key = k2 < key ? k2 : key;
-  }
-  key = __shfl_sync(FULL, key, 0, width);
-  const int rx = __shfl_sync(FULL, __float_as_int(rec.x), 8, width), ry = __shfl_sync(FULL, __float_as_int(rec.y), 8, width);
-  FieldStart f{{INFINITY, -1}, make_int2(rx, ry)};
-  if (key != ~0ull) {
-    f.nn.d2 = __uint_as_float((unsigned)(key >> 32));
-    f.nn.idx = (int)(unsigned)(key & 0xffffffffu);
-  }
-  return f;
 }
 
 __device__ __forceinline__ int f2o(float f) {

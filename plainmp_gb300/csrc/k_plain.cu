@@ -3,6 +3,7 @@
 // ompl/motion_validator.cpp) with bit-identical FP64 arithmetic (compiled --fmad=false).
 #include "pm_launch.h"
 #include "pm_view.cuh"
+#include "pm_warp.cuh"
 
 using namespace pmd;
 
@@ -225,16 +226,19 @@ __global__ void k_sphere_centres64(const PmTablesHdr* __restrict__ T, const doub
     }
   }
 }
+// With a point cloud, a warp per sphere (CLOUD), for the cooperative search; else a thread.
+template <bool CLOUD>
 __global__ void k_sphere_sdf64(const PmTablesHdr* __restrict__ T, const double* __restrict__ centres, int64_t n,
                                double* __restrict__ dist) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (CLOUD) i >>= 5;
   if (i >= n) return;
   TView v(T);
   const int k = (int)(i % T->n_spheres);
   const D3 c{centres[3 * i], centres[3 * i + 1], centres[3 * i + 2]};
   double d = INFINITY;
-  for (int pi = 0; pi < T->n_prims; pi++) d = fmin(d, prim_eval(v.P[pi], v.C, c) - v.sr[k]);
-  dist[i] = d;
+  for (int pi = 0; pi < T->n_prims; pi++) d = fmin(d, (CLOUD ? prim_eval_warp(v.P[pi], v.C, c) : prim_eval(v.P[pi], v.C, c)) - v.sr[k]);
+  if (!CLOUD || (threadIdx.x & 31) == 0) dist[i] = d;
 }
 
 __global__ void k_spheres_of_state(const PmTablesHdr* __restrict__ T, const double* __restrict__ state, int groups,
@@ -420,46 +424,43 @@ __global__ void k_link_poses(const double* __restrict__ state, const int32_t* __
 }
 
 // ------------------------------------------------------------------ SDF utilities
+// A thread per point, or with point clouds (CLOUD) a warp, for the cooperative search.
+template <bool CLOUD>
 __global__ void k_sdf_points(const PmPrim* __restrict__ prims, int n_prims, const PmGridDev* __restrict__ clouds, int is_union,
                              const double* __restrict__ pts, const double* __restrict__ radii, int64_t n, double* eval_out,
                              uint8_t* outside_out) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (CLOUD) i >>= 5;
   if (i >= n) return;
+  const bool writer = !CLOUD || (threadIdx.x & 31) == 0;
   D3 p{pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]};
   if (eval_out) {
     double v = is_union ? 1.7976931348623157e308 : 0.0;
-    if (is_union) {
-      for (int k = 0; k < n_prims; k++) v = fmin(v, prim_eval(prims[k], clouds, p));
-    } else if (n_prims > 0) {
-      v = prim_eval(prims[0], clouds, p);
+    for (int k = 0; k < (is_union ? n_prims : min(n_prims, 1)); k++) {
+      const double e = CLOUD ? prim_eval_warp(prims[k], clouds, p) : prim_eval(prims[k], clouds, p);
+      v = is_union ? fmin(v, e) : e;
     }
-    eval_out[i] = v;
+    if (writer) eval_out[i] = v;
   }
   if (outside_out) {
     bool o = true;
-    for (int k = 0; k < n_prims && o; k++) o = prim_outside(prims[k], clouds, p, radii[i]);
-    outside_out[i] = o ? 1 : 0;
+    for (int k = 0; k < n_prims && o; k++)
+      o = CLOUD && prims[k].kind == PM_SDF_CLOUD ? cloud_outside_warp(prims[k], clouds, p, radii[i], nullptr)
+                                                 : prim_outside(prims[k], clouds, p, radii[i]);
+    if (writer) outside_out[i] = o ? 1 : 0;
   }
 }
 
-__global__ void k_cloud_nearest(const PmGridDev* __restrict__ grid, const double* __restrict__ pts, int64_t n, double* sq,
-                                double* near3) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// KDTree::query / sqdist: one warp per query (warp_nearest64).
+__global__ void __launch_bounds__(256) k_cloud_nearest(const PmGridDev* __restrict__ grid, const double* __restrict__ pts, int64_t n,
+                                                       double* sq, double* near3) {
+  const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   if (i >= n) return;
-  D3 p{pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]};
-  NNResult64 r = grid_nearest64(*grid, p);
-  if (sq) sq[i] = r.d2;
-  if (near3) {
-    double x = NAN, y = NAN, z = NAN;
-    if (r.idx >= 0) {
-      x = grid->px[r.idx];
-      y = grid->py[r.idx];
-      z = grid->pz[r.idx];
-    }
-    near3[3 * i] = x;
-    near3[3 * i + 1] = y;
-    near3[3 * i + 2] = z;
-  }
+  const int lane = threadIdx.x & 31;
+  const D3 p{pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]};
+  const NNResult64 r = warp_nearest64(*grid, p);
+  if (lane == 0 && sq) sq[i] = r.d2;
+  if (lane < 3 && near3) near3[3 * i + lane] = r.idx < 0 ? NAN : (lane == 0 ? grid->px : (lane == 1 ? grid->py : grid->pz))[r.idx];
 }
 
 inline unsigned grid_for(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
@@ -503,7 +504,10 @@ cudaError_t launch_sphere_dist64(const PmTablesHdr* T, const PmTablesHdr& h, con
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || !dist) return e;
   const int64_t n = B * h.n_spheres;
-  k_sphere_sdf64<<<grid_for(n, 128), 128, 0, s>>>(T, centres, n, dist);
+  if (h.n_clouds > 0)
+    k_sphere_sdf64<true><<<grid_for(n, 8), 256, 0, s>>>(T, centres, n, dist);
+  else
+    k_sphere_sdf64<false><<<grid_for(n, 128), 128, 0, s>>>(T, centres, n, dist);
   return cudaGetLastError();
 }
 cudaError_t launch_spheres_of_state(const PmTablesHdr* T, const double* state, int groups, double* out4, cudaStream_t s) {
@@ -517,16 +521,19 @@ cudaError_t launch_check_motion64(const PmTablesHdr* T, const double* state, con
   k_check_motion64<<<grid_for(E, 64), 64, 0, s>>>(T, state, s1, s2, E, type, width, resolution, seq, out, n_checked);
   return cudaGetLastError();
 }
-cudaError_t launch_sdf_points(const PmPrim* prims, int n_prims, const PmGridDev* clouds, int is_union, const double* pts,
-                              const double* radii, int64_t n, double* eval_out, uint8_t* outside_out, cudaStream_t s) {
+cudaError_t launch_sdf_points(const PmPrim* prims, int n_prims, const PmGridDev* clouds, int n_clouds, int is_union,
+                              const double* pts, const double* radii, int64_t n, double* eval_out, uint8_t* outside_out, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_sdf_points<<<grid_for(n, 128), 128, 0, s>>>(prims, n_prims, clouds, is_union, pts, radii, n, eval_out, outside_out);
+  if (n_clouds > 0)
+    k_sdf_points<true><<<grid_for(n, 8), 256, 0, s>>>(prims, n_prims, clouds, is_union, pts, radii, n, eval_out, outside_out);
+  else
+    k_sdf_points<false><<<grid_for(n, 128), 128, 0, s>>>(prims, n_prims, clouds, is_union, pts, radii, n, eval_out, outside_out);
   return cudaGetLastError();
 }
 cudaError_t launch_cloud_nearest(const PmGridDev* grid, const double* pts, int64_t n, double* sq, double* near3,
                                  cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_cloud_nearest<<<grid_for(n, 128), 128, 0, s>>>(grid, pts, n, sq, near3);
+  k_cloud_nearest<<<grid_for(n, 8), 256, 0, s>>>(grid, pts, n, sq, near3);
   return cudaGetLastError();
 }
 

@@ -96,8 +96,8 @@ cudaError_t launch_posecst_valid64(const PmTablesHdr* T, const double* state, co
                                    int64_t B, uint8_t* out, cudaStream_t s);
 
 // ---- SDF utilities (k_plain.cu): prims/clouds describe one SDF (a union is flattened)
-cudaError_t launch_sdf_points(const PmPrim* prims, int n_prims, const PmGridDev* clouds, int is_union, const double* pts,
-                              const double* radii, int64_t n, double* eval_out, uint8_t* outside_out, cudaStream_t s);
+cudaError_t launch_sdf_points(const PmPrim* prims, int n_prims, const PmGridDev* clouds, int n_clouds, int is_union,
+                              const double* pts, const double* radii, int64_t n, double* eval_out, uint8_t* outside_out, cudaStream_t s);
 cudaError_t launch_cloud_nearest(const PmGridDev* grid, const double* pts, int64_t n, double* sq, double* near3,
                                  cudaStream_t s);
 
