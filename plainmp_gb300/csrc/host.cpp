@@ -764,6 +764,89 @@ struct HostCst {
     }
   }
 
+  // The FP32 image of the tables: the records of the fast kernels as a block keeps them.  Slots
+  // without a control joint and the base pose are filled in by the block from the model state.
+  static std::vector<char> fast_image(const std::vector<PmSlot>& slots, const std::vector<PmGroup>& groups, const std::vector<double>& sx,
+                                      const std::vector<double>& sy, const std::vector<double>& sz, const std::vector<double>& sr,
+                                      const std::vector<int32_t>& sgroup, const std::vector<int32_t>& pairs,
+                                      const std::vector<PmPrim>& prims) {
+    std::vector<char> img;
+    auto add = [&](const void* p, size_t bytes) {
+      const size_t off = img.size();
+      img.resize(up16(off + bytes), 0);
+      if (bytes) std::memcpy(img.data() + off, p, bytes);
+    };
+    // |v| in FP32, rounded up
+    auto norm_up = [](const float* v) { return std::sqrt(std::fmaf(v[0], v[0], std::fmaf(v[1], v[1], v[2] * v[2]))) * 1.000002f + 1e-9f; };
+    std::vector<PmSlotF> sl(slots.size());
+    for (size_t i = 0; i < slots.size(); i++) {
+      const PmSlot& s = slots[i];
+      PmSlotF& f = sl[i];
+      std::memset(&f, 0, sizeof(f));
+      f.parent = s.parent;
+      f.mode = s.mode;
+      f.qcol = s.qcol;
+      f.split = s.split;
+      f.lid = s.origin_identity;
+      for (int k = 0; k < 3; k++) f.axis[k] = (float)s.axis[k];
+      for (int k = 0; k < 4; k++) f.lq[k] = (float)s.oq[k];
+      for (int k = 0; k < 3; k++) f.lt[k] = (float)s.ot[k];
+      f.lt1 = (float)((std::fabs(s.ot[0]) + std::fabs(s.ot[1]) + std::fabs(s.ot[2])) * (1.0 + 1e-6));
+    }
+    std::vector<PmSphereF> sp(sr.size());
+    for (size_t i = 0; i < sr.size(); i++) {
+      const float v[3] = {(float)sx[i], (float)sy[i], (float)sz[i]};
+      sp[i] = PmSphereF{v[0], v[1], v[2], (float)sr[i], sgroup[i], sr[i] < 1e-6, norm_up(v)};
+    }
+    std::vector<PmGroupF> gr(groups.size());
+    for (size_t i = 0; i < groups.size(); i++) {
+      const PmGroup& G = groups[i];
+      const float v[3] = {(float)G.rel[0], (float)G.rel[1], (float)G.rel[2]};
+      gr[i] = PmGroupF{{v[0], v[1], v[2]}, (float)G.radius, G.slot, G.begin, G.count, G.only_self, G.radius < 1e-6, norm_up(v), {0, 0}};
+    }
+    std::vector<PmPrimF> pr(prims.size());
+    for (size_t i = 0; i < prims.size(); i++) {
+      const PmPrim& P = prims[i];
+      PmPrimF& f = pr[i];
+      f.kind = P.kind;
+      f.aa = P.axis_aligned;
+      f.za = P.z_axis_aligned;
+      f.cloud = P.cloud;
+      for (int k = 0; k < 3; k++) {
+        f.lb[k] = (float)P.lb[k];
+        f.ub[k] = (float)P.ub[k];
+        f.pos[k] = (float)P.pos[k];
+      }
+      for (int k = 0; k < 9; k++) f.rot[k] = (float)P.rot[k];
+      f.a = (float)P.a;
+      f.b = (float)P.b;
+      f.c = (float)P.c;
+      f.mag = (P.kind == PM_SDF_GROUND || P.kind == PM_SDF_CLOUD)
+                  ? (float)std::fabs(P.a)
+                  : (float)(std::fabs(P.pos[0]) + std::fabs(P.pos[1]) + std::fabs(P.pos[2]) + std::fabs(P.a) + std::fabs(P.b) + std::fabs(P.c));
+    }
+    // the two-thread FK's slot lists, parents first (the slot order): the trunk, then the two threads'
+    // subtrees, and their lengths
+    static_assert(3 * PM_MAX_SLOTS + 12 <= PM_IMG_TAIL, "image tail");
+    char tail[PM_IMG_TAIL];
+    std::memset(tail, 0, sizeof(tail));
+    int32_t n[3] = {0, 0, 0};
+    for (size_t i = 0; i < slots.size(); i++) {
+      const int sp_ = slots[i].split, l = sp_ == 0 ? 0 : (sp_ == 2 ? 1 : 2);
+      tail[l * PM_MAX_SLOTS + n[l]++] = (char)i;
+    }
+    std::memcpy(tail + 3 * PM_MAX_SLOTS, n, sizeof(n));
+    const float base8[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    add(sl.data(), sl.size() * sizeof(PmSlotF));
+    add(base8, sizeof(base8));
+    add(sp.data(), sp.size() * sizeof(PmSphereF));
+    add(gr.data(), gr.size() * sizeof(PmGroupF));
+    add(pr.data(), pr.size() * sizeof(PmPrimF));
+    add(pairs.data(), pairs.size() * sizeof(int32_t));
+    add(tail, sizeof(tail));
+    return img;
+  }
+
   void build_tables() {
     HostModel& m = *kin;
     const int nl = m.n_link();
@@ -893,6 +976,9 @@ struct HostCst {
     h.off_pairs = put(prs.data(), prs.size() * 4);
     h.off_prims = put(prims.data(), prims.size() * sizeof(PmPrim));
     h.off_clouds = put(clouds.data(), clouds.size() * sizeof(PmGridDev));
+    const std::vector<char> img = fast_image(slots, grec, sx, sy, sz, sr, sgroup, prs, prims);
+    h.img_bytes = (int64_t)img.size();
+    h.off_img = put(img.data(), img.size());
     align();
     h.total_bytes = (int64_t)buf.size();
     std::memcpy(buf.data(), &h, sizeof(h));

@@ -41,34 +41,10 @@ constexpr float kU = 5.9604645e-8f;  // 2^-24
 // gives about 52 units for the box, the largest case.
 __device__ __forceinline__ float margin32(float mag) { return 1e-6f + 64.0f * kU * (1.0f + mag); }
 
-struct PrimF {
-  int kind, aa, za, cloud;
-  float lb[3], ub[3], pos[3], rot[9];
-  float a, b, c, mag;
-};
-struct SphereF {
-  float x, y, z, r;
-  int group, tiny;  // tiny: the FP64 radius is below 1e-6 (the reference's special cases)
-  float sn;         // |offset in the link frame|, rounded up (for the FK error bound)
-};
-struct GroupF {
-  float rel[3], radius;
-  int slot, begin, count, only_self;
-  int tiny;
-  float gn;  // |group centre in the link frame|, rounded up
-  int pad[2];
-};
-
-// FP32 FK slot: the local transform's constant part (joint origin, or the fixed transform of a
-// slot without a control joint, taken from the model state when the block starts).
-struct SlotF {
-  int parent, mode, qcol, lid;
-  int split;  // PmSlot::split: the FK phase and thread that compute this slot
-  float axis[3];
-  float lq[4];
-  float lt[3];
-  float lt1;  // |lt|_1 (prismatic: of the origin part)
-};
+using PrimF = PmPrimF;
+using SphereF = PmSphereF;
+using GroupF = PmGroupF;
+using SlotF = PmSlotF;
 // Per slot and configuration in shared memory: [0..8] R, [9..11] t, [12] et = bound on |t - t64|,
 // [13] eb = bound on |R - R64| as an operator (8 eq + 24 u), [14..17] world quaternion,
 // [18] eq = bound on |q - q64|_2.  A point s of the link frame then lies within et + eb |s| of
@@ -1144,7 +1120,8 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
   __syncthreads();
 }
 
-// Shared-memory layout of a fast block; every array starts on a 16-byte boundary.
+// Shared-memory layout of a fast block; every array starts on a 16-byte boundary.  slot .. pairs are the
+// tables' FP32 image in its own order, fkl its tail.
 struct SmemLayout {
   size_t pose, slot, base8, sph, grp, prm, pairs, flags, cull, qbuf, fkl, hq_n, hq, sdist, total;
 };
@@ -1173,7 +1150,7 @@ __host__ __device__ inline SmemLayout smem_layout(const PmTablesHdr& h, int cpb,
   L.qbuf = o;
   o = a16(o + sizeof(double) * (size_t)cpb * h.q_dim);
   L.fkl = o;
-  o = a16(o + 3 * PM_MAX_SLOTS + 3 * sizeof(int));
+  o = a16(o + PM_IMG_TAIL);
   L.hq_n = o;
   o = a16(o + 16);
   L.hq = o;
@@ -1205,99 +1182,38 @@ __device__ Smem carve(unsigned char* p, const PmTablesHdr* T, int cpb) {
   return sm;
 }
 
-// The FK slots (FP32, the local transforms' constant parts from the model state) and the fixed base
-// pose into shared memory (no barrier).
-__device__ void stage_slots(const TView& v, SlotF* __restrict__ slot, float* __restrict__ base8, const double* __restrict__ state) {
-  const PmTablesHdr* T = v.T;
-  const int tid = threadIdx.x;
-  for (int i = tid; i < T->n_slots; i += blockDim.x) {
-    const PmSlot& S = v.S[i];
-    SlotF f;
-    f.parent = S.parent;
-    f.mode = S.mode;
-    f.qcol = S.qcol;
-    f.split = S.split;
-    for (int k = 0; k < 3; k++) f.axis[k] = (float)S.axis[k];
-    double lt[3];
-    if (S.mode == PM_FK_STATE) {
-      const double* r = state + (int64_t)PM_STATE_LINK_ROW(S.link) * PM_STATE_STRIDE;
-      for (int k = 0; k < 4; k++) f.lq[k] = (float)r[k];
-      for (int k = 0; k < 3; k++) lt[k] = r[4 + k];
-      f.lid = r[7] != 0.0;
-    } else {
-      for (int k = 0; k < 4; k++) f.lq[k] = (float)S.oq[k];
-      for (int k = 0; k < 3; k++) lt[k] = S.ot[k];
-      f.lid = S.origin_identity;
-    }
-    for (int k = 0; k < 3; k++) f.lt[k] = (float)lt[k];
-    f.lt1 = (float)((fabs(lt[0]) + fabs(lt[1]) + fabs(lt[2])) * (1.0 + 1e-6));
-    slot[i] = f;
-  }
-  if (tid < 8) {
-    const double* b = state + (int64_t)PM_STATE_BASE_ROW * PM_STATE_STRIDE;
-    base8[tid] = tid < 7 ? (float)b[tid] : 0.0f;
-  }
-}
-
+// The block's tables: the FP32 image by 16-byte copies, then the parts that the model state holds (the
+// fixed transforms of slots without a control joint, the fixed base pose), whose loads are issued before
+// the image has arrived.
 __device__ void stage_tables(const TView& v, const Smem& sm, const double* __restrict__ state) {
   const PmTablesHdr* T = v.T;
   const int tid = threadIdx.x;
-  stage_slots(v, sm.slot, sm.base8, state);
-  for (int i = tid; i < T->n_spheres; i += blockDim.x) {
-    SphereF s;
-    s.x = (float)v.sx[i];
-    s.y = (float)v.sy[i];
-    s.z = (float)v.sz[i];
-    s.r = (float)v.sr[i];
-    s.group = v.sgroup[i];
-    s.tiny = v.sr[i] < 1e-6;
-    s.sn = sqrtf(fmaf(s.x, s.x, fmaf(s.y, s.y, s.z * s.z))) * 1.000002f + 1e-9f;  // rounded up
-    sm.sph[i] = s;
+  const float4* src = pm_at<float4>(T, T->off_img);
+  float4* body = reinterpret_cast<float4*>(sm.slot);
+  float4* tail = reinterpret_cast<float4*>(sm.fkl);
+  const int n = (int)(T->img_bytes / 16);
+  for (int i = tid; i < n - PM_IMG_TAIL / 16; i += blockDim.x) body[i] = __ldg(src + i);
+  if (tid < PM_IMG_TAIL / 16) tail[tid] = __ldg(src + n - PM_IMG_TAIL / 16 + tid);
+  float row[8];
+  int mine = -2;  // the slot whose state row this thread holds (-1: the base pose)
+  if (tid < T->n_slots && v.S[tid].mode == PM_FK_STATE && v.S[tid].parent >= 0) mine = tid;
+  if (tid == T->n_slots) mine = -1;
+  if (mine >= -1) {
+    const double* r = state + (int64_t)(mine < 0 ? PM_STATE_BASE_ROW : PM_STATE_LINK_ROW(v.S[mine].link)) * PM_STATE_STRIDE;
+    for (int k = 0; k < 7; k++) row[k] = (float)r[k];
+    // |t|_1, and in its sign the identity flag
+    row[7] = (float)((fabs(r[4]) + fabs(r[5]) + fabs(r[6])) * (1.0 + 1e-6));
+    if (r[7] != 0.0) row[7] = copysignf(row[7], -1.0f);
   }
-  for (int i = tid; i < T->n_groups; i += blockDim.x) {
-    const PmGroup& G = v.G[i];
-    GroupF g;
-    g.rel[0] = (float)G.rel[0];
-    g.rel[1] = (float)G.rel[1];
-    g.rel[2] = (float)G.rel[2];
-    g.radius = (float)G.radius;
-    g.slot = G.slot;
-    g.begin = G.begin;
-    g.count = G.count;
-    g.only_self = G.only_self;
-    g.tiny = G.radius < 1e-6;
-    g.gn = sqrtf(fmaf(g.rel[0], g.rel[0], fmaf(g.rel[1], g.rel[1], g.rel[2] * g.rel[2]))) * 1.000002f + 1e-9f;
-    sm.grp[i] = g;
-  }
-  for (int i = tid; i < T->n_prims; i += blockDim.x) {
-    const PmPrim& P = v.P[i];
-    PrimF f;
-    f.kind = P.kind;
-    f.aa = P.axis_aligned;
-    f.za = P.z_axis_aligned;
-    f.cloud = P.cloud;
-    for (int k = 0; k < 3; k++) {
-      f.lb[k] = (float)P.lb[k];
-      f.ub[k] = (float)P.ub[k];
-      f.pos[k] = (float)P.pos[k];
-    }
-    for (int k = 0; k < 9; k++) f.rot[k] = (float)P.rot[k];
-    f.a = (float)P.a;
-    f.b = (float)P.b;
-    f.c = (float)P.c;
-    f.mag = (P.kind == PM_SDF_GROUND || P.kind == PM_SDF_CLOUD)
-                ? (float)fabs(P.a)
-                : (float)(fabs(P.pos[0]) + fabs(P.pos[1]) + fabs(P.pos[2]) + fabs(P.a) + fabs(P.b) + fabs(P.c));
-    sm.prm[i] = f;
-  }
-  for (int i = tid; i < T->n_pairs; i += blockDim.x) sm.pairs[i] = make_int2(v.pairs[2 * i], v.pairs[2 * i + 1]);
-  if (tid == 0) {  // the two-thread FK's slot lists, parents first (the slot order)
-    int n[3] = {0, 0, 0};
-    for (int i = 0; i < T->n_slots; i++) {
-      const int sp = v.S[i].split, l = sp == 0 ? 0 : (sp == 2 ? 1 : 2);
-      sm.fkl[l * PM_MAX_SLOTS + n[l]++] = (unsigned char)i;
-    }
-    for (int l = 0; l < 3; l++) sm.fkn[l] = n[l];
+  __syncthreads();
+  if (mine >= 0) {
+    SlotF& f = sm.slot[mine];
+    for (int k = 0; k < 4; k++) f.lq[k] = row[k];
+    for (int k = 0; k < 3; k++) f.lt[k] = row[4 + k];
+    f.lid = signbit(row[7]);
+    f.lt1 = fabsf(row[7]);
+  } else if (mine == -1) {
+    for (int k = 0; k < 8; k++) sm.base8[k] = k < 7 ? row[k] : 0.0f;
   }
   __syncthreads();
 }
@@ -1306,9 +1222,8 @@ __device__ void stage_tables(const TView& v, const Smem& sm, const double* __res
 // per SM): the same budget the compiler picks for NT alone, but its allocation under the explicit
 // target measured 4-8 % faster in both modes.
 template <int CPB, int NT>
-__global__ void __launch_bounds__(NT, 65536 / (NT * 64)) k_fast_valid(const PmTablesHdr* __restrict__ T, const double* __restrict__ state,
-                                                    const double* __restrict__ q, int64_t B, uint8_t* __restrict__ out,
-                                                    float* __restrict__ dist32, float cutoff, Scratch scr) {
+__global__ void __launch_bounds__(NT, 65536 / (NT * 64)) k_fast_valid(const PmTablesHdr* __restrict__ T, const double* __restrict__ state, const double* __restrict__ q, int64_t B,
+                                                    uint8_t* __restrict__ out, float* __restrict__ dist32, float cutoff, Scratch scr) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TView v(T);
   Smem sm = carve(smem_raw, T, CPB);
@@ -1322,8 +1237,7 @@ __global__ void __launch_bounds__(NT, 65536 / (NT * 64)) k_fast_valid(const PmTa
 // 64 registers a thread as the occupancy target (8 blocks of 128 per SM), as for k_fast_valid:
 // 9-15 % faster than the compiler's own choice (72 registers, with spills).
 template <int CPB, int NT>
-__global__ void __launch_bounds__(NT, 65536 / (NT * 64)) k_fast_edges(const PmTablesHdr* __restrict__ T, const double* __restrict__ state, EdgeSource src,
-                                                    unsigned long long* next, Scratch scr) {
+__global__ void __launch_bounds__(NT, 65536 / (NT * 64)) k_fast_edges(const PmTablesHdr* __restrict__ T, const double* __restrict__ state, EdgeSource src, unsigned long long* next, Scratch scr) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ long long chunk;
   TView v(T);
@@ -1715,7 +1629,7 @@ cudaError_t launch_fast_valid(const PmTablesHdr* T, const PmTablesHdr& h, const 
 #define PM_FAST_CASE(C, N)                                                                      \
   if (cpb == C && nt == N) {                                                                     \
     if ((e = prep(k_fast_valid<C, N>, sm)) != cudaSuccess) return e;                             \
-    k_fast_valid<C, N><<<grid, N, sm, s>>>(T, state, q, B, out, dist32, cutoff, scr);            \
+    k_fast_valid<C, N><<<grid, N, sm, s>>>(T, state, q, B, out, dist32, cutoff, scr);         \
     launched = true;                                                                             \
   }
   bool launched = false;
@@ -1775,7 +1689,7 @@ cudaError_t launch_fast_edges(const PmTablesHdr* T, const PmTablesHdr& h, const 
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fast_edges<C, N>, N, sm)) != cudaSuccess) return e; \
     const unsigned grid = (unsigned)std::min<int64_t>((int64_t)n_sm * (per_sm > 0 ? per_sm : 1), std::max<int64_t>(1, 4 * E)); \
     prof_begin("k_fast_edges", s);                                                                                        \
-    k_fast_edges<C, N><<<grid, N, sm, s>>>(T, state, src, next, scr);                                                     \
+    k_fast_edges<C, N><<<grid, N, sm, s>>>(T, state, src, next, scr);                                                  \
     prof_end("k_fast_edges", s);                                                                                          \
     launched = true;                                                                                                     \
   }

@@ -146,11 +146,44 @@ struct PmLinkBounds {
   int32_t n;
 };
 
+// FP32 records of the fast kernels, written by the host in the order and layout that a block keeps them
+// in shared memory, so that a block stages them with one pass of 16-byte copies.
+struct PmSlotF {  // FK slot: the local transform's constant part (joint origin, or the fixed transform of a
+                  // slot without a control joint, which the block takes from the model state)
+  int32_t parent, mode, qcol, lid;
+  int32_t split;  // PmSlot::split: the FK phase and thread that compute this slot
+  float axis[3];
+  float lq[4];
+  float lt[3];
+  float lt1;      // |lt|_1 (prismatic: of the origin part), rounded up
+};
+struct PmSphereF {
+  float x, y, z, r;
+  int32_t group, tiny;  // tiny: the FP64 radius is below 1e-6 (the reference's special cases)
+  float sn;             // |offset in the link frame|, rounded up (for the FK error bound)
+};
+struct PmGroupF {
+  float rel[3], radius;
+  int32_t slot, begin, count, only_self;
+  int32_t tiny;
+  float gn;  // |group centre in the link frame|, rounded up
+  int32_t pad[2];
+};
+struct PmPrimF {
+  int32_t kind, aa, za, cloud;
+  float lb[3], ub[3], pos[3], rot[9];
+  float a, b, c, mag;
+};
+// The image: slots, fixed base pose (8 floats), spheres, groups, primitives, pairs, each on a 16-byte
+// boundary, and a tail with the two-thread FK's slot lists [3][PM_MAX_SLOTS] (bytes) and their lengths [3].
+#define PM_IMG_TAIL 208
+
 struct PmTablesHdr {
   int32_t n_slots, n_ctrl, n_groups, n_spheres;
   int32_t n_pairs, n_prims, q_dim, base_type;
   int32_t root_slot, n_clouds, pad0, pad1;
   int64_t off_slots, off_joints, off_groups, off_sx, off_sy, off_sz, off_sr, off_sgroup, off_pairs, off_prims, off_clouds;
+  int64_t off_img, img_bytes;  // the FP32 image
   int64_t total_bytes;
 };
 
