@@ -186,15 +186,17 @@ int pmgpu_cst_is_valid_fast(pmgpu_cst* c, const double* q, int64_t B, uint8_t* o
 
 /* Launch shape of the fast kernel: configurations per block and threads per block, one of
  * (16,128) (32,128) (16,256) (32,256) (64,256) (32,512) (64,512) (128,512); chosen per workload by the
- * autotuner (plainmp_gb300/autotune.py).  No counterpart in the reference. */
+ * autotuner (plainmp_gb300/autotune.py).  Until it is set, each call chooses by the batch and sphere
+ * counts, and the getter gives (32,256).  No counterpart in the reference. */
 int pmgpu_cst_set_fast_launch(pmgpu_cst* c, int configs_per_block, int threads_per_block);
 int pmgpu_cst_get_fast_launch(const pmgpu_cst* c, int* configs_per_block, int* threads_per_block);
 /* The fast kernels' other tuning parameters, chosen per workload by the autotuner.  No counterpart
  * in the reference.  sphere_tile: spheres of one configuration per warp row of sphere tasks (0 or a
- * power of two up to 32; 0 and values below 32 / configurations-per-block give the least);
+ * power of two up to 32; at least 32 / configurations-per-block are used; 0: 8);
  * hq_blocks_per_sm: blocks of 256 threads per SM of the hard cloud-query kernel (1..8);
  * edge_configs_per_block, edge_threads: the edge kernel's waypoints and threads per block, one of
- * (16,128) (32,128) (32,256) (64,256).  Defaults: 0, 4, 32, 128. */
+ * (16,128) (32,128) (32,256) (64,256).  Defaults: 0, 4, and an edge shape of the call's choice, which the
+ * getter gives as 32, 128. */
 int pmgpu_cst_set_fast_tuning(pmgpu_cst* c, int sphere_tile, int hq_blocks_per_sm, int edge_configs_per_block, int edge_threads);
 int pmgpu_cst_get_fast_tuning(const pmgpu_cst* c, int* sphere_tile, int* hq_blocks_per_sm, int* edge_configs_per_block,
                               int* edge_threads);

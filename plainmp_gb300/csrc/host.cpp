@@ -673,6 +673,7 @@ struct HostCst {
   int fast_nt = 256;  // threads per block of the fast kernel
   FastTuning tune;    // the fast kernels' other autotuned parameters
   int edge_cpb = 32, edge_nt = 128;  // waypoints and threads per block of the edge kernel
+  bool shape_set = false, tune_set = false;  // set by the caller (the autotuner); else chosen per call
   std::vector<int> slot_of_link;
   std::vector<PmSlot> ctrl_recs;  // per control joint (child link, REV/PRIS) for state updates
   DevBuf d_ctrl_recs;
@@ -1004,6 +1005,40 @@ struct HostCst {
     if (!ctrl_recs.empty())
       cuda_check(cudaMemcpy(d_ctrl_recs.p, ctrl_recs.data(), ctrl_recs.size() * sizeof(PmSlot), cudaMemcpyHostToDevice),
                  "control records upload");
+  }
+
+  // Launch shape and tuning of a fast call of B configurations where the caller set none.  (16, 256) and
+  // tiles of 8 spheres while every block is resident at once (4 of 256 threads per SM): the block's serial
+  // parts then weigh most.  Beyond that, robots of up to 64 spheres run (16, 128), twice as many blocks in
+  // flight; larger ones stay at (16, 256).  Measured against (32, 256) with the least tile, us:
+  // dual arm (120 spheres) x cloud, 65,536 with distances 622 -> 510, 200,003 validity 630 -> 469; chain
+  // (56) x 20 primitives, 4,096 with distances 81 -> 64, 65,536 273 -> 218; 16,384 at (16, 256) 97, at
+  // (16, 128) 89; the same chain at 4,096 and (16, 128) 76.
+  FastTuning fast_shape(int64_t B, bool want_dist, int* cpb, int* nt) const {
+    *cpb = fast_cpb;
+    *nt = fast_nt;
+    FastTuning t = tune;
+    if (t.sphere_tile_log2 < 0) t.sphere_tile_log2 = 3;
+    if (!shape_set && fast_smem_bytes(hdr, fast_cpb, want_dist) <= 200 * 1024) {  // what does not fit at (32, 256) is refused as it was
+      int n_sm = 0;
+      cuda_check(sm_count(&n_sm), "device attribute");
+      *cpb = 16;
+      *nt = (B + 15) / 16 > 4 * (int64_t)n_sm && hdr.n_spheres <= 64 ? 128 : 256;
+    }
+    return t;
+  }
+
+  // Launch shape and tile of the edge kernel where the caller set none: (16, 128) and tiles of 8 spheres.
+  // Measured against (32, 128) with the least tile, us, 1,024 edges of 1 to 120 waypoints: chain x
+  // primitives 169 -> 156, planar chain x cloud 150 -> 140, dual arm x cloud 264 -> 201; 24 edges: 74 -> 66,
+  // 86 -> 80, 68 -> 61.
+  FastTuning edge_shape(int* cpb, int* nt) const {
+    *cpb = edge_cpb;
+    *nt = edge_nt;
+    FastTuning t = tune;
+    if (t.sphere_tile_log2 < 0) t.sphere_tile_log2 = 3;
+    if (!tune_set && fast_smem_bytes(hdr, edge_cpb, false) <= 200 * 1024) *cpb = 16;  // what does not fit at (32, 128) is refused as it was
+    return t;
   }
 
   const int16_t* seq_table() {
@@ -1890,6 +1925,7 @@ int pmgpu_cst_set_fast_launch(pmgpu_cst* c, int configs_per_block, int threads_p
     if (!found) throw std::invalid_argument("unsupported (configs_per_block, threads_per_block) pair");
     c->c.fast_cpb = configs_per_block;
     c->c.fast_nt = threads_per_block;
+    c->c.shape_set = true;
   });
 }
 int pmgpu_cst_set_fast_tuning(pmgpu_cst* c, int sphere_tile, int hq_blocks_per_sm, int edge_configs_per_block, int edge_threads) {
@@ -1904,17 +1940,18 @@ int pmgpu_cst_set_fast_tuning(pmgpu_cst* c, int sphere_tile, int hq_blocks_per_s
     bool found = false;
     for (auto& p : ok) found = found || (p[0] == edge_configs_per_block && p[1] == edge_threads);
     if (!found) throw std::invalid_argument("unsupported edge (configs_per_block, threads_per_block) pair");
-    c->c.tune.sphere_tile_log2 = sphere_tile == 0 ? 0 : l;
+    c->c.tune.sphere_tile_log2 = l;
     c->c.tune.hq_blocks_per_sm = hq_blocks_per_sm;
     c->c.edge_cpb = edge_configs_per_block;
     c->c.edge_nt = edge_threads;
+    c->c.tune_set = true;
   });
 }
 int pmgpu_cst_get_fast_tuning(const pmgpu_cst* c, int* sphere_tile, int* hq_blocks_per_sm, int* edge_configs_per_block,
                               int* edge_threads) {
   return guarded([&] {
     check_ptr(c, "cst");
-    if (sphere_tile) *sphere_tile = c->c.tune.sphere_tile_log2 == 0 ? 0 : (1 << c->c.tune.sphere_tile_log2);
+    if (sphere_tile) *sphere_tile = c->c.tune.sphere_tile_log2 <= 0 ? 0 : (1 << c->c.tune.sphere_tile_log2);
     if (hq_blocks_per_sm) *hq_blocks_per_sm = c->c.tune.hq_blocks_per_sm;
     if (edge_configs_per_block) *edge_configs_per_block = c->c.edge_cpb;
     if (edge_threads) *edge_threads = c->c.edge_nt;
@@ -1946,6 +1983,8 @@ static void fast_host_pipelined(HostCst& C, const PmTablesHdr* T, const double* 
   const int64_t n_chunks = std::max<int64_t>(2, std::min<int64_t>(4, B / 32768));
   const int64_t chunk = ((B + n_chunks - 1) / n_chunks + 127) / 128 * 128;
   const unsigned cap = (unsigned)std::min<int64_t>(std::max<int64_t>(4 * chunk, 1 << 16), (int64_t)1 << 28);
+  int cpb, nt;
+  const FastTuning tune = C.fast_shape(chunk, dist32 != nullptr, &cpb, &nt);
   char* ctl = (char*)P.ctl.ensure((size_t)n_chunks * 64);
   uint8_t* ovf = (uint8_t*)P.ovf.ensure(std::max<size_t>((size_t)B, 16));
   double* din[2];
@@ -1974,8 +2013,7 @@ static void fast_host_pipelined(HostCst& C, const PmTablesHdr* T, const double* 
     cuda_check(cudaMemcpyAsync(din[k], q + c0 * d, (size_t)(n * d) * 8, cudaMemcpyHostToDevice, cs), "H2D copy");
     char* cc = ctl + i * 64;
     cuda_check(launch_fast_valid(T, C.hdr, st, din[k], n, dout[k], ddist[k], 0.1f, items[k], (unsigned int*)cc, cap, ovf + c0,
-                                 (unsigned long long*)(cc + 16), C.fast_cpb, C.fast_nt, cs, hqb[k], (unsigned long long*)(cc + 48), hq_cap,
-                                 C.tune, bnd),
+                                 (unsigned long long*)(cc + 16), cpb, nt, cs, hqb[k], (unsigned long long*)(cc + 48), hq_cap, tune, bnd),
                "is_valid_fast");
     cuda_check(cudaMemcpyAsync(out + c0, dout[k], (size_t)n, cudaMemcpyDeviceToHost, cs), "D2H copy");
     if (dist32) cuda_check(cudaMemcpyAsync(dist32 + c0 * ns, ddist[k], (size_t)(n * ns) * 4, cudaMemcpyDeviceToHost, cs), "D2H copy");
@@ -2037,10 +2075,12 @@ static int fast_valid_entry(pmgpu_cst* c, const double* q, int64_t B, uint8_t* o
       dout = (uint8_t*)C.w_out.ensure(std::max<size_t>((size_t)B, 16));
       dd = dist32 ? (float*)C.w_out2.ensure(std::max<size_t>(nd, 16)) : nullptr;
     }
+    int cpb, nt;
+    const FastTuning tune = C.fast_shape(B, dd != nullptr, &cpb, &nt);
     const unsigned hq_cap = hard_query_cap(B, C.n_spheres());
     void* hq = dd ? C.f_hq.ensure((size_t)hq_cap * 32) : nullptr;
-    cuda_check(launch_fast_valid(T, C.hdr, st, dq, B, dout, dd, 0.1f, items, count, cap, ovf, dstats, C.fast_cpb, C.fast_nt, s, hq,
-                                 (unsigned long long*)(ctl + 48), hq_cap, C.tune, bnd),
+    cuda_check(launch_fast_valid(T, C.hdr, st, dq, B, dout, dd, 0.1f, items, count, cap, ovf, dstats, cpb, nt, s, hq,
+                                 (unsigned long long*)(ctl + 48), hq_cap, tune, bnd),
                "is_valid_fast");
     char* pin_out = pin ? pin + up16(nq) : nullptr;
     char* pin_dist = pin ? pin_out + up16((size_t)B) : nullptr;
@@ -2188,8 +2228,10 @@ static int fast_edges_entry(pmgpu_cst* c, const double* s1, const double* s2, in
     }
     int n_sm = 0;
     cuda_check(sm_count(&n_sm), "device attribute");
+    int cpb, nt;
+    const FastTuning tune = C.edge_shape(&cpb, &nt);
     cuda_check(launch_fast_edges(T, C.hdr, st, d1, d2, E, validator_type, dw, resolution, seq, sr, n, off, next, dout, items, count, cap,
-                                 ovf, dstats, C.edge_cpb, C.edge_nt, n_sm, s, bnd),
+                                 ovf, dstats, cpb, nt, n_sm, s, tune, bnd),
                "check_motion_fast");
     char* pin_out = pin ? pin + 2 * up16(ns_) + up16(nw) : nullptr;
     if (mem == PMGPU_MEM_HOST && E) cuda_check(cudaMemcpyAsync(pin_out, dout, (size_t)E, cudaMemcpyDeviceToHost, s), "D2H copy");

@@ -1667,10 +1667,10 @@ cudaError_t launch_fast_edges(const PmTablesHdr* T, const PmTablesHdr& h, const 
                               int64_t E, int type, const double* width, double resolution, const int16_t* seq, double* sr, int32_t* n,
                               int64_t* off, unsigned long long* next, uint8_t* out, int4* items, unsigned int* count,
                               unsigned int cap, uint8_t* overflow, unsigned long long* stats, int cpb, int nt, int n_sm, cudaStream_t s,
-                              PmLinkBounds bnd) {
+                              const FastTuning& tune, PmLinkBounds bnd) {
   if (E <= 0) return cudaSuccess;
   if (!fast_table_sizes_ok(h)) return cudaErrorInvalidConfiguration;
-  Scratch scr{items, count, cap, overflow, stats};
+  Scratch scr{items, count, cap, overflow, stats, nullptr, nullptr, 0u, tune.sphere_tile_log2};
   k_edge_setup<<<(unsigned)((E + 127) / 128), 128, 0, s>>>(s1, s2, E, h.q_dim, type, width, resolution, sr, n, out);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;

@@ -48,7 +48,8 @@ cudaError_t sm_count(int* n);
 cudaError_t upload_offsets();
 // Tuning of the fast kernels beyond the launch shape (the autotuner's other dimensions).
 struct FastTuning {
-  int sphere_tile_log2 = 0;  // log2 of the spheres per warp row of sphere tasks (0: the least for the shape)
+  int sphere_tile_log2 = -1;  // log2 of the spheres per warp row of sphere tasks (at least 32 / configurations per
+                              // block; < 0: the call's choice, or the least)
   int hq_blocks_per_sm = 4;  // k_hard_queries: blocks of 256 threads per SM
 };
 // bnd: link-position bounds of a composite constraint, decided in the same kernels (none by default).
@@ -64,7 +65,7 @@ cudaError_t launch_fast_edges(const PmTablesHdr* T, const PmTablesHdr& h, const 
                               int64_t E, int type, const double* width, double resolution, const int16_t* seq, double* sr, int32_t* n,
                               int64_t* off, unsigned long long* next, uint8_t* out, int4* items, unsigned int* count,
                               unsigned int cap, uint8_t* overflow, unsigned long long* stats, int cpb, int nt, int n_sm, cudaStream_t s,
-                              PmLinkBounds bnd = PmLinkBounds{nullptr, 0});
+                              const FastTuning& tune, PmLinkBounds bnd = PmLinkBounds{nullptr, 0});
 
 // ---- differentiable costs (k_grad.cu): FP32 forward + reverse-mode adjoint
 #define PM_GRAD_MAXQ (PM_MAX_CTRL + 8)
