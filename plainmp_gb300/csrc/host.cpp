@@ -977,6 +977,22 @@ struct HostCst {
     h.off_pairs = put(prs.data(), prs.size() * 4);
     h.off_prims = put(prims.data(), prims.size() * sizeof(PmPrim));
     h.off_clouds = put(clouds.data(), clouds.size() * sizeof(PmGridDev));
+    // slots by depth in the tree (the levels of the block FK), in slot order within a level
+    std::vector<int> depth(slots.size(), 0);
+    int n_levels = 0;
+    for (size_t i = 0; i < slots.size(); i++) {
+      depth[i] = slots[i].parent < 0 ? 0 : depth[slots[i].parent] + 1;
+      n_levels = std::max(n_levels, depth[i] + 1);
+    }
+    std::vector<int32_t> lev(1, 0), by_depth;
+    for (int d = 0; d < n_levels; d++) {
+      for (size_t i = 0; i < slots.size(); i++)
+        if (depth[i] == d) by_depth.push_back((int)i);
+      lev.push_back((int)by_depth.size());
+    }
+    lev.insert(lev.end(), by_depth.begin(), by_depth.end());
+    h.n_levels = n_levels;
+    h.off_lev = put(lev.data(), lev.size() * 4);
     const std::vector<char> img = fast_image(slots, grec, sx, sy, sz, sr, sgroup, prs, prims);
     h.img_bytes = (int64_t)img.size();
     h.off_img = put(img.data(), img.size());
@@ -1825,12 +1841,12 @@ int pmgpu_cst_is_valid(pmgpu_cst* c, const double* q, int64_t B, uint8_t* out, i
     const double* st = C.kin->d_state.as<double>();
     cudaStream_t s = as_stream(stream);
     if (mem == PMGPU_MEM_DEVICE) {
-      cuda_check(launch_is_valid64(T, st, q, B, out, s), "is_valid");
+      cuda_check(launch_is_valid64(T, C.hdr, st, q, B, out, s), "is_valid");
       return;
     }
     const double* dq = stage_in(C.w_in, q, (size_t)B * C.q_dim(), s);
     uint8_t* dout = (uint8_t*)C.w_out.ensure(std::max<size_t>((size_t)B, 16));
-    cuda_check(launch_is_valid64(T, st, dq, B, dout, s), "is_valid");
+    cuda_check(launch_is_valid64(T, C.hdr, st, dq, B, dout, s), "is_valid");
     stage_out(out, dout, (size_t)B, s);
     cuda_check(cudaStreamSynchronize(s), "is_valid");
   });
@@ -1849,13 +1865,13 @@ int pmgpu_cst_evaluate(pmgpu_cst* c, const double* q, int64_t B, double* vals, d
     cudaStream_t s = as_stream(stream);
     int m = C.cst_dim(), d = C.q_dim();
     if (mem == PMGPU_MEM_DEVICE) {
-      cuda_check(launch_evaluate64(T, st, q, B, 1, vals, jac, s), "evaluate");
+      cuda_check(launch_evaluate64(T, C.hdr, st, q, B, 1, vals, jac, s), "evaluate");
       return;
     }
     const double* dq = stage_in(C.w_in, q, (size_t)B * d, s);
     double* dv = (double*)C.w_out.ensure(std::max<size_t>((size_t)B * m * 8, 16));
     double* dj = (double*)C.w_out2.ensure(std::max<size_t>((size_t)B * m * d * 8, 16));
-    cuda_check(launch_evaluate64(T, st, dq, B, 1, dv, dj, s), "evaluate");
+    cuda_check(launch_evaluate64(T, C.hdr, st, dq, B, 1, dv, dj, s), "evaluate");
     stage_out(vals, dv, (size_t)B * m, s);
     stage_out(jac, dj, (size_t)B * m * d, s);
     cuda_check(cudaStreamSynchronize(s), "evaluate");
@@ -2139,7 +2155,7 @@ int pmgpu_check_motion(pmgpu_cst* c, const double* s1, const double* s2, int64_t
     unsigned long long* cnt = (unsigned long long*)C.w_aux.ensure(64);
     cuda_check(cudaMemsetAsync(cnt, 0, 8, s), "memset");
     if (mem == PMGPU_MEM_DEVICE) {
-      cuda_check(launch_check_motion64(T, st, s1, s2, E, validator_type, dw, resolution, seq, out, cnt, s), "check_motion");
+      cuda_check(launch_check_motion64(T, C.hdr, st, s1, s2, E, validator_type, dw, resolution, seq, out, cnt, s), "check_motion");
       if (n_checked) {
         unsigned long long h = 0;
         cuda_check(cudaMemcpyAsync(&h, cnt, 8, cudaMemcpyDeviceToHost, s), "D2H");
@@ -2151,7 +2167,7 @@ int pmgpu_check_motion(pmgpu_cst* c, const double* s1, const double* s2, int64_t
     const double* d1 = stage_in(C.w_in, s1, (size_t)E * d, s);
     const double* d2 = stage_in(C.w_in2, s2, (size_t)E * d, s);
     uint8_t* dout = (uint8_t*)C.w_out.ensure(std::max<size_t>((size_t)E, 16));
-    cuda_check(launch_check_motion64(T, st, d1, d2, E, validator_type, dw, resolution, seq, dout, cnt, s), "check_motion");
+    cuda_check(launch_check_motion64(T, C.hdr, st, d1, d2, E, validator_type, dw, resolution, seq, dout, cnt, s), "check_motion");
     stage_out(out, dout, (size_t)E, s);
     unsigned long long h = 0;
     cuda_check(cudaMemcpyAsync(&h, cnt, 8, cudaMemcpyDeviceToHost, s), "D2H");

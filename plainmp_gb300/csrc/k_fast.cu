@@ -26,6 +26,7 @@
 #include <mutex>
 #include <vector>
 
+#include "pm_clear.cuh"
 #include "pm_grad.cuh"
 #include "pm_launch.h"
 #include "pm_view.cuh"
@@ -34,12 +35,6 @@
 using namespace pmd;
 
 namespace {
-
-constexpr float kU = 5.9604645e-8f;  // 2^-24
-// Margin of an FP32 clearance: 64 units of roundoff of the magnitudes involved, plus 1 um.  The
-// error analysis of the FP32 evaluation (pose rounding, one dot product, one square root)
-// gives about 52 units for the box, the largest case.
-__device__ __forceinline__ float margin32(float mag) { return 1e-6f + 64.0f * kU * (1.0f + mag); }
 
 using PrimF = PmPrimF;
 using SphereF = PmSphereF;
@@ -75,11 +70,6 @@ struct Scratch {
                            // least, 32 / configurations per block)
   PmLinkBounds bnd = PmLinkBounds{nullptr, 0};  // a composite constraint's link-position bounds
 };
-
-__device__ __forceinline__ float3 xf(const float* P, float x, float y, float z) {  // R (row-major 9) * v + t (P[9..11])
-  return make_float3(fmaf(P[0], x, fmaf(P[1], y, fmaf(P[2], z, P[9]))), fmaf(P[3], x, fmaf(P[4], y, fmaf(P[5], z, P[10]))),
-                     fmaf(P[6], x, fmaf(P[7], y, fmaf(P[8], z, P[11]))));
-}
 
 // compute_approx_sin_cos (kinematics/algorithm.cpp:50-86) with the range reduction in FP64 and
 // the polynomial in FP32 (Horner form): within 8 units of roundoff (sin) and 12 (cos) of the FP64
@@ -219,82 +209,6 @@ __device__ __forceinline__ void fk32(const SlotF* __restrict__ S, int nsl, const
     o[17 * stride] = wq.w;
     o[18 * stride] = eq;
   }
-}
-
-// Clearance g (the reference reports a collision iff g <= 0, up to its own rounding), the
-// evaluate()-based signed distance sd (minus r) and the magnitude for the margin.
-__device__ __forceinline__ void clearance(const PrimF& P, const PmGridDev* clouds, float cx, float cy, float cz, float r, bool tiny,
-                                          float extra, float& g, float& sd, float& mag) {
-  const float dx = cx - P.pos[0], dy = cy - P.pos[1], dz = cz - P.pos[2];
-  mag = fabsf(cx) + fabsf(cy) + fabsf(cz) + P.mag;
-  switch (P.kind) {
-    case PM_SDF_BOX: {
-      float lx, ly, lz;
-      if (P.aa) {
-        lx = dx;
-        ly = dy;
-        lz = dz;
-      } else {
-        lx = fmaf(dx, P.rot[0], fmaf(dy, P.rot[3], dz * P.rot[6]));
-        ly = fmaf(dx, P.rot[1], fmaf(dy, P.rot[4], dz * P.rot[7]));
-        lz = fmaf(dx, P.rot[2], fmaf(dy, P.rot[5], dz * P.rot[8]));
-      }
-      const float sx = fabsf(lx) - P.a, sy = fabsf(ly) - P.b, sz = fabsf(lz) - P.c;
-      const float mx = fmaxf(sx, 0.f), my = fmaxf(sy, 0.f), mz = fmaxf(sz, 0.f);
-      const float ext = sqrtf(fmaf(mx, mx, fmaf(my, my, mz * mz)));
-      const float ms = fmaxf(sx, fmaxf(sy, sz));
-      g = tiny ? ms - r : ext - r;
-      sd = ext + fminf(ms, 0.f) - r;
-      return;
-    }
-    case PM_SDF_CYLINDER: {
-      float lx, ly, lz;
-      if (P.za) {
-        lx = dx;
-        ly = dy;
-        lz = dz;
-      } else {
-        lx = fmaf(dx, P.rot[0], fmaf(dy, P.rot[3], dz * P.rot[6]));
-        ly = fmaf(dx, P.rot[1], fmaf(dy, P.rot[4], dz * P.rot[7]));
-        lz = fmaf(dx, P.rot[2], fmaf(dy, P.rot[5], dz * P.rot[8]));
-      }
-      const float zs = fabsf(lz) - P.c;
-      const float rs = sqrtf(fmaf(lx, lx, ly * ly)) - P.a;
-      const float a = fmaxf(rs, 0.f), b = fmaxf(zs, 0.f);
-      const float ext = sqrtf(fmaf(a, a, b * b));
-      g = tiny ? fmaxf(zs - r, rs) : ext - r;
-      sd = ext + fminf(fmaxf(rs, zs), 0.f) - r;
-      return;
-    }
-    case PM_SDF_SPHERE: {
-      const float d = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) - P.a;
-      g = tiny ? d : d - r;
-      sd = d - r;
-      return;
-    }
-    case PM_SDF_GROUND: {  // the reference's AABB (z in [0, 0]) is part of its decision
-      g = fmaxf(fabsf(cz) - r, cz + P.a - r);
-      sd = cz + P.a - r;
-      return;
-    }
-    case PM_SDF_CLOUD: {
-      const float reach = P.a + r + extra;
-      NNResult32 nn = grid_nearest32(clouds[P.cloud], cx, cy, cz, reach * reach);
-      if (nn.idx < 0) {
-        g = reach - P.a - r;  // nothing closer than reach
-        sd = 3.0e38f;
-        mag = fabsf(cx) + fabsf(cy) + fabsf(cz);
-        return;
-      }
-      const float d = sqrtf(nn.d2);
-      g = d - P.a - r;
-      sd = g;
-      mag = fabsf(cx) + fabsf(cy) + fabsf(cz) + d;
-      return;
-    }
-  }
-  g = 3.0e38f;
-  sd = 3.0e38f;
 }
 
 // Block offsets (dx, dy, dz) with max |d| <= kOffR, sorted by the minimum distance between two

@@ -1,207 +1,580 @@
-// Plain FP64 method: one device thread per configuration (or edge), replicating the
-// reference's branch structure and early exits (constraints/primitive_sphere_collision.cpp,
-// ompl/motion_validator.cpp) with bit-identical FP64 arithmetic (compiled --fmad=false).
+// Plain FP64 method: the reference's decisions and values (constraints/primitive_sphere_collision.cpp,
+// ompl/motion_validator.cpp) in FP64, bit for bit (compiled --fmad=false), one configuration per warp or per
+// four warps (pm_team.cuh).  FP32 only skips what it clears by more than its error bound.
+#include <algorithm>
+
 #include "pm_launch.h"
-#include "pm_view.cuh"
-#include "pm_warp.cuh"
+#include "pm_team.cuh"
 
 using namespace pmd;
 
 namespace {
 
-__global__ void k_is_valid64(const PmTablesHdr* __restrict__ T, const double* __restrict__ state, const double* __restrict__ q,
-                             int64_t B, uint8_t* __restrict__ out) {
-  int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (b >= B) return;
-  TView v(T);
-  out[b] = is_valid_cfg(v, state, q + b * T->q_dim) ? 1 : 0;
+#define PM_CUTOFF 0.1
+#define PM_MAX_DOF (PM_MAX_CTRL + 6)
+
+// Collision-free validity of one configuration (is_valid_dirty, primitive_sphere_collision.cpp:181-254) by
+// the WPC warps of a team; wi: this warp's number.  Collision = OR over (group, primitive) of [gate AND OR over
+// the group's spheres of test], and likewise over pairs, so the order of the tests is free.  `failed` (shared,
+// zeroed by the caller) is set when one collides and ends the other warps' loops.
+template <int WPC>
+__device__ void valid_team(const TView& v, const Image& im, const TeamPose& P, int wi, volatile int* failed) {
+  const unsigned FULL = 0xffffffffu;
+  const PmTablesHdr* T = v.T;
+  const int lane = threadIdx.x & 31;
+  const int ng = T->n_groups, np = T->n_prims;
+  // ---- groups against primitives, then the spheres of the pairs that FP32 does not clear
+  for (int base = 32 * wi; base < ng * np; base += 32 * WPC) {  // warp-uniform
+    if (__any_sync(FULL, *failed)) return;
+    const int t = base + lane;
+    const int gi = t / np, pi = t - gi * np;
+    int n = 0;
+    if (t < ng * np) {
+      const PmGroupF& G = im.grp[gi];
+      if (!G.only_self) {
+        const PmPrimF& Q = im.prm[pi];
+        const float* R = P.at32(G.slot);
+        const float3 gc = xf(R, G.rel[0], G.rel[1], G.rel[2]);
+        float g, sd, mag;
+        if (Q.kind == PM_SDF_CLOUD) {
+          const float lb = grid_field_lb16(v.C[Q.cloud], gc.x, gc.y, gc.z);
+          g = lb - Q.a - G.radius;
+          mag = fabsf(gc.x) + fabsf(gc.y) + fabsf(gc.z) + lb;
+        } else {
+          clearance(Q, v.C, gc.x, gc.y, gc.z, G.radius, G.tiny, 0.f, g, sd, mag);
+        }
+        if (!(g > margin32(mag) + cast_error(R, G.gn))) n = G.count;
+      }
+    }
+    bool hit = false;
+    warp_spread(n, [&](int owner, int j, bool have) {
+      const int g2 = __shfl_sync(FULL, gi, owner), p2 = __shfl_sync(FULL, pi, owner);
+      const PmPrim& Q = v.P[p2];
+      const PmGroup& G = v.G[g2];
+      const int k = G.begin + j;
+      bool open = false, search = false;
+      int known = -1;
+      if (have) {
+        const PmSphereF& S = im.sph[k];
+        const float* R = P.at32(G.slot);
+        const float3 c = xf(R, S.x, S.y, S.z);
+        const float ek = cast_error(R, S.sn);
+        if (Q.kind == PM_SDF_CLOUD) {
+          const FieldLB f = grid_field32(v.C[Q.cloud], c.x, c.y, c.z);
+          search = !(f.lb - (float)Q.a - S.r > margin32(fabsf(c.x) + fabsf(c.y) + fabsf(c.z) + f.lb) + ek);
+          known = f.idx;
+        } else {
+          float g, sd, mag;
+          clearance(im.prm[p2], v.C, c.x, c.y, c.z, S.r, S.tiny, 0.f, g, sd, mag);
+          open = !(g > margin32(mag) + ek);
+        }
+      }
+      if (open) {  // FP64: gate AND test
+        const DPose lp = P.at(G.slot);
+        const DM3 R = qmat(lp.q);
+        const D3 c = add(mv(R, v.rel(k)), lp.t);
+        const double r = v.sr[k];
+        hit = !outside_aabb(Q, c, r) && !prim_outside(Q, nullptr, c, r) &&
+              gate_open(Q, add(mv(R, D3{G.rel[0], G.rel[1], G.rel[2]}), lp.t), G.radius);
+      }
+      D3 c{0, 0, 0}, gc{0, 0, 0};
+      bool gate = true;
+      if (search) {
+        const DPose lp = P.at(G.slot);
+        const DM3 R = qmat(lp.q);
+        c = add(mv(R, v.rel(k)), lp.t);
+        gc = add(mv(R, D3{G.rel[0], G.rel[1], G.rel[2]}), lp.t);
+        search = !outside_aabb(Q, c, v.sr[k]) && !outside_aabb(Q, gc, G.radius);
+        if (search && known >= 0) {
+          // a point of the cloud inside both spheres settles the search and the gate: the nearest points
+          // are no farther, and rounding is monotone
+          const PmGridDev& Gd = v.C[Q.cloud];
+          const D3 p{Gd.px[known], Gd.py[known], Gd.pz[known]};
+          const D3 d = sub(p, c), e = sub(p, gc);
+          gate = sqrt(sqn(e)) - Q.a > G.radius;
+          hit = hit || (!(sqrt(sqn(d)) - Q.a > v.sr[k]) && !gate);
+        }
+      }
+      if (__any_sync(FULL, hit)) return false;
+      for (unsigned bal = __ballot_sync(FULL, search); bal != 0; bal &= bal - 1) {  // warp-uniform
+        const int src = __ffs(bal) - 1;
+        const int ps = __shfl_sync(FULL, p2, src), ks = __shfl_sync(FULL, k, src), gs = __shfl_sync(FULL, g2, src);
+        const PmPrim& Qs = v.P[ps];
+        const D3 cs = shfl_d3(c, src), gcs = shfl_d3(gc, src);
+        const int hint = __shfl_sync(FULL, known, src);
+        int near = -1;
+        if (!cloud_outside_warp(Qs, v.C, cs, v.sr[ks], &near, hint)) {
+          const PmGridDev& Gd = v.C[Qs.cloud];
+          const D3 e = sub(D3{Gd.px[near], Gd.py[near], Gd.pz[near]}, gcs);
+          const double rg = v.G[gs].radius;
+          hit = !(sqrt(sqn(e)) - Qs.a > rg);
+          if (!hit) hit = !cloud_outside_warp(Qs, v.C, gcs, rg, nullptr);
+          if (hit) return false;
+        }
+      }
+      return true;
+    });
+    if (__any_sync(FULL, hit)) {
+      if (lane == 0) *failed = 1;
+      return;
+    }
+  }
+  // ---- self pairs: the group spheres, then the sphere pairs of the group pairs that FP32 does not clear
+  for (int base = 32 * wi; base < T->n_pairs; base += 32 * WPC) {  // warp-uniform
+    if (__any_sync(FULL, *failed)) return;
+    const int t = base + lane;
+    bool near = false;
+    int ga = 0, gb = 0;
+    if (t < T->n_pairs) {
+      ga = v.pairs[2 * t];
+      gb = v.pairs[2 * t + 1];
+      const PmGroupF &G1 = im.grp[ga], &G2 = im.grp[gb];
+      const float *R1 = P.at32(G1.slot), *R2 = P.at32(G2.slot);
+      const float3 a = xf(R1, G1.rel[0], G1.rel[1], G1.rel[2]), b = xf(R2, G2.rel[0], G2.rel[1], G2.rel[2]);
+      const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+      const float mag = fabsf(a.x) + fabsf(a.y) + fabsf(a.z) + fabsf(b.x) + fabsf(b.y) + fabsf(b.z);
+      near = !(sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) - (G1.radius + G2.radius) >
+               2.0f * margin32(mag) + cast_error(R1, G1.gn) + cast_error(R2, G2.gn));
+    }
+    for (unsigned bal = __ballot_sync(FULL, near); bal != 0; bal &= bal - 1) {  // warp-uniform
+      const int src = __ffs(bal) - 1;
+      const int a = __shfl_sync(FULL, ga, src), b = __shfl_sync(FULL, gb, src);
+      const PmGroup &G1 = v.G[a], &G2 = v.G[b];
+      const float *R1 = P.at32(G1.slot), *R2 = P.at32(G2.slot);
+      const int n = G1.count * G2.count;
+      bool hit = false;
+      for (int u = lane; u < n; u += 32) {
+        const int i = G1.begin + u / G2.count, j = G2.begin + u % G2.count;
+        const PmSphereF &S1 = im.sph[i], &S2 = im.sph[j];
+        const float3 ci = xf(R1, S1.x, S1.y, S1.z), cj = xf(R2, S2.x, S2.y, S2.z);
+        const float ex = ci.x - cj.x, ey = ci.y - cj.y, ez = ci.z - cj.z;
+        const float mag = fabsf(ci.x) + fabsf(ci.y) + fabsf(ci.z) + fabsf(cj.x) + fabsf(cj.y) + fabsf(cj.z);
+        if (sqrtf(fmaf(ex, ex, fmaf(ey, ey, ez * ez))) - (S1.r + S2.r) >
+            2.0f * margin32(mag) + cast_error(R1, S1.sn) + cast_error(R2, S2.sn))
+          continue;
+        const DPose p1 = P.at(G1.slot), p2 = P.at(G2.slot);
+        const DM3 M1 = qmat(p1.q), M2 = qmat(p2.q);
+        const D3 c1 = add(mv(M1, D3{G1.rel[0], G1.rel[1], G1.rel[2]}), p1.t), c2 = add(mv(M2, D3{G2.rel[0], G2.rel[1], G2.rel[2]}), p2.t);
+        const double ors = G1.radius + G2.radius;
+        if (sqn(sub(c1, c2)) > ors * ors) continue;
+        const double rs = v.sr[i] + v.sr[j];
+        hit = hit || sqn(sub(add(mv(M1, v.rel(i)), p1.t), add(mv(M2, v.rel(j)), p2.t))) < rs * rs;
+      }
+      if (__any_sync(FULL, hit)) {
+        if (lane == 0) *failed = 1;
+        return;
+      }
+    }
+  }
 }
 
-// get_attached_point_jacobian (algorithm.cpp:346-433); column c of the 3 x dof jacobian is
-// written to jac[3*c .. 3*c+2]
-__device__ void attached_jacobian(const TView& v, const DPose* pose, int plink_slot, const D3& p, double* jac) {
-  const int nc = v.T->n_ctrl;
-  const uint64_t rel = v.S[plink_slot].relevant;
-  for (int i = 0; i < nc; i++) {
-    double* c = jac + 3 * i;
-    const PmJoint& J = v.J[i];
-    if (J.slot < 0 || !((rel >> i) & 1ull)) {
-      c[0] = c[1] = c[2] = 0.0;
-      continue;
+// Dynamic shared memory of a block of nc configurations.
+inline size_t team_smem(const PmTablesHdr& h, int nc) { return (size_t)nc * h.n_slots * (kRec * sizeof(double) + kRec32 * sizeof(float)); }
+
+// NC configurations per block, WPC warps each; 128 registers a thread.
+template <int NC, int WPC>
+__global__ void __launch_bounds__(NC * WPC * 32, 512 / (NC * WPC * 32)) k_is_valid64(const PmTablesHdr* __restrict__ T, const double* __restrict__ state,
+                                                             const double* __restrict__ q, int64_t B, uint8_t* __restrict__ out) {
+  extern __shared__ __align__(16) double team_mem[];
+  __shared__ int failed[NC];
+  const TView v(T);
+  const Image im(T);
+  const int nsl = T->n_slots, qd = T->q_dim;
+  const int64_t c0 = (int64_t)blockIdx.x * NC;
+  const int ncfg = (int)min((int64_t)NC, B - c0);
+  if (threadIdx.x < NC) failed[threadIdx.x] = 0;
+  float* p32 = reinterpret_cast<float*>(team_mem + (size_t)NC * nsl * kRec);
+  fk64_block<NC * WPC * 32>(v, state, [&](int c, int col) { return q[(c0 + c) * qd + col]; }, ncfg, T->base_type == PM_BASE_FIXED,
+                            team_mem, p32);
+  const int c = (threadIdx.x >> 5) / WPC, wi = (threadIdx.x >> 5) % WPC;
+  if (c < ncfg) valid_team<WPC>(v, im, TeamPose{team_mem + (size_t)c * nsl * kRec, p32 + (size_t)c * nsl * kRec32}, wi, failed + c);
+  __syncthreads();
+  if (threadIdx.x < ncfg) out[c0 + threadIdx.x] = failed[threadIdx.x] ? 0 : 1;
+}
+
+// CustomValidatorBase::checkMotion (motion_validator.cpp:17-79), a block per edge: its waypoints in the
+// reference's visiting order, NC at a time, a warp each; the first round with a collision ends it.
+// n_checked counts the waypoints up to and including the first that collides, as the reference visits them.
+template <int NC>
+__global__ void __launch_bounds__(NC * 32, 512 / (NC * 32)) k_check_motion64(const PmTablesHdr* __restrict__ T, const double* __restrict__ state,
+                                                            const double* __restrict__ s1, const double* __restrict__ s2, int type,
+                                                            const double* __restrict__ width, double resolution,
+                                                            const int16_t* __restrict__ seq, uint8_t* __restrict__ out,
+                                                            unsigned long long* n_checked) {
+  extern __shared__ __align__(16) double team_mem[];
+  __shared__ int failed[NC];
+  __shared__ double step;
+  __shared__ unsigned long long n_way;  // waypoints to check (0: decided already)
+  const TView v(T);
+  const Image im(T);
+  const int64_t e = blockIdx.x;
+  const int dim = T->q_dim, nsl = T->n_slots;
+  const double* a = s1 + e * dim;
+  const double* b = s2 + e * dim;
+  if (threadIdx.x == 0) {
+    double sr;
+    if (type == 0) {  // BoxMotionValidator::determine_step_ratio (:89-111)
+      double diff_long = 0.0, max_diff = -INFINITY;
+      int li = 0;
+      for (int i = 0; i < dim; i++) {
+        double diff = b[i] - a[i];
+        double asd = fabs(diff) * (1.0 / width[i]);
+        if (asd > max_diff) {
+          max_diff = asd;
+          li = i;
+          diff_long = diff;
+        }
+      }
+      sr = fabs(diff_long) < 1e-6 ? INFINITY : width[li] / fabs(diff_long);
+    } else {  // EuclideanMotionValidator (:118-126)
+      double dist = 0.0;
+      for (int i = 0; i < dim; i++) {
+        double d = a[i] - b[i];
+        dist += d * d;
+      }
+      sr = resolution / sqrt(dist);
     }
-    const DPose& tc = pose[J.slot];
-    D3 wa = qrot(tc.q, D3{J.axis[0], J.axis[1], J.axis[2]});
-    D3 d = J.prismatic ? wa : cross(wa, sub(p, tc.t));
-    c[0] = d.x;
-    c[1] = d.y;
-    c[2] = d.z;
+    step = sr;
+    n_way = 0;
+    if (sr == INFINITY) {
+      out[e] = 1;
+    } else if (!(sr > 0.0) || 1.0 / sr > 67108864.0) {
+      // NaN / non-positive step ratios, and edges needing more than 2^26 waypoints, are reported
+      // invalid instead of looping (the reference has no bound here)
+      out[e] = 0;
+    } else {
+      n_way = (unsigned long long)(floor(1 / sr) + 1);
+    }
   }
-  if (v.T->base_type == PM_BASE_FIXED) return;
+  __syncthreads();
+  const double sr = step;
+  const unsigned long long n = n_way;
+  if (n == 0) return;  // block-uniform
+  float* p32 = reinterpret_cast<float*>(team_mem + (size_t)NC * nsl * kRec);
+  unsigned long long k0 = 0, checked = n;
+  bool ok = true;
+  for (; k0 < n && ok; k0 += NC) {  // block-uniform
+    const int ncfg = (int)min((unsigned long long)NC, n - k0);
+    if (threadIdx.x < NC) failed[threadIdx.x] = 0;
+    // waypoint k: s2 for k = 0, then the interior points in visiting order (:45-78)
+    auto qf = [&](int c, int col) {
+      const unsigned long long k = k0 + c;
+      if (k == 0) return b[col];
+      const double t = n + 1 < 129 ? (double)seq[n * 128 + (k + 1)] * sr : (double)k * sr;
+      return a[col] + (b[col] - a[col]) * t;
+    };
+    fk64_block<NC * 32>(v, state, qf, ncfg, T->base_type == PM_BASE_FIXED, team_mem, p32);
+    const int c = threadIdx.x >> 5;
+    if (c < ncfg) valid_team<1>(v, im, TeamPose{team_mem + (size_t)c * nsl * kRec, p32 + (size_t)c * nsl * kRec32}, 0, failed + c);
+    __syncthreads();
+    for (int i = 0; i < ncfg && ok; i++)
+      if (failed[i]) {
+        ok = false;
+        checked = k0 + i + 1;
+      }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    out[e] = ok ? 1 : 0;
+    if (n_checked) atomicAdd(n_checked, checked);
+  }
+}
+
+// The smallest of a warp's values and its place in the reference's order (ties go to the earlier term).
+struct Least {
+  double val;
+  unsigned long long order;
+  __device__ __forceinline__ void take(double v, unsigned long long o) {
+    if (v < val || (v == val && o < order)) {
+      val = v;
+      order = o;
+    }
+  }
+  __device__ __forceinline__ void share() {
+    for (int o = 16; o > 0; o >>= 1) {
+      const double ov = __shfl_xor_sync(0xffffffffu, val, o);
+      const unsigned long long oo = __shfl_xor_sync(0xffffffffu, order, o);
+      take(ov, oo);
+    }
+  }
+};
+constexpr unsigned long long kNoTerm = ~0ull;
+
+// Column d of get_attached_point_jacobian (algorithm.cpp:346-433) for the point p of a slot's link.
+__device__ D3 attached_column(const TView& v, const TeamPose& P, int plink_slot, const D3& p, int d) {
+  const int nc = v.T->n_ctrl;
+  if (d < nc) {
+    const PmJoint& J = v.J[d];
+    if (J.slot < 0 || !((v.S[plink_slot].relevant >> d) & 1ull)) return D3{0.0, 0.0, 0.0};
+    const DPose tc = P.at(J.slot);
+    const D3 wa = qrot(tc.q, D3{J.axis[0], J.axis[1], J.axis[2]});
+    return J.prismatic ? wa : cross(wa, sub(p, tc.t));
+  }
+  const int k = d - nc;  // FLOATING: x y z roll pitch yaw; PLANAR: x y yaw
+  const bool floating = v.T->base_type == PM_BASE_FLOATING;
+  const int n_trans = floating ? 3 : 2;
+  if (k < n_trans) return D3{k == 0 ? 1.0 : 0.0, k == 1 ? 1.0 : 0.0, k == 2 ? 1.0 : 0.0};
+  // the angle columns by the reference's forward differences
+  const double eps = 1e-7;
   DPose te;
   te.q = DQ{0, 0, 0, 1};
   te.t = p;
-  const DPose tb = pose[v.T->root_slot];
-  DPose tbinv = pose_inverse(tb);
-  D3 rpy = get_rpy(tb.q);
-  DPose tbe = pose_mul(tbinv, te);
-  const double eps = 1e-7;
-  double rpya[3] = {rpy.x, rpy.y, rpy.z};
-  if (v.T->base_type == PM_BASE_FLOATING) {
-    for (int k = 0; k < 9; k++) jac[3 * nc + k] = 0.0;
-    jac[3 * (nc + 0) + 0] = 1.0;
-    jac[3 * (nc + 1) + 1] = 1.0;
-    jac[3 * (nc + 2) + 2] = 1.0;
-    for (int k = 0; k < 3; k++) {
-      double r2[3] = {rpya[0], rpya[1], rpya[2]};
-      r2[k] += eps;
-      DPose tw = tb;
-      tw.q = quat_from_rpy(r2[0], r2[1], r2[2]);
-      DPose o = pose_mul(tw, tbe);
-      D3 dp = sub(o.t, te.t);
-      jac[3 * (nc + 3 + k) + 0] = dp.x / eps;
-      jac[3 * (nc + 3 + k) + 1] = dp.y / eps;
-      jac[3 * (nc + 3 + k) + 2] = dp.z / eps;
-    }
-  } else {
-    for (int k = 0; k < 9; k++) jac[3 * nc + k] = 0.0;
-    jac[3 * (nc + 0) + 0] = 1.0;
-    jac[3 * (nc + 1) + 1] = 1.0;
-    double r2[3] = {rpya[0], rpya[1], rpya[2] + eps};
-    DPose tw = tb;
-    tw.q = quat_from_rpy(r2[0], r2[1], r2[2]);
-    DPose o = pose_mul(tw, tbe);
-    D3 dp = sub(o.t, te.t);
-    jac[3 * (nc + 2) + 0] = dp.x / eps;
-    jac[3 * (nc + 2) + 1] = dp.y / eps;
-    jac[3 * (nc + 2) + 2] = dp.z / eps;
-  }
+  const DPose tb = P.at(v.T->root_slot);
+  const DPose tbe = pose_mul(pose_inverse(tb), te);
+  const D3 rpy = get_rpy(tb.q);
+  const int ang = floating ? k - 3 : 2;
+  DPose tw = tb;
+  tw.q = quat_from_rpy(ang == 0 ? rpy.x + eps : rpy.x, ang == 1 ? rpy.y + eps : rpy.y, ang == 2 ? rpy.z + eps : rpy.z);
+  const D3 dp = sub(pose_mul(tw, tbe).t, te.t);
+  return D3{dp.x / eps, dp.y / eps, dp.z / eps};
 }
 
-#define PM_CUTOFF 0.1
-
-// evaluate_ext_collision (primitive_sphere_collision.cpp:256-322)
-__device__ double eval_ext(const TView& v, const DPose* pose, double* grad, double* jtmp) {
-  const int dof = v.T->q_dim;
-  double minv = PM_CUTOFF;
-  int mg = -1, mp = -1, mk = -1;
-  for (int gi = 0; gi < v.T->n_groups; gi++) {
-    const PmGroup& g = v.G[gi];
-    if (g.only_self) continue;
-    const DPose& lp = pose[g.slot];
-    DM3 R;
-    D3 gc = group_centre(v, g, lp, R);
-    for (int pi = 0; pi < v.T->n_prims; pi++) {
-      const PmPrim& P = v.P[pi];
-      if (!outside_aabb(P, gc, g.radius + PM_CUTOFF)) {
-        if (!prim_outside(P, v.C, gc, g.radius + PM_CUTOFF)) {
-          for (int k = g.begin; k < g.begin + g.count; k++) {
-            D3 c = add(mv(R, v.rel(k)), lp.t);
-            if (outside_aabb(P, c, v.sr[k] + PM_CUTOFF)) continue;
-            double val = prim_eval(P, v.C, c) - v.sr[k];
-            if (val < minv) {
-              minv = val;
-              mg = gi;
-              mp = pi;
-              mk = k;
+// evaluate_ext_collision (primitive_sphere_collision.cpp:256-322) by one warp: the least value of a sphere
+// against a primitive below the cutoff, and its gradient row.  FP32 finds an upper bound of that value (each
+// term's distance plus its error; the nearest point that the field stores, for a cloud), then FP64 evaluates
+// the terms whose lower bound does not exceed it: one to three of a few hundred.
+__device__ double eval_ext_warp(const TView& v, const Image& im, const TeamPose& P, double* grad) {
+  const unsigned FULL = 0xffffffffu;
+  const PmTablesHdr* T = v.T;
+  const int lane = threadIdx.x & 31;
+  const int ng = T->n_groups, np = T->n_prims, dof = T->q_dim;
+  Least best{PM_CUTOFF, kNoTerm};
+  float upper = (float)PM_CUTOFF;  // no term above it can be the least
+  for (int pass = 0; pass < 2; pass++) {  // 0: the bound; 1: the values
+    for (int base = 0; base < ng * np; base += 32) {  // warp-uniform
+      const int t = base + lane;
+      const int gi = t / np, pi = t - gi * np;
+      int n = 0;
+      if (t < ng * np) {
+        const PmGroupF& G = im.grp[gi];
+        if (!G.only_self) {
+          const PmPrimF& Q = im.prm[pi];
+          const float* R = P.at32(G.slot);
+          const float3 gc = xf(R, G.rel[0], G.rel[1], G.rel[2]);
+          float g, sd, mag;
+          if (Q.kind == PM_SDF_CLOUD) {
+            const float lb = grid_field_lb16(v.C[Q.cloud], gc.x, gc.y, gc.z);
+            sd = g = lb - Q.a - G.radius;
+            mag = fabsf(gc.x) + fabsf(gc.y) + fabsf(gc.z) + lb;
+          } else {
+            clearance(Q, v.C, gc.x, gc.y, gc.z, G.radius, G.tiny, 0.f, g, sd, mag);
+          }
+          // sd bounds the values of the group's spheres from below: beyond the cutoff its gate is closed,
+          // beyond the bound none of them is the least.  The ground's gate tests more than the distance
+          // (g), and only the cutoff counts for it.  (g of a box or cylinder ends at -radius inside it.)
+          const bool by_gate = Q.kind == PM_SDF_GROUND;
+          if (!((by_gate ? g : sd) > (by_gate ? (float)PM_CUTOFF : upper) + margin32(mag) + cast_error(R, G.gn))) n = G.count;
+        }
+      }
+      warp_spread(n, [&](int owner, int j, bool have) {
+        const int g2 = __shfl_sync(FULL, gi, owner), p2 = __shfl_sync(FULL, pi, owner), t2 = __shfl_sync(FULL, t, owner);
+        const PmPrim& Q = v.P[p2];
+        const PmGroup& G = v.G[g2];
+        const int k = G.begin + j;
+        bool open = false, search = false;
+        int known = -1;
+        if (have) {
+          const PmSphereF& S = im.sph[k];
+          const float* R = P.at32(G.slot);
+          const float3 c = xf(R, S.x, S.y, S.z);
+          const float ek = cast_error(R, S.sn);
+          if (Q.kind == PM_SDF_CLOUD) {
+            const PmGridDev& Gd = v.C[Q.cloud];
+            const float qmag = fabsf(c.x) + fabsf(c.y) + fabsf(c.z);
+            const FieldLB f = grid_field32(Gd, c.x, c.y, c.z, true);
+            search = !(f.lb - (float)Q.a - S.r > upper + margin32(qmag + f.lb) + ek);
+            known = f.idx;
+            if (pass == 0 && f.idx >= 0) {
+              const float ex = f.np.x - c.x, ey = f.np.y - c.y, ez = f.np.z - c.z;
+              const float ub = sqrtf(fmaf(ex, ex, fmaf(ey, ey, ez * ez)));
+              upper = fminf(upper, ub - (float)Q.a - S.r + margin32(qmag + ub) + ek);
             }
+          } else {
+            float g, sd, mag;
+            clearance(im.prm[p2], v.C, c.x, c.y, c.z, S.r, S.tiny, 0.f, g, sd, mag);
+            const float m = margin32(mag) + ek;
+            open = !(sd > upper + m);
+            if (pass == 0 && Q.kind != PM_SDF_GROUND) upper = fminf(upper, sd + m);
           }
         }
-      }
-    }
-  }
-  if (mg < 0) {
-    for (int d = 0; d < dof; d++) grad[d] = 0.0;
-    return minv;
-  }
-  const PmGroup& g = v.G[mg];
-  DM3 R = qmat(pose[g.slot].q);
-  D3 sc = add(mv(R, v.rel(mk)), pose[g.slot].t);
-  double r = v.sr[mk];
-  double g3[3];
-  for (int i = 0; i < 3; i++) {
-    D3 pc = sc;
-    if (i == 0) pc.x += 1e-6;
-    if (i == 1) pc.y += 1e-6;
-    if (i == 2) pc.z += 1e-6;
-    double val = prim_eval(v.P[mp], v.C, pc) - r;
-    g3[i] = (val - minv) / 1e-6;
-  }
-  attached_jacobian(v, pose, g.slot, sc, jtmp);
-  for (int d = 0; d < dof; d++) grad[d] = jtmp[3 * d + 0] * g3[0] + jtmp[3 * d + 1] * g3[1] + jtmp[3 * d + 2] * g3[2];
-  return minv;
-}
-
-// evaluate_self_collision (primitive_sphere_collision.cpp:324-383)
-__device__ double eval_self(const TView& v, const DPose* pose, double* grad, double* jtmp, double* jtmp2) {
-  const int dof = v.T->q_dim;
-  double dmin = PM_CUTOFF;
-  int a = -1, ai = -1, b = -1, bj = -1;
-  for (int pr = 0; pr < v.T->n_pairs; pr++) {
-    const int ga = v.pairs[2 * pr], gb = v.pairs[2 * pr + 1];
-    const PmGroup& g1 = v.G[ga];
-    const PmGroup& g2 = v.G[gb];
-    DM3 R1, R2;
-    D3 c1 = group_centre(v, g1, pose[g1.slot], R1);
-    D3 c2 = group_centre(v, g2, pose[g2.slot], R2);
-    double osq = sqn(sub(c1, c2));
-    double orm = g1.radius + g2.radius + PM_CUTOFF;
-    if (osq > orm * orm) continue;
-    const D3 t1 = pose[g1.slot].t, t2 = pose[g2.slot].t;
-    for (int i = g1.begin; i < g1.begin + g1.count; i++) {
-      D3 s1 = add(mv(R1, v.rel(i)), t1);
-      for (int j = g2.begin; j < g2.begin + g2.count; j++) {
-        D3 s2 = add(mv(R2, v.rel(j)), t2);
-        double d = nrm(sub(s1, s2)) - (v.sr[i] + v.sr[j]);
-        if (d < dmin) {
-          dmin = d;
-          a = ga;
-          ai = i;
-          b = gb;
-          bj = j;
+        if (pass == 0) return true;
+        const unsigned long long order = (unsigned long long)t2 << 32 | (unsigned)k;
+        const double r = v.sr[k];
+        D3 c{0, 0, 0}, gc{0, 0, 0};
+        if (open || search) {
+          const DPose lp = P.at(G.slot);
+          const DM3 R = qmat(lp.q);
+          c = add(mv(R, v.rel(k)), lp.t);
+          gc = add(mv(R, D3{G.rel[0], G.rel[1], G.rel[2]}), lp.t);
+          const bool far = outside_aabb(Q, c, r + PM_CUTOFF) || outside_aabb(Q, gc, G.radius + PM_CUTOFF);
+          open = open && !far && !prim_outside(Q, nullptr, gc, G.radius + PM_CUTOFF);
+          search = search && !far;
+          if (open) best.take(prim_eval(Q, nullptr, c) - r, order);
         }
-      }
+        for (unsigned bal = __ballot_sync(FULL, search); bal != 0; bal &= bal - 1) {  // warp-uniform
+          const int src = __ffs(bal) - 1;
+          const int ps = __shfl_sync(FULL, p2, src), hint = __shfl_sync(FULL, known, src);
+          const PmPrim& Qs = v.P[ps];
+          const D3 cs = shfl_d3(c, src), gcs = shfl_d3(gc, src);
+          const double rs = shfl_d(r, src), rg = shfl_d(G.radius, src);
+          const unsigned long long os = __shfl_sync(FULL, order, src);
+          // only a value up to the smallest so far matters: search slightly beyond its reach
+          const double reach = ((double)upper + Qs.a + rs) * (1.0 + 1e-6) + 1e-6;
+          if (!(reach > 0.0)) continue;
+          const NNResult64 nn = warp_nearest64(v.C[Qs.cloud], cs, reach * reach, hint);
+          if (nn.idx < 0) continue;
+          const double val = sqrt(nn.d2) - Qs.a - rs;
+          // below the cutoff the gate is open, but for rounding at the cutoff itself
+          if (val > PM_CUTOFF - 1e-7 && cloud_outside_warp(Qs, v.C, gcs, rg + PM_CUTOFF, nullptr)) continue;
+          if (val < PM_CUTOFF) best.take(val, os);  // the same on every lane
+          upper = fminf(upper, (float)val + 1e-6f * (1.0f + fabsf((float)val)));
+        }
+        return true;
+      });
     }
+    if (pass == 0)
+      for (int o = 16; o > 0; o >>= 1) upper = fminf(upper, __shfl_xor_sync(FULL, upper, o));
   }
-  if (a < 0) {
-    for (int d = 0; d < dof; d++) grad[d] = 0.0;
-    return dmin;
+  if (!(best.val < PM_CUTOFF)) best = Least{PM_CUTOFF, kNoTerm};
+  best.share();
+  if (best.order == kNoTerm) {
+    for (int d = lane; d < dof; d += 32) grad[d] = 0.0;
+    return best.val;
   }
-  const PmGroup& g1 = v.G[a];
-  const PmGroup& g2 = v.G[b];
-  D3 c1 = add(mv(qmat(pose[g1.slot].q), v.rel(ai)), pose[g1.slot].t);
-  D3 c2 = add(mv(qmat(pose[g2.slot].q), v.rel(bj)), pose[g2.slot].t);
-  D3 cd = sub(c1, c2);
-  attached_jacobian(v, pose, g1.slot, c1, jtmp);
-  attached_jacobian(v, pose, g2.slot, c2, jtmp2);
-  double ni = 1.0 / nrm(cd);
-  for (int d = 0; d < dof; d++) {
-    grad[d] = cd.x * ni * (jtmp[3 * d + 0] - jtmp2[3 * d + 0]) + cd.y * ni * (jtmp[3 * d + 1] - jtmp2[3 * d + 1]) +
-              cd.z * ni * (jtmp[3 * d + 2] - jtmp2[3 * d + 2]);
+  const int t = (int)(best.order >> 32), k = (int)(best.order & 0xffffffffu);
+  const PmGroup& G = v.G[t / np];
+  const PmPrim& Q = v.P[t % np];
+  const D3 sc = P.point(G.slot, v.rel(k));
+  const double r = v.sr[k];
+  double g3[3];
+  if (Q.kind == PM_SDF_CLOUD) {
+    for (int i = 0; i < 3; i++) {
+      D3 pc = sc;
+      if (i == 0) pc.x += 1e-6;
+      if (i == 1) pc.y += 1e-6;
+      if (i == 2) pc.z += 1e-6;
+      g3[i] = ((prim_eval_warp(Q, v.C, pc) - r) - best.val) / 1e-6;
+    }
+  } else {  // a lane per axis
+    D3 pc = sc;
+    if (lane == 0) pc.x += 1e-6;
+    if (lane == 1) pc.y += 1e-6;
+    if (lane == 2) pc.z += 1e-6;
+    const double g = ((prim_eval(Q, nullptr, pc) - r) - best.val) / 1e-6;
+    for (int i = 0; i < 3; i++) g3[i] = shfl_d(g, i);
   }
-  return dmin;
+  for (int d = lane; d < dof; d += 32) {
+    const D3 j = attached_column(v, P, G.slot, sc, d);
+    grad[d] = j.x * g3[0] + j.y * g3[1] + j.z * g3[2];
+  }
+  return best.val;
 }
 
-#define PM_MAX_DOF (PM_MAX_CTRL + 6)
-
-__global__ void k_evaluate64(const PmTablesHdr* __restrict__ T, const double* __restrict__ state, const double* __restrict__ q,
-                             int64_t B, int high_accuracy, double* __restrict__ vals, double* __restrict__ jac) {
-  int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (b >= B) return;
-  TView v(T);
+// evaluate_self_collision (primitive_sphere_collision.cpp:324-383) by one warp, in the same two passes.
+__device__ double eval_self_warp(const TView& v, const Image& im, const TeamPose& P, double* grad) {
+  const unsigned FULL = 0xffffffffu;
+  const PmTablesHdr* T = v.T;
+  const int lane = threadIdx.x & 31;
   const int dof = T->q_dim;
+  Least best{PM_CUTOFF, kNoTerm};
+  float upper = (float)PM_CUTOFF;
+  for (int pass = 0; pass < 2; pass++) {
+    for (int base = 0; base < T->n_pairs; base += 32) {  // warp-uniform
+      const int t = base + lane;
+      bool near = false;
+      int ga = 0, gb = 0;
+      if (t < T->n_pairs) {
+        ga = v.pairs[2 * t];
+        gb = v.pairs[2 * t + 1];
+        const PmGroupF &G1 = im.grp[ga], &G2 = im.grp[gb];
+        const float *R1 = P.at32(G1.slot), *R2 = P.at32(G2.slot);
+        const float3 a = xf(R1, G1.rel[0], G1.rel[1], G1.rel[2]), b = xf(R2, G2.rel[0], G2.rel[1], G2.rel[2]);
+        const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+        const float mag = fabsf(a.x) + fabsf(a.y) + fabsf(a.z) + fabsf(b.x) + fabsf(b.y) + fabsf(b.z);
+        near = !(sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) - (G1.radius + G2.radius) >
+                 upper + 2.0f * margin32(mag) + cast_error(R1, G1.gn) + cast_error(R2, G2.gn));
+      }
+      for (unsigned bal = __ballot_sync(FULL, near); bal != 0; bal &= bal - 1) {  // warp-uniform
+        const int src = __ffs(bal) - 1;
+        const int a = __shfl_sync(FULL, ga, src), b = __shfl_sync(FULL, gb, src);
+        const PmGroup &G1 = v.G[a], &G2 = v.G[b];
+        const float *R1 = P.at32(G1.slot), *R2 = P.at32(G2.slot);
+        const int n = G1.count * G2.count;
+        for (int u = lane; u < n; u += 32) {
+          const int i = G1.begin + u / G2.count, j = G2.begin + u % G2.count;
+          const PmSphereF &S1 = im.sph[i], &S2 = im.sph[j];
+          const float3 ci = xf(R1, S1.x, S1.y, S1.z), cj = xf(R2, S2.x, S2.y, S2.z);
+          const float ex = ci.x - cj.x, ey = ci.y - cj.y, ez = ci.z - cj.z;
+          const float mag = fabsf(ci.x) + fabsf(ci.y) + fabsf(ci.z) + fabsf(cj.x) + fabsf(cj.y) + fabsf(cj.z);
+          const float d32 = sqrtf(fmaf(ex, ex, fmaf(ey, ey, ez * ez))) - (S1.r + S2.r);
+          const float m = 2.0f * margin32(mag) + cast_error(R1, S1.sn) + cast_error(R2, S2.sn);
+          if (pass == 0) {
+            upper = fminf(upper, d32 + m);
+            continue;
+          }
+          if (d32 > upper + m) continue;
+          const DPose p1 = P.at(G1.slot), p2 = P.at(G2.slot);
+          const DM3 M1 = qmat(p1.q), M2 = qmat(p2.q);
+          const D3 c1 = add(mv(M1, D3{G1.rel[0], G1.rel[1], G1.rel[2]}), p1.t);
+          const D3 c2 = add(mv(M2, D3{G2.rel[0], G2.rel[1], G2.rel[2]}), p2.t);
+          const double orm = G1.radius + G2.radius + PM_CUTOFF;
+          if (sqn(sub(c1, c2)) > orm * orm) continue;
+          const double d = nrm(sub(add(mv(M1, v.rel(i)), p1.t), add(mv(M2, v.rel(j)), p2.t))) - (v.sr[i] + v.sr[j]);
+          if (d < PM_CUTOFF) best.take(d, (unsigned long long)(base + src) << 42 | (unsigned long long)(i - G1.begin) << 21 | (unsigned)(j - G2.begin));
+        }
+        __syncwarp();
+      }
+    }
+    if (pass == 0)
+      for (int o = 16; o > 0; o >>= 1) upper = fminf(upper, __shfl_xor_sync(FULL, upper, o));
+  }
+  best.share();
+  if (best.order == kNoTerm) {
+    for (int d = lane; d < dof; d += 32) grad[d] = 0.0;
+    return best.val;
+  }
+  const int pr = (int)(best.order >> 42);
+  const PmGroup &G1 = v.G[v.pairs[2 * pr]], &G2 = v.G[v.pairs[2 * pr + 1]];
+  const int i = G1.begin + (int)(best.order >> 21 & 0x1fffffu), j = G2.begin + (int)(best.order & 0x1fffffu);
+  const D3 c1 = P.point(G1.slot, v.rel(i)), c2 = P.point(G2.slot, v.rel(j));
+  const D3 cd = sub(c1, c2);
+  const double ni = 1.0 / nrm(cd);
+  for (int d = lane; d < dof; d += 32) {
+    const D3 a = attached_column(v, P, G1.slot, c1, d), b = attached_column(v, P, G2.slot, c2, d);
+    grad[d] = cd.x * ni * (a.x - b.x) + cd.y * ni * (a.y - b.y) + cd.z * ni * (a.z - b.z);
+  }
+  return best.val;
+}
+
+// NC configurations per block, a warp each.
+template <int NC>
+__global__ void __launch_bounds__(NC * 32, 512 / (NC * 32)) k_evaluate64(const PmTablesHdr* __restrict__ T, const double* __restrict__ state,
+                                                        const double* __restrict__ q, int64_t B, int high_accuracy,
+                                                        double* __restrict__ vals, double* __restrict__ jac) {
+  extern __shared__ __align__(16) double team_mem[];
+  const TView v(T);
+  const Image im(T);
+  const int nsl = T->n_slots, qd = T->q_dim;
+  const int64_t c0 = (int64_t)blockIdx.x * NC;
+  const int ncfg = (int)min((int64_t)NC, B - c0);
+  float* p32 = reinterpret_cast<float*>(team_mem + (size_t)NC * nsl * kRec);
+  fk64_block<NC * 32>(v, state, [&](int c, int col) { return q[(c0 + c) * qd + col]; }, ncfg, !high_accuracy, team_mem, p32);
+  const int c = threadIdx.x >> 5;
+  if (c >= ncfg) return;
+  const TeamPose P{team_mem + (size_t)c * nsl * kRec, p32 + (size_t)c * nsl * kRec32};
   const int m = (T->n_prims > 0 ? 1 : 0) + (T->n_pairs > 0 ? 1 : 0);
-  DPose pose[PM_MAX_SLOTS];
-  double jtmp[3 * PM_MAX_DOF], jtmp2[3 * PM_MAX_DOF];
-  const double* qb = q + b * dof;
-  fk64(T, state, qb, !high_accuracy, pose);
-  double* vb = vals + b * m;
-  double* jb = jac + b * (int64_t)m * dof;
+  double* vb = vals + (c0 + c) * m;
+  double* jb = jac + (c0 + c) * (int64_t)m * qd;
   int head = 0;
   if (T->n_prims > 0) {
-    vb[head] = eval_ext(v, pose, jb + head * dof, jtmp);
+    const double val = eval_ext_warp(v, im, P, jb);
+    if ((threadIdx.x & 31) == 0) vb[0] = val;
     head++;
   }
-  if (T->n_pairs > 0) vb[head] = eval_self(v, pose, jb + head * dof, jtmp, jtmp2);
+  if (T->n_pairs > 0) {
+    const double val = eval_self_warp(v, im, P, jb + head * qd);
+    if ((threadIdx.x & 31) == 0) vb[head] = val;
+  }
 }
 
 // Per-sphere signed distances in two launches: the FP64 sphere centres (one thread per configuration:
@@ -279,76 +652,6 @@ __global__ void k_spheres_of_state(const PmTablesHdr* __restrict__ T, const doub
       out4[4 * k + 3] = v.sr[s];
     }
   }
-}
-
-// ------------------------------------------------------------------ motion validator
-// CustomValidatorBase::checkMotion (motion_validator.cpp:17-79), one thread per edge
-__global__ void k_check_motion64(const PmTablesHdr* __restrict__ T, const double* __restrict__ state, const double* __restrict__ s1,
-                                 const double* __restrict__ s2, int64_t E, int type, const double* __restrict__ width,
-                                 double resolution, const int16_t* __restrict__ seq, uint8_t* __restrict__ out,
-                                 unsigned long long* n_checked) {
-  int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= E) return;
-  TView v(T);
-  const int dim = T->q_dim;
-  const double* a = s1 + e * dim;
-  const double* b = s2 + e * dim;
-  double sr;
-  if (type == 0) {  // BoxMotionValidator::determine_step_ratio (:89-111)
-    double diff_long = 0.0, max_diff = -INFINITY;
-    int li = 0;
-    for (int i = 0; i < dim; i++) {
-      double diff = b[i] - a[i];
-      double asd = fabs(diff) * (1.0 / width[i]);
-      if (asd > max_diff) {
-        max_diff = asd;
-        li = i;
-        diff_long = diff;
-      }
-    }
-    sr = fabs(diff_long) < 1e-6 ? INFINITY : width[li] / fabs(diff_long);
-  } else {  // EuclideanMotionValidator (:118-126)
-    double dist = 0.0;
-    for (int i = 0; i < dim; i++) {
-      double d = a[i] - b[i];
-      dist += d * d;
-    }
-    sr = resolution / sqrt(dist);
-  }
-  if (sr == INFINITY) {
-    out[e] = 1;
-    return;
-  }
-  // NaN / non-positive step ratios, and edges needing more than 2^26 waypoints, are reported
-  // invalid instead of looping (the reference has no bound here)
-  if (!(sr > 0.0) || 1.0 / sr > 67108864.0) {
-    out[e] = 0;
-    return;
-  }
-  unsigned long long n_test = (unsigned long long)(floor(1 / sr) + 2);
-  double qt[PM_MAX_DOF];
-  unsigned long long cnt = 1;
-  bool ok = is_valid_cfg(v, state, b);
-  if (ok) {
-    if (n_test < 129) {
-      const int16_t* sq = seq + (n_test - 1) * 128;
-      for (unsigned long long i = 2; i < n_test && ok; i++) {
-        double t = (double)sq[i] * sr;
-        for (int k = 0; k < dim; k++) qt[k] = a[k] + (b[k] - a[k]) * t;
-        cnt++;
-        ok = is_valid_cfg(v, state, qt);
-      }
-    } else {
-      for (unsigned long long i = 1; i < n_test - 1 && ok; i++) {
-        double t = (double)i * sr;
-        for (int k = 0; k < dim; k++) qt[k] = a[k] + (b[k] - a[k]) * t;
-        cnt++;
-        ok = is_valid_cfg(v, state, qt);
-      }
-    }
-  }
-  out[e] = ok ? 1 : 0;
-  if (n_checked) atomicAdd(n_checked, cnt);
 }
 
 // ------------------------------------------------------------------ model state
@@ -465,6 +768,18 @@ __global__ void __launch_bounds__(256) k_cloud_nearest(const PmGridDev* __restri
 
 inline unsigned grid_for(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
+// Launches a kernel of nc configurations per block, wpc warps each.
+template <class K, class... A>
+cudaError_t team_launch(K kern, int64_t blocks, int nc, int wpc, const PmTablesHdr& h, cudaStream_t s, A... args) {
+  const size_t sm = team_smem(h, nc);
+  if (sm > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+  }
+  kern<<<(unsigned)blocks, nc * wpc * 32, sm, s>>>(args...);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 namespace pmg {
@@ -483,19 +798,28 @@ cudaError_t launch_link_poses(const double* state, const int32_t* parents, const
   k_link_poses<<<grid_for(n, 64), 64, 0, s>>>(state, parents, links, n, out7);
   return cudaGetLastError();
 }
-cudaError_t launch_is_valid64(const PmTablesHdr* T, const double* state, const double* q, int64_t B, uint8_t* out,
-                              cudaStream_t s) {
+cudaError_t launch_is_valid64(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* q, int64_t B,
+                              uint8_t* out, cudaStream_t s) {
   if (B <= 0) return cudaSuccess;
+  int n_sm = 0;
+  cudaError_t e = sm_count(&n_sm);
+  if (e != cudaSuccess) return e;
   prof_begin("k_is_valid64", s);
-  k_is_valid64<<<grid_for(B, 128), 128, 0, s>>>(T, state, q, B, out);
+  if (B <= 4 * (int64_t)n_sm)
+    e = team_launch(k_is_valid64<1, 4>, B, 1, 4, h, s, T, state, q, B, out);
+  else
+    e = team_launch(k_is_valid64<8, 1>, (B + 7) / 8, 8, 1, h, s, T, state, q, B, out);
   prof_end("k_is_valid64", s);
-  return cudaGetLastError();
+  return e;
 }
-cudaError_t launch_evaluate64(const PmTablesHdr* T, const double* state, const double* q, int64_t B, int high_accuracy,
-                              double* vals, double* jac, cudaStream_t s) {
+cudaError_t launch_evaluate64(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* q, int64_t B,
+                              int high_accuracy, double* vals, double* jac, cudaStream_t s) {
   if (B <= 0) return cudaSuccess;
-  k_evaluate64<<<grid_for(B, 64), 64, 0, s>>>(T, state, q, B, high_accuracy, vals, jac);
-  return cudaGetLastError();
+  int n_sm = 0;
+  const cudaError_t e = sm_count(&n_sm);
+  if (e != cudaSuccess) return e;
+  if (B <= 4 * (int64_t)n_sm) return team_launch(k_evaluate64<1>, B, 1, 1, h, s, T, state, q, B, high_accuracy, vals, jac);
+  return team_launch(k_evaluate64<4>, (B + 3) / 4, 4, 1, h, s, T, state, q, B, high_accuracy, vals, jac);
 }
 cudaError_t launch_sphere_dist64(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* q, int64_t B,
                                  int high_accuracy, double* dist, double* centres, cudaStream_t s) {
@@ -514,12 +838,15 @@ cudaError_t launch_spheres_of_state(const PmTablesHdr* T, const double* state, i
   k_spheres_of_state<<<1, 1, 0, s>>>(T, state, groups, out4);
   return cudaGetLastError();
 }
-cudaError_t launch_check_motion64(const PmTablesHdr* T, const double* state, const double* s1, const double* s2, int64_t E,
-                                  int type, const double* width, double resolution, const int16_t* seq, uint8_t* out,
-                                  unsigned long long* n_checked, cudaStream_t s) {
+cudaError_t launch_check_motion64(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* s1,
+                                  const double* s2, int64_t E, int type, const double* width, double resolution,
+                                  const int16_t* seq, uint8_t* out, unsigned long long* n_checked, cudaStream_t s) {
   if (E <= 0) return cudaSuccess;
-  k_check_motion64<<<grid_for(E, 64), 64, 0, s>>>(T, state, s1, s2, E, type, width, resolution, seq, out, n_checked);
-  return cudaGetLastError();
+  int n_sm = 0;
+  cudaError_t e = sm_count(&n_sm);
+  if (e != cudaSuccess) return e;
+  if (E <= n_sm) return team_launch(k_check_motion64<16>, E, 16, 1, h, s, T, state, s1, s2, type, width, resolution, seq, out, n_checked);
+  return team_launch(k_check_motion64<8>, E, 8, 1, h, s, T, state, s1, s2, type, width, resolution, seq, out, n_checked);
 }
 cudaError_t launch_sdf_points(const PmPrim* prims, int n_prims, const PmGridDev* clouds, int n_clouds, int is_union,
                               const double* pts, const double* radii, int64_t n, double* eval_out, uint8_t* outside_out, cudaStream_t s) {

@@ -24,19 +24,19 @@ cudaError_t launch_link_poses(const double* state, const int32_t* parents, const
                               cudaStream_t s);
 
 // ---- constraint batches (k_plain.cu)
-cudaError_t launch_is_valid64(const PmTablesHdr* T, const double* state, const double* q, int64_t B, uint8_t* out,
-                              cudaStream_t s);
-cudaError_t launch_evaluate64(const PmTablesHdr* T, const double* state, const double* q, int64_t B, int high_accuracy,
-                              double* vals, double* jac, cudaStream_t s);
+cudaError_t launch_is_valid64(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* q, int64_t B,
+                              uint8_t* out, cudaStream_t s);
+cudaError_t launch_evaluate64(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* q, int64_t B,
+                              int high_accuracy, double* vals, double* jac, cudaStream_t s);
 // centres (B x n_spheres x 3) is required: the distances are computed from it
 cudaError_t launch_sphere_dist64(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* q, int64_t B,
                                  int high_accuracy, double* dist, double* centres, cudaStream_t s);
 // spheres (all: groups=0, group spheres: groups=1) of the current state, out4 n x 4
 cudaError_t launch_spheres_of_state(const PmTablesHdr* T, const double* state, int groups, double* out4, cudaStream_t s);
 // checkMotion over E edges; seq: 128 x 128 int16 sequence table; width: q_dim (box) or NULL
-cudaError_t launch_check_motion64(const PmTablesHdr* T, const double* state, const double* s1, const double* s2, int64_t E,
-                                  int type, const double* width, double resolution, const int16_t* seq, uint8_t* out,
-                                  unsigned long long* n_checked, cudaStream_t s);
+cudaError_t launch_check_motion64(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* s1,
+                                  const double* s2, int64_t E, int type, const double* width, double resolution,
+                                  const int16_t* seq, uint8_t* out, unsigned long long* n_checked, cudaStream_t s);
 
 // ---- fast path (k_fast.cu): FP32 decisions + FP64 recheck of uncertain terms.
 size_t fast_smem_bytes(const PmTablesHdr& h, int cpb, bool want_dist);
