@@ -186,6 +186,14 @@ def f64(a, shape=None) -> np.ndarray:
     return out
 
 
+def _torch_dtype(torch, dtype):
+    if dtype is np.float64:
+        return torch.float64
+    if dtype is np.float32:
+        return torch.float32
+    return {np.uint8: torch.uint8, np.int64: torch.int64}[dtype]
+
+
 class Batch:
     """Normalises a batch argument: a numpy array (host memory) or a torch CUDA tensor
     (device memory, enqueued on torch's current stream)."""
@@ -205,12 +213,12 @@ class Batch:
             if x.device.index != cur:  # the library's kernels run on the current device
                 raise ValueError(f"the batch is on {x.device} but the current CUDA device is cuda:{cur}: "
                                  "select its device first (torch.cuda.set_device)")
-            tdt = {np.float64: self.torch.float64, np.float32: self.torch.float32, np.uint8: self.torch.uint8,
-                   np.int64: self.torch.int64}[dtype]
-            self.keep = x.detach().to(tdt).contiguous()
+            tdt = _torch_dtype(self.torch, dtype)
+            x = x.detach()
+            self.keep = x if x.dtype is tdt and x.is_contiguous() else x.to(tdt).contiguous()
             self.mem = MEM_DEVICE
             self.ptr = C.c_void_p(self.keep.data_ptr())
-            self.stream = C.c_void_p(self.torch.cuda.current_stream(self.keep.device).cuda_stream)
+            self.stream = C.c_void_p(self.torch.cuda.current_stream(cur).cuda_stream)
             self.shape = tuple(self.keep.shape)
         else:
             if self.torch is not None and isinstance(x, self.torch.Tensor):
@@ -229,8 +237,7 @@ class Batch:
         would be overrun."""
         shape = tuple(int(x) for x in shape)
         if self.mem == MEM_DEVICE:
-            tdt = {np.float64: self.torch.float64, np.float32: self.torch.float32, np.uint8: self.torch.uint8,
-                   np.int64: self.torch.int64}[dtype]
+            tdt = _torch_dtype(self.torch, dtype)
             ok = (isinstance(buf, self.torch.Tensor) and buf.is_cuda and buf.device == self.keep.device and buf.dtype == tdt
                   and buf.is_contiguous() and tuple(buf.shape) == shape)
             if not ok:
@@ -249,8 +256,7 @@ class Batch:
     def empty(self, shape, dtype):
         """An output buffer in the same memory space."""
         if self.mem == MEM_DEVICE:
-            tdt = {np.float64: self.torch.float64, np.float32: self.torch.float32, np.uint8: self.torch.uint8,
-                   np.int64: self.torch.int64}[dtype]
+            tdt = _torch_dtype(self.torch, dtype)
             t = self.torch.empty(shape, dtype=tdt, device=self.keep.device)
             return t, C.c_void_p(t.data_ptr())
         a = np.empty(shape, dtype=dtype)

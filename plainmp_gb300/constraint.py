@@ -74,6 +74,7 @@ class SphereCollisionCst(IneqConstraintBase):
             len(selcol_pairs), cstrs([a for a, _ in selcol_pairs]), cstrs([b for _, b in selcol_pairs]),
             fixed_sdf._h if fixed_sdf is not None else None, int(bool(reorder_spheres)), C.byref(h)))
         self._h = h
+        self._q_dim, _, self._n_spheres, self._n_groups = self._dims()  # fixed from here on
 
     def __del__(self):
         h = getattr(self, "_h", None)
@@ -88,18 +89,18 @@ class SphereCollisionCst(IneqConstraintBase):
         return a.value, b.value, c.value, d.value
 
     def q_dim(self) -> int:
-        return self._dims()[0]
+        return self._q_dim
 
     def cst_dim(self) -> int:
         return self._dims()[1]
 
     @property
     def n_spheres(self) -> int:
-        return self._dims()[2]
+        return self._n_spheres
 
     @property
     def n_groups(self) -> int:
-        return self._dims()[3]
+        return self._n_groups
 
     def groups(self) -> dict:
         """Constructed group table (post-reorder order)."""

@@ -3,8 +3,9 @@
 The forward value and the gradient come from the library's FP32 kernels (include/pmgpu.h,
 "differentiable costs"); the gradient is a hand-written reverse-mode adjoint through the FK
 chain and the SDF, not autograd.  ``IKCost`` and ``TrajectoryCost`` wrap them as
-``torch.autograd.Function``s: the forward pass evaluates the cost only and the backward pass
-recomputes FK and runs the adjoint, so nothing per link or per waypoint is kept between the two.
+``torch.autograd.Function``s: where q needs a gradient, the forward pass runs the cost and its adjoint
+in one launch and keeps the gradient (one row per configuration, the size of q; no transforms), and the
+backward pass scales it.  Otherwise the forward pass evaluates the cost only.
 
 Terms (all FP32):
     d_s       min over primitives of SDF.evaluate(c_s) - r_s (the SphereCollisionCst ext-row
@@ -85,12 +86,13 @@ def ik_cost_grad(cst, q, target=None, pose_link=None, want_grad: bool = True, **
     """Cost (B,) and, if want_grad, its gradient (B, q_dim) for a batch of configurations.
     q and target are numpy arrays (host) or CUDA tensors (device, torch's current stream)."""
     b = Batch(q, np.float32)
-    if len(b.shape) != 2 or b.shape[1] != cst.q_dim():
-        raise ValueError(f"q must be (B, {cst.q_dim()}), got {b.shape}")
+    qd = cst.q_dim()
+    if len(b.shape) != 2 or b.shape[1] != qd:
+        raise ValueError(f"q must be (B, {qd}), got {b.shape}")
     tb, tp = _pair(b, target)
     p, keep = make_params(cst, pose_link=pose_link, **weights)
     cost, cp = b.empty((b.shape[0],), np.float32)
-    grad, gp = b.empty((b.shape[0], cst.q_dim()), np.float32) if want_grad else (None, None)
+    grad, gp = b.empty((b.shape[0], qd), np.float32) if want_grad else (None, None)
     check(lib.pmgpu_ik_cost(cst._h, C.byref(p), b.ptr, tp, b.shape[0], cp, gp, b.mem, b.stream))
     del keep, tb
     return (cost, grad) if want_grad else cost
@@ -177,14 +179,17 @@ class IKCost:
             class _F(torch.autograd.Function):
                 @staticmethod
                 def forward(ctx, q, target, cst, pose_link, weights):
-                    ctx.cst, ctx.pose_link, ctx.weights = cst, pose_link, weights
-                    ctx.save_for_backward(q, target)
-                    return ik_cost_grad(cst, q, target, pose_link, want_grad=False, **weights)
+                    if not ctx.needs_input_grad[0]:
+                        return ik_cost_grad(cst, q, target, pose_link, want_grad=False, **weights)
+                    cost, grad = ik_cost_grad(cst, q, target, pose_link, want_grad=True, **weights)
+                    ctx.save_for_backward(q, target, grad)  # q and target: a change in place is an error
+                    return cost
 
                 @staticmethod
                 def backward(ctx, g):
-                    q, target = ctx.saved_tensors
-                    _, grad = ik_cost_grad(ctx.cst, q, target, ctx.pose_link, want_grad=True, **ctx.weights)
+                    if not ctx.needs_input_grad[0]:
+                        return None, None, None, None, None
+                    q, _, grad = ctx.saved_tensors
                     return (g[:, None] * grad).to(q.dtype), None, None, None, None
 
             cls._fn = _F
@@ -193,7 +198,7 @@ class IKCost:
 
 class TrajectoryCost:
     """torch.autograd.Function: per-trajectory cost (n_traj,) of back-to-back waypoints q
-    (n_waypoints, q_dim) with offsets (n_traj + 1); FK is recomputed in the backward pass."""
+    (n_waypoints, q_dim) with offsets (n_traj + 1)."""
 
     _fn = None
 
@@ -205,14 +210,17 @@ class TrajectoryCost:
             class _F(torch.autograd.Function):
                 @staticmethod
                 def forward(ctx, q, offsets, cst, weights):
-                    ctx.cst, ctx.weights = cst, weights
-                    ctx.save_for_backward(q, offsets)
-                    return traj_cost_grad(cst, q, offsets, want_grad=False, **dict(weights))
+                    if not ctx.needs_input_grad[0]:
+                        return traj_cost_grad(cst, q, offsets, want_grad=False, **dict(weights))
+                    cost, grad = traj_cost_grad(cst, q, offsets, want_grad=True, **dict(weights))
+                    ctx.save_for_backward(q, offsets, grad)
+                    return cost
 
                 @staticmethod
                 def backward(ctx, g):
-                    q, offsets = ctx.saved_tensors
-                    _, grad = traj_cost_grad(ctx.cst, q, offsets, want_grad=True, **dict(ctx.weights))
+                    if not ctx.needs_input_grad[0]:
+                        return None, None, None, None
+                    q, offsets, grad = ctx.saved_tensors
                     # d cost_i / d q_u for u in trajectory i: scale each waypoint row by g[i]
                     counts = offsets[1:] - offsets[:-1]
                     scale = torch.repeat_interleave(g, counts, output_size=q.shape[0])

@@ -52,9 +52,9 @@ class KinematicModel:
         return [int(v) for v in out]
 
     def get_link_ids(self, link_names: Sequence[str]) -> List[int]:
-        out = np.empty(len(link_names), dtype=np.int64)
-        check(lib.pmgpu_model_get_link_ids(self._h, cstrs(link_names), len(link_names), out.ctypes.data_as(C.POINTER(C.c_int64))))
-        return [int(v) for v in out]
+        out = (C.c_int64 * max(len(link_names), 1))()
+        check(lib.pmgpu_model_get_link_ids(self._h, cstrs(link_names), len(link_names), out))
+        return out[: len(link_names)]
 
     def get_joint_position_limits(self, joint_ids: Sequence[int]) -> List[Tuple[float, float]]:
         ids = np.asarray(joint_ids, dtype=np.int64)
