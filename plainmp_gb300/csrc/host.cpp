@@ -977,7 +977,7 @@ struct HostCst {
     h.off_pairs = put(prs.data(), prs.size() * 4);
     h.off_prims = put(prims.data(), prims.size() * sizeof(PmPrim));
     h.off_clouds = put(clouds.data(), clouds.size() * sizeof(PmGridDev));
-    // slots by depth in the tree (the levels of the block FK), in slot order within a level
+    // slots by depth in the tree (the levels of the FP64 FK), in slot order within a level: slot | parent << 16
     std::vector<int> depth(slots.size(), 0);
     int n_levels = 0;
     for (size_t i = 0; i < slots.size(); i++) {
@@ -987,7 +987,7 @@ struct HostCst {
     std::vector<int32_t> lev(1, 0), by_depth;
     for (int d = 0; d < n_levels; d++) {
       for (size_t i = 0; i < slots.size(); i++)
-        if (depth[i] == d) by_depth.push_back((int)i);
+        if (depth[i] == d) by_depth.push_back((int)i | (std::max(slots[i].parent, 0) << 16));
       lev.push_back((int)by_depth.size());
     }
     lev.insert(lev.end(), by_depth.begin(), by_depth.end());

@@ -29,8 +29,7 @@
 #include "pm_clear.cuh"
 #include "pm_grad.cuh"
 #include "pm_launch.h"
-#include "pm_view.cuh"
-#include "pm_warp.cuh"
+#include "pm_team.cuh"
 
 using namespace pmd;
 
@@ -613,6 +612,9 @@ struct CfgSource {  // a batch of configurations q[B x q_dim]
   uint8_t* out;
   PmLinkBounds bnd;  // link-position bounds checked with the collision terms (composite constraint)
   __device__ const double* cfg(const PmTablesHdr* T, int64_t i, double*) const { return q + i * T->q_dim; }
+  // one value of a configuration (locate: what a source needs to find out once per configuration)
+  __device__ int locate(int64_t) const { return 0; }
+  __device__ double value(const PmTablesHdr* T, int, int64_t i, int col) const { return q[i * T->q_dim + col]; }
   __device__ bool pre_skip(int64_t) const { return false; }     // before the fast pass: nothing known
   __device__ bool skip(int64_t i) const { return out[i] == 0; }  // after it: already invalid
   __device__ void fail(int64_t i) const { out[i] = 0; }
@@ -645,6 +647,25 @@ struct EdgeSource {
     }
     return lo;
   }
+  // position of waypoint k of edge e, and of waypoint w with its edge
+  __device__ double step(int64_t e, int64_t k) const {
+    const double r = sr[e];
+    const unsigned long long n_test = (unsigned long long)n[e] + 1;  // floor(1 / r) + 2, from k_edge_setup
+    return n_test < 129 ? (double)seq[(n_test - 1) * 128 + (k + 1)] * r : (double)k * r;
+  }
+  struct Where {
+    int64_t e;
+    bool end;
+    double t;
+  };
+  __device__ Where locate(int64_t w) const {
+    const int64_t e = edge_of(w), k = w - off[e];
+    return Where{e, k == 0, k == 0 ? 0.0 : step(e, k)};
+  }
+  __device__ double value(const PmTablesHdr* T, const Where& p, int64_t, int col) const {
+    const double a = s1[p.e * T->q_dim + col], b = s2[p.e * T->q_dim + col];
+    return p.end ? b : a + (b - a) * p.t;
+  }
   __device__ const double* cfg(const PmTablesHdr* T, int64_t w, double* buf) const {
     const int64_t e = edge_of(w);
     const int64_t k = w - off[e];
@@ -652,14 +673,7 @@ struct EdgeSource {
     const double* a = s1 + e * d;
     const double* b = s2 + e * d;
     if (k == 0) return b;
-    const double r = sr[e];
-    const unsigned long long n_test = (unsigned long long)n[e] + 1;  // floor(1 / r) + 2, from k_edge_setup
-    double t;
-    if (n_test < 129) {
-      t = (double)seq[(n_test - 1) * 128 + (k + 1)] * r;
-    } else {
-      t = (double)k * r;
-    }
+    const double t = step(e, k);
     for (int i = 0; i < d; i++) buf[i] = a[i] + (b[i] - a[i]) * t;
     return buf;
   }
@@ -1281,74 +1295,77 @@ __global__ void __launch_bounds__(256, 4) k_hard_queries(const PmTablesHdr* __re
 }
 
 // Exact FP64 evaluation of the queued terms, and full plain checks of the configurations (or
-// edges) whose terms overflowed the queue.
+// edges) whose terms overflowed the queue.  A warp per term; few terms reach FP64 (15 to 100 of 65,536
+// configurations), so the kernel's time is the latency of one: the FK runs level by level in shared memory,
+// four lanes per slot (fk64_levels), and a block is one warp, so that up to a term per SM no two share an
+// SM's FP64 pipe (16 cycles a warp instruction, however few lanes).
+constexpr int kRecheckWarps = 1;
 template <class Src>
-__global__ void k_fast_recheck(const PmTablesHdr* __restrict__ T, const double* __restrict__ state, Src src, Scratch scr) {
+__global__ void __launch_bounds__(32 * kRecheckWarps) k_fast_recheck(const PmTablesHdr* __restrict__ T, const double* __restrict__ state,
+                                                                     Src src, Scratch scr) {
+  extern __shared__ __align__(16) double recheck_rec[];  // [warp][n_slots][kRec]
   TView v(T);
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned int n_items = min(*scr.count, scr.cap);
-  double qbuf[PM_MAX_SLOTS + 8];
-  // queued terms, one warp per term: lane 0 runs the FP64 FK and the primitive tests, the warp
-  // runs the cloud searches
+  double* rec = recheck_rec + (size_t)(threadIdx.x >> 5) * T->n_slots * kRec;
+  const TeamPose P{rec, nullptr};
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t i = warp; i < (int64_t)n_items; i += n_warps) {
     const int4 it = scr.items[i];
     if (__shfl_sync(FULL, src.skip(it.x) ? 1 : 0, 0)) continue;
+    __syncwarp();  // the last term's readers of rec are done
+    const auto where = src.locate(it.x);
+    fk64_levels<32, true>(v, state, [&](int, int col) { return src.value(T, where, it.x, col); }, 1, T->base_type == PM_BASE_FIXED, rec);
     bool hit = false;
-    if (it.y < 0) {  // link-position bound -1 - it.y of a composite constraint, in FP64 (every lane)
+    if (it.y < 0) {  // link-position bound -1 - it.y of a composite constraint
       const PmPoseTerm& b = src.bnd.t[-1 - it.y];
-      DPose pose[PM_MAX_SLOTS];
-      fk64_need_warp(T, state, src.cfg(T, it.x, qbuf), T->base_type == PM_BASE_FIXED, slot_chain(T, b.slot), pose);
-      const D3& p = pose[b.slot].t;
+      const D3 p = P.at(b.slot).t;
       const double x = b.axis == 0 ? p.x : (b.axis == 1 ? p.y : p.z);
       hit = (b.has_lb && x < b.lb) || (b.has_ub && x > b.ub);
     } else if ((it.y & 1) == 0) {  // sphere it.z vs primitive it.y >> 1: gate AND test
-      const PmPrim& P = v.P[it.y >> 1];
+      const PmPrim& Q = v.P[it.y >> 1];
       const PmGroup& g = v.G[v.sgroup[it.z]];
-      // the FP64 FK of the slot's chain of ancestors, by the whole warp (every lane gets the poses)
-      DPose pose[PM_MAX_SLOTS];
-      fk64_need_warp(T, state, src.cfg(T, it.x, qbuf), T->base_type == PM_BASE_FIXED, slot_chain(T, g.slot), pose);
-      const DM3 R = qmat(pose[g.slot].q);
-      const D3 gc = add(mv(R, D3{g.rel[0], g.rel[1], g.rel[2]}), pose[g.slot].t);
-      const D3 c = add(mv(R, v.rel(it.z)), pose[g.slot].t);
+      const DPose lp = P.at(g.slot);
+      const DM3 R = qmat(lp.q);
+      const D3 gc = add(mv(R, D3{g.rel[0], g.rel[1], g.rel[2]}), lp.t);
+      const D3 c = add(mv(R, v.rel(it.z)), lp.t);
       const double r = v.sr[it.z];
-      if (P.kind == PM_SDF_CLOUD) {
+      if (Q.kind == PM_SDF_CLOUD) {
         // the sphere's own test first (small reach); its nearest point then settles the gate
         // exactly unless rounding leaves it undecided: min_p |gc - p| <= |gc - p_near|
-        const PmGridDev& Gd = v.C[P.cloud];
+        const PmGridDev& Gd = v.C[Q.cloud];
         int near = -1;
-        bool test = !outside_aabb(P, c, r) && !cloud_outside_warp(P, v.C, c, r, &near, it.w);
-        if (test && !outside_aabb(P, gc, g.radius)) {
+        bool test = !outside_aabb(Q, c, r) && !cloud_outside_warp(Q, v.C, c, r, &near, it.w);
+        if (test && !outside_aabb(Q, gc, g.radius)) {
           const D3 d{Gd.px[near] - gc.x, Gd.py[near] - gc.y, Gd.pz[near] - gc.z};
           const double d2n = d.x * d.x + (d.y * d.y + d.z * d.z);
-          hit = !(sqrt(d2n) - P.a > g.radius) || !cloud_outside_warp(P, v.C, gc, g.radius, nullptr);
+          hit = !(sqrt(d2n) - Q.a > g.radius) || !cloud_outside_warp(Q, v.C, gc, g.radius, nullptr);
         }
-      } else if (lane == 0 && !outside_aabb(P, gc, g.radius) && !prim_outside(P, v.C, gc, g.radius)) {
-        hit = !outside_aabb(P, c, r) && !prim_outside(P, v.C, c, r);
+      } else {
+        hit = gate_open(Q, gc, g.radius) && !outside_aabb(Q, c, r) && !prim_outside(Q, nullptr, c, r);
       }
-    } else {  // sphere pair (it.z, it.w) of self pair it.y >> 1: gate AND test (every lane, same values)
+    } else {  // sphere pair (it.z, it.w) of self pair it.y >> 1: gate AND test
       const int pr = it.y >> 1;
       const PmGroup& g1 = v.G[v.pairs[2 * pr]];
       const PmGroup& g2 = v.G[v.pairs[2 * pr + 1]];
-      DPose pose[PM_MAX_SLOTS];
-      fk64_need_warp(T, state, src.cfg(T, it.x, qbuf), T->base_type == PM_BASE_FIXED, slot_chain(T, g1.slot) | slot_chain(T, g2.slot),
-                     pose);
-      const DM3 R1 = qmat(pose[g1.slot].q), R2 = qmat(pose[g2.slot].q);
-      const D3 c1 = add(mv(R1, D3{g1.rel[0], g1.rel[1], g1.rel[2]}), pose[g1.slot].t);
-      const D3 c2 = add(mv(R2, D3{g2.rel[0], g2.rel[1], g2.rel[2]}), pose[g2.slot].t);
+      const DPose p1 = P.at(g1.slot), p2 = P.at(g2.slot);
+      const DM3 R1 = qmat(p1.q), R2 = qmat(p2.q);
+      const D3 c1 = add(mv(R1, D3{g1.rel[0], g1.rel[1], g1.rel[2]}), p1.t);
+      const D3 c2 = add(mv(R2, D3{g2.rel[0], g2.rel[1], g2.rel[2]}), p2.t);
       const double osq = sqn(sub(c1, c2));
       const double ors = g1.radius + g2.radius;
       if (!(osq > ors * ors)) {
-        const D3 a = add(mv(R1, v.rel(it.z)), pose[g1.slot].t);
-        const D3 bb = add(mv(R2, v.rel(it.w)), pose[g2.slot].t);
+        const D3 a = add(mv(R1, v.rel(it.z)), p1.t);
+        const D3 bb = add(mv(R2, v.rel(it.w)), p2.t);
         const double rs = v.sr[it.z] + v.sr[it.w];
         hit = sqn(sub(a, bb)) < rs * rs;
       }
     }
     if (__shfl_sync(FULL, hit ? 1 : 0, 0) && lane == 0) src.fail(it.x);
   }
+  double qbuf[PM_MAX_SLOTS + 8];
   // configurations (or edges) whose terms overflowed the queue: the plain FP64 check, one thread each
   const int64_t slots = src.n_overflow_slots();
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < slots; k += (int64_t)gridDim.x * blockDim.x) {
@@ -1515,12 +1532,15 @@ static cudaError_t prep(K kern, size_t sm) {
   return e;
 }
 
-// Blocks of the recheck kernel: one 4-warp block per 32 configurations (or 8 edges), at most 4 per
-// SM; its loops stride over the grid, so a small batch launches few blocks.
+// Blocks of the recheck kernel: one warp per 8 configurations (or 2 edges), at most 16 per SM; its loops
+// stride over the grid, so a small batch launches few blocks.
 static unsigned recheck_grid(int64_t units, int per_block, int n_sm) {
   const int64_t want = (units + per_block - 1) / per_block;
-  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)n_sm * 4));
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)n_sm * 16));
 }
+
+// At most 64 slots x 64 bytes: 4 KB.
+static size_t recheck_smem(const PmTablesHdr& h) { return (size_t)kRecheckWarps * h.n_slots * kRec * sizeof(double); }
 
 // count, overflow and stats must be zeroed by the caller
 cudaError_t launch_fast_valid(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* q, int64_t B,
@@ -1570,7 +1590,7 @@ cudaError_t launch_fast_valid(const PmTablesHdr* T, const PmTablesHdr& h, const 
     prof_end("k_hard_queries", s);
   }
   prof_begin("k_fast_recheck", s);
-  k_fast_recheck<CfgSource><<<recheck_grid(B, 32, n_sm), 128, 0, s>>>(T, state, src, scr);
+  k_fast_recheck<CfgSource><<<recheck_grid(B, 8, n_sm), 32 * kRecheckWarps, recheck_smem(h), s>>>(T, state, src, scr);
   prof_end("k_fast_recheck", s);
   return cudaGetLastError();
 }
@@ -1615,7 +1635,7 @@ cudaError_t launch_fast_edges(const PmTablesHdr* T, const PmTablesHdr& h, const 
   if (!launched) return cudaErrorInvalidValue;
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   prof_begin("k_fast_recheck_edges", s);
-  k_fast_recheck<EdgeSource><<<recheck_grid(E, 8, n_sm), 128, 0, s>>>(T, state, src, scr);
+  k_fast_recheck<EdgeSource><<<recheck_grid(E, 2, n_sm), 32 * kRecheckWarps, recheck_smem(h), s>>>(T, state, src, scr);
   prof_end("k_fast_recheck_edges", s);
   return cudaGetLastError();
 }

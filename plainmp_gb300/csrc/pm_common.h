@@ -184,7 +184,7 @@ struct PmTablesHdr {
   int32_t root_slot, n_clouds, n_levels, pad1;
   int64_t off_slots, off_joints, off_groups, off_sx, off_sy, off_sz, off_sr, off_sgroup, off_pairs, off_prims, off_clouds;
   int64_t off_img, img_bytes;  // the FP32 image
-  int64_t off_lev;  // slots by depth: the n_levels + 1 starts, then the slots (int32)
+  int64_t off_lev;  // slots by depth: the n_levels + 1 starts, then slot | parent << 16 (int32)
   int64_t total_bytes;
 };
 

@@ -56,14 +56,21 @@ __device__ __forceinline__ float cast_error(const float* P, float sn) {
   return kU * (64.0f * sn + 4.0f * (fabsf(P[9]) + fabsf(P[10]) + fabsf(P[11]))) + 1e-9f;
 }
 
-// FK of configurations 0 .. ncfg - 1 of a block of NT threads into rec [ncfg][n_slots][kRec] and p32
-// [ncfg][n_slots][kRec32]; qf(c, col) gives a joint or base value.  The pose of a slot replaces its local
+// FK of configurations 0 .. ncfg - 1 by NT threads (a block, or a warp of one: WARP) into rec
+// [ncfg][n_slots][kRec]; qf(c, col) gives a joint or base value.  The pose of a slot replaces its local
 // transform in place.  Poses are bit for bit those of fk64.
-template <int NT, class QF>
-__device__ void fk64_block(const TView& v, const double* __restrict__ state, const QF& qf, int ncfg, bool taylor, double* rec, float* p32) {
+template <int NT, bool WARP, class QF>
+__device__ void fk64_levels(const TView& v, const double* __restrict__ state, const QF& qf, int ncfg, bool taylor, double* rec) {
   const unsigned FULL = 0xffffffffu;
   const PmTablesHdr* T = v.T;
-  const int tid = threadIdx.x, nsl = T->n_slots, nc = T->n_ctrl;
+  const int tid = WARP ? threadIdx.x & 31 : threadIdx.x, nsl = T->n_slots, nc = T->n_ctrl;
+  auto sync = [] {
+    if (WARP) {
+      __syncwarp();
+    } else {
+      __syncthreads();
+    }
+  };
   for (int t = tid; t < ncfg * nsl; t += NT) {
     const int c = t / nsl, i = t - c * nsl;
     const PmSlot& s = v.S[i];
@@ -98,15 +105,15 @@ __device__ void fk64_block(const TView& v, const double* __restrict__ state, con
   const int32_t* order = lev + T->n_levels + 1;
   const int quad = tid >> 2, k = tid & 3, w0 = (tid >> 5) << 3;  // the lane's quad and component, the warp's first quad
   const int i1 = k == 0 ? 1 : (k == 1 ? 2 : 0), i2 = k == 0 ? 2 : (k == 1 ? 0 : 1);  // the cyclic next two of x y z
-  __syncthreads();
+  sync();
   for (int l = 1; l < T->n_levels; l++) {
     const int s0 = lev[l], nl = lev[l + 1] - s0, tasks = ncfg * nl;
     for (int t0 = 0; t0 + w0 < tasks; t0 += NT / 4) {  // warp-uniform
       const bool on = t0 + quad < tasks;
       const int t = on ? t0 + quad : tasks - 1;
-      const int c = t / nl, i = order[s0 + t - c * nl];
-      double* o = rec + ((size_t)c * nsl + i) * kRec;
-      const double* a = rec + ((size_t)c * nsl + v.S[i].parent) * kRec;
+      const int c = t / nl, sp = order[s0 + t - c * nl];  // slot and parent, 16 bits each
+      double* o = rec + ((size_t)c * nsl + (sp & 0xffff)) * kRec;
+      const double* a = rec + ((size_t)c * nsl + (sp >> 16)) * kRec;
       // component k of qmul(a, o): x y z: aw o_k + a_k ow + a_i1 o_i2 - a_i2 o_i1;
       //                            w:     aw ow - ax ox - ay oy - az oz
       const bool w = k == 3;
@@ -126,9 +133,15 @@ __device__ void fk64_block(const TView& v, const double* __restrict__ state, con
         if (!w) o[4 + k] = tr;
       }
     }
-    __syncthreads();
+    sync();
   }
-  for (int t = tid; t < ncfg * nsl; t += NT) {
+}
+
+// fk64_levels by a block of NT threads, and the poses in FP32 (p32 [ncfg][n_slots][kRec32]).
+template <int NT, class QF>
+__device__ void fk64_block(const TView& v, const double* __restrict__ state, const QF& qf, int ncfg, bool taylor, double* rec, float* p32) {
+  fk64_levels<NT, false>(v, state, qf, ncfg, taylor, rec);
+  for (int t = threadIdx.x; t < ncfg * v.T->n_slots; t += NT) {
     const double* r = rec + (size_t)t * kRec;
     float* f = p32 + (size_t)t * kRec32;
     const float x = (float)r[0], y = (float)r[1], z = (float)r[2], w = (float)r[3];
