@@ -163,10 +163,13 @@ int pmgpu_cst_get_all_spheres(pmgpu_cst* c, double* out4);
 int pmgpu_cst_get_group_spheres(pmgpu_cst* c, double* out4);
 
 /* is_valid(q) for B configs (IneqConstraintBase::is_valid, primitive.hpp:113-117 ->
- * is_valid_dirty, primitive_sphere_collision.cpp:181-254).  Plain method: FP64, Taylor
- * sin/cos for FIXED bases, the reference's branch structure, one device thread per config.
- * q is B x q_dim row-major; out[b] is 1 (valid) or 0. */
+ * is_valid_dirty, primitive_sphere_collision.cpp:181-254).  Plain method: FP64 FK and decisions in
+ * the reference's expressions (Taylor sin/cos for FIXED bases), FP32 only to skip what it clears by
+ * more than its error bound.  q is B x q_dim row-major; out[b] is 1 (valid) or 0. */
 int pmgpu_cst_is_valid(pmgpu_cst* c, const double* q, int64_t B, uint8_t* out, int mem, void* stream);
+/* pmgpu_cst_is_valid of one config in host memory followed by pmgpu_cst_update_kintree(q,
+ * high_accuracy), in one launch: what the reference's is_valid(q) leaves behind. */
+int pmgpu_cst_is_valid_state(pmgpu_cst* c, const double* q, int high_accuracy, uint8_t* out);
 /* evaluate(q) for B configs (ConstraintBase::evaluate, primitive.hpp:74-79 ->
  * evaluate_dirty, primitive_sphere_collision.cpp:256-399): vals B x cst_dim, jac
  * B x cst_dim x q_dim (row-major), FP64 with libm-accuracy sin/cos. */

@@ -97,6 +97,7 @@ _SIGS = {
     "pmgpu_cst_get_all_spheres": (_i, [_p, _dp]),
     "pmgpu_cst_get_group_spheres": (_i, [_p, _dp]),
     "pmgpu_cst_is_valid": (_i, [_p, _p, _i64, _p, _i, _p]),
+    "pmgpu_cst_is_valid_state": (_i, [_p, _p, _i, _u8p]),
     "pmgpu_cst_evaluate": (_i, [_p, _p, _i64, _p, _p, _i, _p]),
     "pmgpu_cst_sphere_distances": (_i, [_p, _p, _i64, _i, _p, _p, _i, _p]),
     "pmgpu_cst_is_valid_fast": (_i, [_p, _p, _i64, _p, _p, _p, _i, _p]),

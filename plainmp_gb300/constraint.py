@@ -136,9 +136,9 @@ class SphereCollisionCst(IneqConstraintBase):
     def is_valid(self, q) -> bool:
         """IneqConstraintBase.is_valid: also leaves the model in q's state, as the reference does."""
         qq = f64(q, (1, self.q_dim()))
-        ok = bool(self.is_valid_batch(qq)[0])
-        self.update_kintree(qq[0], high_accuracy=self.base_type != BaseType.FIXED)
-        return ok
+        ok = C.c_uint8()
+        check(lib.pmgpu_cst_is_valid_state(self._h, C.c_void_p(qq.ctypes.data), int(self.base_type != BaseType.FIXED), C.byref(ok)))
+        return ok.value != 0
 
     def evaluate(self, q) -> Tuple[np.ndarray, np.ndarray]:
         qq = f64(q, (1, self.q_dim()))

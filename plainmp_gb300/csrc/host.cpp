@@ -171,6 +171,10 @@ struct PinBuf {
   }
 };
 static size_t up16(size_t x) { return (x + 15) & ~(size_t)15; }
+// Host-memory calls of up to this many configurations or edges of the FP64 method stage in page-locked memory
+// that the kernel itself reads and writes: no copies on the stream.  A call of one state took 66 us with them,
+// 32 us without (update of the model state included).
+constexpr int64_t kZeroCopy = 64;
 
 // ---------------------------------------------------------------------------- host quaternion
 // construction-time helpers (setQuaternionFromRPY, transform.hpp:122-130)
@@ -1338,7 +1342,7 @@ int pmgpu_model_set_joint_positions(pmgpu_model* m, const int64_t* ids, int n, c
     cuda_check(cudaMemcpy(d, recs.data(), rb, cudaMemcpyHostToDevice), "H2D");
     double* dq = (double*)(d + ((rb + 15) / 16) * 16);
     cuda_check(cudaMemcpy(dq, q, (size_t)n * 8, cudaMemcpyHostToDevice), "H2D");
-    cuda_check(launch_set_joints(M.d_state.as<double>(), (const PmSlot*)d, dq, n, accurate, 0), "set joints");
+    cuda_check(launch_update_state(M.d_state.as<double>(), (const PmSlot*)d, dq, n, accurate, PM_BASE_FIXED, 0), "set joints");
     cuda_check(cudaDeviceSynchronize(), "set joints");
   });
 }
@@ -1799,11 +1803,10 @@ static void update_kintree_of(HostCst& C, const double* q, int high_accuracy) {
   HostModel& M = *C.kin;
   int nq = C.q_dim(), nc = (int)C.ids.size();
   for (int i = 0; i < nc; i++) M.angles[C.ids[i]] = q[i];
-  double* dq = (double*)C.w_aux.ensure((size_t)nq * 8 + 16);
-  cuda_check(cudaMemcpy(dq, q, (size_t)nq * 8, cudaMemcpyHostToDevice), "H2D");
+  double* pin = (double*)C.h_pin.ensure((size_t)nq * 8 + 16);  // the kernel reads q from page-locked host memory
+  std::memcpy(pin, q, (size_t)nq * 8);
   int accurate = (C.base_type != PM_BASE_FIXED) ? 1 : (high_accuracy ? 1 : 0);
-  if (nc > 0) cuda_check(launch_set_joints(M.d_state.as<double>(), C.d_ctrl_recs.as<PmSlot>(), dq, nc, accurate, 0), "update_kintree");
-  if (C.base_type != PM_BASE_FIXED) cuda_check(launch_set_base_from_q(M.d_state.as<double>(), C.base_type, dq + nc, 0), "update_kintree");
+  cuda_check(launch_update_state(M.d_state.as<double>(), C.d_ctrl_recs.as<PmSlot>(), pin, nc, accurate, C.base_type, 0), "update_kintree");
   cuda_check(cudaDeviceSynchronize(), "update_kintree");
 }
 
@@ -1844,11 +1847,40 @@ int pmgpu_cst_is_valid(pmgpu_cst* c, const double* q, int64_t B, uint8_t* out, i
       cuda_check(launch_is_valid64(T, C.hdr, st, q, B, out, s), "is_valid");
       return;
     }
+    if (B <= kZeroCopy) {
+      const size_t nq = (size_t)B * C.q_dim() * 8;
+      char* pin = C.h_pin.ensure(up16(nq) + up16((size_t)B));
+      std::memcpy(pin, q, nq);
+      cuda_check(launch_is_valid64(T, C.hdr, st, (const double*)pin, B, (uint8_t*)(pin + up16(nq)), s), "is_valid");
+      cuda_check(cudaStreamSynchronize(s), "is_valid");
+      std::memcpy(out, pin + up16(nq), (size_t)B);
+      return;
+    }
     const double* dq = stage_in(C.w_in, q, (size_t)B * C.q_dim(), s);
     uint8_t* dout = (uint8_t*)C.w_out.ensure(std::max<size_t>((size_t)B, 16));
     cuda_check(launch_is_valid64(T, C.hdr, st, dq, B, dout, s), "is_valid");
     stage_out(out, dout, (size_t)B, s);
     cuda_check(cudaStreamSynchronize(s), "is_valid");
+  });
+}
+int pmgpu_cst_is_valid_state(pmgpu_cst* c, const double* q, int high_accuracy, uint8_t* out) {
+  return guarded([&] {
+    check_ptr(c, "cst");
+    check_ptr(out, "out");
+    HostCst& C = c->c;
+    check_arr(q, C.q_dim(), "q");
+    const PmTablesHdr* T = C.tables();
+    HostModel& M = *C.kin;
+    const size_t nq = (size_t)C.q_dim() * 8;
+    char* pin = C.h_pin.ensure(up16(nq) + 16);
+    std::memcpy(pin, q, nq);
+    for (size_t i = 0; i < C.ids.size(); i++) M.angles[C.ids[i]] = q[i];
+    const int accurate = (C.base_type != PM_BASE_FIXED) ? 1 : (high_accuracy ? 1 : 0);
+    cuda_check(launch_is_valid64_update(T, C.hdr, M.d_state.as<double>(), C.d_ctrl_recs.as<PmSlot>(), (const double*)pin, accurate,
+                                        (uint8_t*)(pin + up16(nq)), 0),
+               "is_valid");
+    cuda_check(cudaStreamSynchronize(0), "is_valid");
+    *out = (uint8_t)pin[up16(nq)];
   });
 }
 int pmgpu_cst_evaluate(pmgpu_cst* c, const double* q, int64_t B, double* vals, double* jac, int mem, void* stream) {
@@ -1866,6 +1898,16 @@ int pmgpu_cst_evaluate(pmgpu_cst* c, const double* q, int64_t B, double* vals, d
     int m = C.cst_dim(), d = C.q_dim();
     if (mem == PMGPU_MEM_DEVICE) {
       cuda_check(launch_evaluate64(T, C.hdr, st, q, B, 1, vals, jac, s), "evaluate");
+      return;
+    }
+    if (B <= kZeroCopy) {
+      const size_t nq = up16((size_t)B * d * 8), nv = up16((size_t)B * m * 8), nj = (size_t)B * m * d * 8;
+      char* pin = C.h_pin.ensure(nq + nv + nj + 16);
+      std::memcpy(pin, q, (size_t)B * d * 8);
+      cuda_check(launch_evaluate64(T, C.hdr, st, (const double*)pin, B, 1, (double*)(pin + nq), (double*)(pin + nq + nv), s), "evaluate");
+      cuda_check(cudaStreamSynchronize(s), "evaluate");
+      if (m) std::memcpy(vals, pin + nq, (size_t)B * m * 8);
+      if (m) std::memcpy(jac, pin + nq + nv, nj);
       return;
     }
     const double* dq = stage_in(C.w_in, q, (size_t)B * d, s);
@@ -2144,8 +2186,25 @@ int pmgpu_check_motion(pmgpu_cst* c, const double* s1, const double* s2, int64_t
     const int16_t* seq = C.seq_table();
     int d = C.q_dim();
     const double* dw = nullptr;
+    if (validator_type == PMGPU_VALIDATOR_BOX) check_ptr(width, "width");
+    if (mem == PMGPU_MEM_HOST && E <= kZeroCopy) {  // page-locked [s1 | s2 | width | counts | out], read and written by the kernel
+      const size_t ns_ = (size_t)E * d * 8, nw = up16((size_t)d * 8), nc = up16((size_t)E * 8);
+      char* pin = C.h_pin.ensure(2 * up16(ns_) + nw + nc + up16((size_t)E) + 16);
+      char *p2 = pin + up16(ns_), *pw = p2 + up16(ns_), *pc = pw + nw, *po = pc + nc;
+      std::memcpy(pin, s1, ns_);
+      std::memcpy(p2, s2, ns_);
+      if (validator_type == PMGPU_VALIDATOR_BOX) std::memcpy(pw, width, (size_t)d * 8);
+      cuda_check(launch_check_motion64(T, C.hdr, st, (const double*)pin, (const double*)p2, E, validator_type, (const double*)pw, resolution,
+                                       seq, (uint8_t*)po, nullptr, (unsigned long long*)pc, s),
+                 "check_motion");
+      cuda_check(cudaStreamSynchronize(s), "check_motion");
+      std::memcpy(out, po, (size_t)E);
+      int64_t total = 0;
+      for (int64_t i = 0; i < E; i++) total += (int64_t)((const unsigned long long*)pc)[i];
+      if (n_checked) *n_checked = total;
+      return;
+    }
     if (validator_type == PMGPU_VALIDATOR_BOX) {
-      check_ptr(width, "width");
       dw = (const double*)C.w_width.ensure((size_t)d * 8 + 16);
       if (mem == PMGPU_MEM_DEVICE)
         cuda_check(cudaMemcpyAsync((void*)dw, width, (size_t)d * 8, cudaMemcpyDeviceToDevice, s), "width");
@@ -2155,7 +2214,7 @@ int pmgpu_check_motion(pmgpu_cst* c, const double* s1, const double* s2, int64_t
     unsigned long long* cnt = (unsigned long long*)C.w_aux.ensure(64);
     cuda_check(cudaMemsetAsync(cnt, 0, 8, s), "memset");
     if (mem == PMGPU_MEM_DEVICE) {
-      cuda_check(launch_check_motion64(T, C.hdr, st, s1, s2, E, validator_type, dw, resolution, seq, out, cnt, s), "check_motion");
+      cuda_check(launch_check_motion64(T, C.hdr, st, s1, s2, E, validator_type, dw, resolution, seq, out, cnt, nullptr, s), "check_motion");
       if (n_checked) {
         unsigned long long h = 0;
         cuda_check(cudaMemcpyAsync(&h, cnt, 8, cudaMemcpyDeviceToHost, s), "D2H");
@@ -2167,7 +2226,7 @@ int pmgpu_check_motion(pmgpu_cst* c, const double* s1, const double* s2, int64_t
     const double* d1 = stage_in(C.w_in, s1, (size_t)E * d, s);
     const double* d2 = stage_in(C.w_in2, s2, (size_t)E * d, s);
     uint8_t* dout = (uint8_t*)C.w_out.ensure(std::max<size_t>((size_t)E, 16));
-    cuda_check(launch_check_motion64(T, C.hdr, st, d1, d2, E, validator_type, dw, resolution, seq, dout, cnt, s), "check_motion");
+    cuda_check(launch_check_motion64(T, C.hdr, st, d1, d2, E, validator_type, dw, resolution, seq, dout, cnt, nullptr, s), "check_motion");
     stage_out(out, dout, (size_t)E, s);
     unsigned long long h = 0;
     cuda_check(cudaMemcpyAsync(&h, cnt, 8, cudaMemcpyDeviceToHost, s), "D2H");

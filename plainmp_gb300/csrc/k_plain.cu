@@ -171,12 +171,72 @@ __device__ void valid_team(const TView& v, const Image& im, const TeamPose& P, i
 // Dynamic shared memory of a block of nc configurations.
 inline size_t team_smem(const PmTablesHdr& h, int nc) { return (size_t)nc * h.n_slots * (kRec * sizeof(double) + kRec32 * sizeof(float)); }
 
+// ConstraintBase::update_kintree (primitive.hpp:38-62) on the model state by a block of at least two warps: the
+// control joints' rows on the first warp's lanes (of a repeated joint the last value counts), the base row on
+// the second warp.  q: the joint values, then the base's.
+__device__ void update_state_block(double* state, const PmSlot* __restrict__ recs, const double* __restrict__ q, int n, int accurate,
+                                   int base_type) {
+  const int tid = threadIdx.x;
+  if (tid < 32) {
+    for (int i = tid; i < n; i += 32) {
+      bool last = true;
+      for (int j = i + 1; j < n; j++) last = last && recs[j].link != recs[i].link;
+      if (!last) continue;
+      DQ lq;
+      D3 lt;
+      bool lid;
+      joint_local(recs[i], q[i], accurate == 0, lq, lt, lid);
+      double* r = state + (int64_t)PM_STATE_LINK_ROW(recs[i].link) * PM_STATE_STRIDE;
+      r[0] = lq.x;
+      r[1] = lq.y;
+      r[2] = lq.z;
+      r[3] = lq.w;
+      r[4] = lt.x;
+      r[5] = lt.y;
+      r[6] = lt.z;
+      r[7] = lid ? 1.0 : 0.0;
+    }
+  } else if (tid == 32 && base_type != PM_BASE_FIXED) {
+    const double* qb = q + n;
+    DQ bq;
+    D3 t;
+    if (base_type == PM_BASE_FLOATING) {
+      t = D3{qb[0], qb[1], qb[2]};
+      bq = quat_from_rpy(qb[3], qb[4], qb[5]);
+    } else {
+      t = D3{qb[0], qb[1], 0.0};
+      bq = quat_from_rpy(0, 0, qb[2]);
+    }
+    double* r = state + PM_STATE_BASE_ROW * PM_STATE_STRIDE;
+    r[0] = bq.x;
+    r[1] = bq.y;
+    r[2] = bq.z;
+    r[3] = bq.w;
+    r[4] = t.x;
+    r[5] = t.y;
+    r[6] = t.z;
+    r[7] = 0.0;
+  }
+}
+
+__global__ void k_update_state(double* state, const PmSlot* recs, const double* q, int n, int accurate, int base_type) {
+  update_state_block(state, recs, q, n, accurate, base_type);
+}
+
 // NC configurations per block, WPC warps each; 128 registers a thread.
-template <int NC, int WPC>
-__global__ void __launch_bounds__(NC * WPC * 32, 512 / (NC * WPC * 32)) k_is_valid64(const PmTablesHdr* __restrict__ T, const double* __restrict__ state,
-                                                             const double* __restrict__ q, int64_t B, uint8_t* __restrict__ out) {
+// UPDATE (one configuration): a second block leaves the model in its state, as is_valid of the reference does.
+// The rows it writes (control joints' links, the base row unless the base is fixed) are not among those that
+// the check reads (links without a control joint, a fixed base).
+template <int NC, int WPC, bool UPDATE = false>
+__global__ void __launch_bounds__(NC * WPC * 32, 512 / (NC * WPC * 32))
+    k_is_valid64(const PmTablesHdr* __restrict__ T, double* state, const double* __restrict__ q, int64_t B, uint8_t* __restrict__ out,
+                 const PmSlot* __restrict__ recs, int accurate) {
   extern __shared__ __align__(16) double team_mem[];
   __shared__ int failed[NC];
+  if (UPDATE && blockIdx.x == 1) {
+    update_state_block(state, recs, q, T->n_ctrl, accurate, T->base_type);
+    return;
+  }
   const TView v(T);
   const Image im(T);
   const int nsl = T->n_slots, qd = T->q_dim;
@@ -194,23 +254,31 @@ __global__ void __launch_bounds__(NC * WPC * 32, 512 / (NC * WPC * 32)) k_is_val
 
 // CustomValidatorBase::checkMotion (motion_validator.cpp:17-79), a block per edge: its waypoints in the
 // reference's visiting order, NC at a time, a warp each; the first round with a collision ends it.
-// n_checked counts the waypoints up to and including the first that collides, as the reference visits them.
+// n_checked (a sum) and counts (per edge), each optional, count the waypoints up to and including the first
+// that collides, as the reference visits them.  The endpoints go to shared memory first: small calls pass them
+// in page-locked host memory.
 template <int NC>
 __global__ void __launch_bounds__(NC * 32, 512 / (NC * 32)) k_check_motion64(const PmTablesHdr* __restrict__ T, const double* __restrict__ state,
                                                             const double* __restrict__ s1, const double* __restrict__ s2, int type,
                                                             const double* __restrict__ width, double resolution,
                                                             const int16_t* __restrict__ seq, uint8_t* __restrict__ out,
-                                                            unsigned long long* n_checked) {
+                                                            unsigned long long* n_checked, unsigned long long* counts) {
   extern __shared__ __align__(16) double team_mem[];
   __shared__ int failed[NC];
+  __shared__ double ends[2][PM_MAX_DOF], wd[PM_MAX_DOF];
   __shared__ double step;
   __shared__ unsigned long long n_way;  // waypoints to check (0: decided already)
   const TView v(T);
   const Image im(T);
   const int64_t e = blockIdx.x;
   const int dim = T->q_dim, nsl = T->n_slots;
-  const double* a = s1 + e * dim;
-  const double* b = s2 + e * dim;
+  const double *a = ends[0], *b = ends[1];
+  for (int i = threadIdx.x; i < dim; i += NC * 32) {
+    ends[0][i] = s1[e * dim + i];
+    ends[1][i] = s2[e * dim + i];
+    if (type == 0) wd[i] = width[i];
+  }
+  __syncthreads();
   if (threadIdx.x == 0) {
     double sr;
     if (type == 0) {  // BoxMotionValidator::determine_step_ratio (:89-111)
@@ -218,14 +286,14 @@ __global__ void __launch_bounds__(NC * 32, 512 / (NC * 32)) k_check_motion64(con
       int li = 0;
       for (int i = 0; i < dim; i++) {
         double diff = b[i] - a[i];
-        double asd = fabs(diff) * (1.0 / width[i]);
+        double asd = fabs(diff) * (1.0 / wd[i]);
         if (asd > max_diff) {
           max_diff = asd;
           li = i;
           diff_long = diff;
         }
       }
-      sr = fabs(diff_long) < 1e-6 ? INFINITY : width[li] / fabs(diff_long);
+      sr = fabs(diff_long) < 1e-6 ? INFINITY : wd[li] / fabs(diff_long);
     } else {  // EuclideanMotionValidator (:118-126)
       double dist = 0.0;
       for (int i = 0; i < dim; i++) {
@@ -236,6 +304,7 @@ __global__ void __launch_bounds__(NC * 32, 512 / (NC * 32)) k_check_motion64(con
     }
     step = sr;
     n_way = 0;
+    if (counts) counts[e] = 0;
     if (sr == INFINITY) {
       out[e] = 1;
     } else if (!(sr > 0.0) || 1.0 / sr > 67108864.0) {
@@ -277,6 +346,7 @@ __global__ void __launch_bounds__(NC * 32, 512 / (NC * 32)) k_check_motion64(con
   if (threadIdx.x == 0) {
     out[e] = ok ? 1 : 0;
     if (n_checked) atomicAdd(n_checked, checked);
+    if (counts) counts[e] = checked;
   }
 }
 
@@ -655,47 +725,6 @@ __global__ void k_spheres_of_state(const PmTablesHdr* __restrict__ T, const doub
 }
 
 // ------------------------------------------------------------------ model state
-__global__ void k_set_joints(double* state, const PmSlot* recs, const double* q, int n, int accurate) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  for (int i = 0; i < n; i++) {  // in order: a repeated joint keeps its last value
-    DQ lq;
-    D3 lt;
-    bool lid;
-    joint_local(recs[i], q[i], accurate == 0, lq, lt, lid);
-    double* r = state + (int64_t)PM_STATE_LINK_ROW(recs[i].link) * PM_STATE_STRIDE;
-    r[0] = lq.x;
-    r[1] = lq.y;
-    r[2] = lq.z;
-    r[3] = lq.w;
-    r[4] = lt.x;
-    r[5] = lt.y;
-    r[6] = lt.z;
-    r[7] = lid ? 1.0 : 0.0;
-  }
-}
-
-__global__ void k_set_base_from_q(double* state, int base_type, const double* qb) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  DQ q;
-  D3 t;
-  if (base_type == PM_BASE_FLOATING) {
-    t = D3{qb[0], qb[1], qb[2]};
-    q = quat_from_rpy(qb[3], qb[4], qb[5]);
-  } else {
-    t = D3{qb[0], qb[1], 0.0};
-    q = quat_from_rpy(0, 0, qb[2]);
-  }
-  double* r = state + PM_STATE_BASE_ROW * PM_STATE_STRIDE;
-  r[0] = q.x;
-  r[1] = q.y;
-  r[2] = q.z;
-  r[3] = q.w;
-  r[4] = t.x;
-  r[5] = t.y;
-  r[6] = t.z;
-  r[7] = 0.0;
-}
-
 // build_cache_until for selected links (algorithm.cpp:160-210)
 __global__ void k_link_poses(const double* __restrict__ state, const int32_t* __restrict__ parents, const int32_t* __restrict__ links,
                              int n, double* __restrict__ out7) {
@@ -784,12 +813,8 @@ cudaError_t team_launch(K kern, int64_t blocks, int nc, int wpc, const PmTablesH
 
 namespace pmg {
 
-cudaError_t launch_set_joints(double* state, const PmSlot* recs, const double* q, int n, int accurate, cudaStream_t s) {
-  k_set_joints<<<1, 1, 0, s>>>(state, recs, q, n, accurate);
-  return cudaGetLastError();
-}
-cudaError_t launch_set_base_from_q(double* state, int base_type, const double* qbase, cudaStream_t s) {
-  k_set_base_from_q<<<1, 1, 0, s>>>(state, base_type, qbase);
+cudaError_t launch_update_state(double* state, const PmSlot* recs, const double* q, int n, int accurate, int base_type, cudaStream_t s) {
+  k_update_state<<<1, 64, 0, s>>>(state, recs, q, n, accurate, base_type);
   return cudaGetLastError();
 }
 cudaError_t launch_link_poses(const double* state, const int32_t* parents, const int32_t* links, int n, double* out7,
@@ -804,13 +829,18 @@ cudaError_t launch_is_valid64(const PmTablesHdr* T, const PmTablesHdr& h, const 
   int n_sm = 0;
   cudaError_t e = sm_count(&n_sm);
   if (e != cudaSuccess) return e;
+  double* st = const_cast<double*>(state);  // written only with UPDATE
   prof_begin("k_is_valid64", s);
   if (B <= 4 * (int64_t)n_sm)
-    e = team_launch(k_is_valid64<1, 4>, B, 1, 4, h, s, T, state, q, B, out);
+    e = team_launch(k_is_valid64<1, 4>, B, 1, 4, h, s, T, st, q, B, out, (const PmSlot*)nullptr, 0);
   else
-    e = team_launch(k_is_valid64<8, 1>, (B + 7) / 8, 8, 1, h, s, T, state, q, B, out);
+    e = team_launch(k_is_valid64<8, 1>, (B + 7) / 8, 8, 1, h, s, T, st, q, B, out, (const PmSlot*)nullptr, 0);
   prof_end("k_is_valid64", s);
   return e;
+}
+cudaError_t launch_is_valid64_update(const PmTablesHdr* T, const PmTablesHdr& h, double* state, const PmSlot* recs, const double* q,
+                                     int accurate, uint8_t* out, cudaStream_t s) {
+  return team_launch(k_is_valid64<1, 4, true>, 2, 1, 4, h, s, T, state, q, (int64_t)1, out, recs, accurate);
 }
 cudaError_t launch_evaluate64(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* q, int64_t B,
                               int high_accuracy, double* vals, double* jac, cudaStream_t s) {
@@ -839,14 +869,15 @@ cudaError_t launch_spheres_of_state(const PmTablesHdr* T, const double* state, i
   return cudaGetLastError();
 }
 cudaError_t launch_check_motion64(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* s1,
-                                  const double* s2, int64_t E, int type, const double* width, double resolution,
-                                  const int16_t* seq, uint8_t* out, unsigned long long* n_checked, cudaStream_t s) {
+                                  const double* s2, int64_t E, int type, const double* width, double resolution, const int16_t* seq,
+                                  uint8_t* out, unsigned long long* n_checked, unsigned long long* counts, cudaStream_t s) {
   if (E <= 0) return cudaSuccess;
   int n_sm = 0;
   cudaError_t e = sm_count(&n_sm);
   if (e != cudaSuccess) return e;
-  if (E <= n_sm) return team_launch(k_check_motion64<16>, E, 16, 1, h, s, T, state, s1, s2, type, width, resolution, seq, out, n_checked);
-  return team_launch(k_check_motion64<8>, E, 8, 1, h, s, T, state, s1, s2, type, width, resolution, seq, out, n_checked);
+  if (E <= n_sm)
+    return team_launch(k_check_motion64<16>, E, 16, 1, h, s, T, state, s1, s2, type, width, resolution, seq, out, n_checked, counts);
+  return team_launch(k_check_motion64<8>, E, 8, 1, h, s, T, state, s1, s2, type, width, resolution, seq, out, n_checked, counts);
 }
 cudaError_t launch_sdf_points(const PmPrim* prims, int n_prims, const PmGridDev* clouds, int n_clouds, int is_union,
                               const double* pts, const double* radii, int64_t n, double* eval_out, uint8_t* outside_out, cudaStream_t s) {

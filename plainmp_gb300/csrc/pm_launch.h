@@ -15,10 +15,9 @@ void prof_begin(const char* kernel, cudaStream_t s);
 void prof_end(const char* kernel, cudaStream_t s);
 
 // ---- model state (k_plain.cu)
-// recs: per joint to set, a PmSlot whose `link` is the child link and mode REV/PRIS.
-cudaError_t launch_set_joints(double* state, const PmSlot* recs, const double* q, int n, int accurate, cudaStream_t s);
-// base pose from q for PLANAR/FLOATING (q points at the base part), written to row 0.
-cudaError_t launch_set_base_from_q(double* state, int base_type, const double* qbase, cudaStream_t s);
+// The model state of q (joint values, then the base's for PLANAR / FLOATING): recs: per control joint, a PmSlot
+// whose `link` is the child link and mode REV/PRIS.
+cudaError_t launch_update_state(double* state, const PmSlot* recs, const double* q, int n, int accurate, int base_type, cudaStream_t s);
 // link poses of the current state: parents[n_link] (-1 root), links[n] -> out7[n*7]
 cudaError_t launch_link_poses(const double* state, const int32_t* parents, const int32_t* links, int n, double* out7,
                               cudaStream_t s);
@@ -26,6 +25,9 @@ cudaError_t launch_link_poses(const double* state, const int32_t* parents, const
 // ---- constraint batches (k_plain.cu)
 cudaError_t launch_is_valid64(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* q, int64_t B,
                               uint8_t* out, cudaStream_t s);
+// validity of one configuration, and the model left in its state (launch_update_state) by the same kernel
+cudaError_t launch_is_valid64_update(const PmTablesHdr* T, const PmTablesHdr& h, double* state, const PmSlot* recs, const double* q,
+                                     int accurate, uint8_t* out, cudaStream_t s);
 cudaError_t launch_evaluate64(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* q, int64_t B,
                               int high_accuracy, double* vals, double* jac, cudaStream_t s);
 // centres (B x n_spheres x 3) is required: the distances are computed from it
@@ -35,8 +37,8 @@ cudaError_t launch_sphere_dist64(const PmTablesHdr* T, const PmTablesHdr& h, con
 cudaError_t launch_spheres_of_state(const PmTablesHdr* T, const double* state, int groups, double* out4, cudaStream_t s);
 // checkMotion over E edges; seq: 128 x 128 int16 sequence table; width: q_dim (box) or NULL
 cudaError_t launch_check_motion64(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* s1,
-                                  const double* s2, int64_t E, int type, const double* width, double resolution,
-                                  const int16_t* seq, uint8_t* out, unsigned long long* n_checked, cudaStream_t s);
+                                  const double* s2, int64_t E, int type, const double* width, double resolution, const int16_t* seq,
+                                  uint8_t* out, unsigned long long* n_checked, unsigned long long* counts, cudaStream_t s);
 
 // ---- fast path (k_fast.cu): FP32 decisions + FP64 recheck of uncertain terms.
 size_t fast_smem_bytes(const PmTablesHdr& h, int cpb, bool want_dist);

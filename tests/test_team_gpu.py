@@ -95,3 +95,22 @@ def test_edges_and_counts(oracle, E):
         got, count = val.check_motion_batch(s1, s2, return_count=True)
         ref, rcount = oc.check_motion(s1, s2, kind, **args)
         assert np.array_equal(got, ref) and count == rcount
+
+
+@pytest.mark.parametrize("base", ["FIXED", "PLANAR", "FLOATING"])
+def test_single_state_check_leaves_the_state(oracle, base):
+    """is_valid(q) checks and updates the model in one launch: the answer is the batch's, the spheres of the
+    state are update_kintree's, over several states in a row and host batches at the zero-copy limit."""
+    cst, oc = _mixed(oracle, base)
+    Q = _configs(base, 65, seed=29)
+    ref = oc.is_valid(Q, threads=8)
+    for n in (63, 64, 65):
+        assert np.array_equal(cst.is_valid_batch(Q[:n]), ref[:n])
+        v, J = cst.evaluate_batch(Q[:n])
+        vd, Jd = cst.evaluate_batch(Q)
+        assert np.array_equal(v, vd[:n]) and np.array_equal(J, Jd[:n])
+    for q, ok in zip(Q[:6], ref[:6]):
+        assert cst.is_valid(q) == bool(ok)
+        got = [(*c, r) for c, r in cst.get_all_spheres()]
+        cst.update_kintree(q, high_accuracy=base != "FIXED")
+        assert np.array_equal(got, [(*c, r) for c, r in cst.get_all_spheres()])
