@@ -5,6 +5,7 @@
 // cell follows atomic arrival and is not fixed; nearest distances do not depend on it.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "pm_grid.cuh"
@@ -595,9 +596,7 @@ cudaError_t grid_build(GridBuild& g, cudaStream_t s) {
   int2* cl_rng = nullptr;
   uint32_t* cl_ent = nullptr;
   int64_t n_cl = 0;
-  int2* sb_rng = nullptr;
-  int32_t* sb_blk = nullptr;
-  float* sb_box = nullptr;
+  float4 *sb_rec = nullptr, *sb_blk = nullptr;
   int32_t n_sb = 0;
   float* blk_reach = nullptr;
   int32_t n_cand = 0;
@@ -656,9 +655,12 @@ cudaError_t grid_build(GridBuild& g, cudaStream_t s) {
         const int bx = (int)(b % nb[0]), by = (int)((b / nb[0]) % nb[1]), bz = (int)(b / ((int64_t)nb[0] * nb[1]));
         members[(bx / PM_GRID_SB) + (size_t)ns[0] * ((by / PM_GRID_SB) + (size_t)ns[1] * (bz / PM_GRID_SB))].push_back((int32_t)b);
       }
-      std::vector<int2> h_rng;
-      std::vector<int32_t> h_blk;
-      std::vector<float> h_sbox;
+      std::vector<float4> h_rec, h_blk;
+      auto bits = [](int v) {
+        float f;
+        std::memcpy(&f, &v, 4);
+        return f;
+      };
       for (auto& m : members) {
         if (m.empty()) continue;
         float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -667,19 +669,20 @@ cudaError_t grid_build(GridBuild& g, cudaStream_t s) {
             lo[a] = std::min(lo[a], h_box[6 * (size_t)b + a]);
             hi[a] = std::max(hi[a], h_box[6 * (size_t)b + 3 + a]);
           }
-        h_rng.push_back(make_int2((int)h_blk.size(), (int)(h_blk.size() + m.size())));
-        h_blk.insert(h_blk.end(), m.begin(), m.end());
-        for (int a = 0; a < 3; a++) h_sbox.push_back(lo[a]);
-        for (int a = 0; a < 3; a++) h_sbox.push_back(hi[a]);
+        h_rec.push_back(make_float4(lo[0], lo[1], lo[2], bits((int)(h_blk.size() / 2))));
+        for (int32_t b : m) {
+          const float* x = &h_box[6 * (size_t)b];
+          h_blk.push_back(make_float4(x[0], x[1], x[2], bits(h_occ[2 * (size_t)b])));
+          h_blk.push_back(make_float4(x[3], x[4], x[5], bits(h_occ[2 * (size_t)b + 1])));
+        }
+        h_rec.push_back(make_float4(hi[0], hi[1], hi[2], bits((int)(h_blk.size() / 2))));
       }
-      n_sb = (int32_t)h_rng.size();
-      if ((e = keep(std::max<size_t>(h_rng.size(), 1) * 8, (void**)&sb_rng)) != cudaSuccess) break;
-      if ((e = keep(std::max<size_t>(h_blk.size(), 1) * 4, (void**)&sb_blk)) != cudaSuccess) break;
-      if ((e = keep(std::max<size_t>(h_sbox.size(), 1) * 4, (void**)&sb_box)) != cudaSuccess) break;
+      n_sb = (int32_t)(h_rec.size() / 2);
+      if ((e = keep(std::max<size_t>(h_rec.size(), 1) * sizeof(float4), (void**)&sb_rec)) != cudaSuccess) break;
+      if ((e = keep(std::max<size_t>(h_blk.size(), 1) * sizeof(float4), (void**)&sb_blk)) != cudaSuccess) break;
       if (n_sb > 0) {
-        if ((e = cudaMemcpyAsync(sb_rng, h_rng.data(), h_rng.size() * 8, cudaMemcpyHostToDevice, s)) != cudaSuccess) break;
-        if ((e = cudaMemcpyAsync(sb_blk, h_blk.data(), h_blk.size() * 4, cudaMemcpyHostToDevice, s)) != cudaSuccess) break;
-        if ((e = cudaMemcpyAsync(sb_box, h_sbox.data(), h_sbox.size() * 4, cudaMemcpyHostToDevice, s)) != cudaSuccess) break;
+        if ((e = cudaMemcpyAsync(sb_rec, h_rec.data(), h_rec.size() * sizeof(float4), cudaMemcpyHostToDevice, s)) != cudaSuccess) break;
+        if ((e = cudaMemcpyAsync(sb_blk, h_blk.data(), h_blk.size() * sizeof(float4), cudaMemcpyHostToDevice, s)) != cudaSuccess) break;
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) break;  // the host vectors go out of scope
       }
     }
@@ -722,9 +725,8 @@ cudaError_t grid_build(GridBuild& g, cudaStream_t s) {
       v.cand_box = nullptr;
       v.cl_rng = nullptr;
       v.cl_ent = nullptr;
-      v.sb_rng = sb_rng;
+      v.sb_rec = sb_rec;
       v.sb_blk = sb_blk;
-      v.sb_box = sb_box;
       v.n_sb = n_sb;
       v.px = px;
       v.py = py;
@@ -830,9 +832,8 @@ cudaError_t grid_build(GridBuild& g, cudaStream_t s) {
   d.cand_box = cand_box;
   d.cl_rng = cl_rng;
   d.cl_ent = cl_ent;
-  d.sb_rng = sb_rng;
+  d.sb_rec = sb_rec;
   d.sb_blk = sb_blk;
-  d.sb_box = sb_box;
   d.n_sb = n_sb;
   g.n_cell_list = n_cl;
   g.n_occupied = n_rec;

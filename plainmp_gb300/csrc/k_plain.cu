@@ -518,13 +518,9 @@ __device__ double eval_ext_warp(const TView& v, const Image& im, const TeamPose&
   const double r = v.sr[k];
   double g3[3];
   if (Q.kind == PM_SDF_CLOUD) {
-    for (int i = 0; i < 3; i++) {
-      D3 pc = sc;
-      if (i == 0) pc.x += 1e-6;
-      if (i == 1) pc.y += 1e-6;
-      if (i == 2) pc.z += 1e-6;
-      g3[i] = ((prim_eval_warp(Q, v.C, pc) - r) - best.val) / 1e-6;
-    }
+    double d3[3] = {INFINITY, INFINITY, INFINITY};
+    warp_nearest64<3>(v.C[Q.cloud], sc, INFINITY, -1, d3);
+    for (int i = 0; i < 3; i++) g3[i] = (((sqrt(d3[i]) - Q.a) - r) - best.val) / 1e-6;
   } else {  // a lane per axis
     D3 pc = sc;
     if (lane == 0) pc.x += 1e-6;
@@ -616,9 +612,10 @@ __device__ double eval_self_warp(const TView& v, const Image& im, const TeamPose
   return best.val;
 }
 
-// NC configurations per block, a warp each.
+// NC configurations per block, two warps each: one for the row against the environment, one for the
+// self-collision row.
 template <int NC>
-__global__ void __launch_bounds__(NC * 32, 512 / (NC * 32)) k_evaluate64(const PmTablesHdr* __restrict__ T, const double* __restrict__ state,
+__global__ void __launch_bounds__(NC * 64, 512 / (NC * 64)) k_evaluate64(const PmTablesHdr* __restrict__ T, const double* __restrict__ state,
                                                         const double* __restrict__ q, int64_t B, int high_accuracy,
                                                         double* __restrict__ vals, double* __restrict__ jac) {
   extern __shared__ __align__(16) double team_mem[];
@@ -628,23 +625,17 @@ __global__ void __launch_bounds__(NC * 32, 512 / (NC * 32)) k_evaluate64(const P
   const int64_t c0 = (int64_t)blockIdx.x * NC;
   const int ncfg = (int)min((int64_t)NC, B - c0);
   float* p32 = reinterpret_cast<float*>(team_mem + (size_t)NC * nsl * kRec);
-  fk64_block<NC * 32>(v, state, [&](int c, int col) { return q[(c0 + c) * qd + col]; }, ncfg, !high_accuracy, team_mem, p32);
-  const int c = threadIdx.x >> 5;
+  fk64_block<NC * 64>(v, state, [&](int c, int col) { return q[(c0 + c) * qd + col]; }, ncfg, !high_accuracy, team_mem, p32);
+  const int c = threadIdx.x >> 6;
   if (c >= ncfg) return;
   const TeamPose P{team_mem + (size_t)c * nsl * kRec, p32 + (size_t)c * nsl * kRec32};
-  const int m = (T->n_prims > 0 ? 1 : 0) + (T->n_pairs > 0 ? 1 : 0);
-  double* vb = vals + (c0 + c) * m;
-  double* jb = jac + (c0 + c) * (int64_t)m * qd;
-  int head = 0;
-  if (T->n_prims > 0) {
-    const double val = eval_ext_warp(v, im, P, jb);
-    if ((threadIdx.x & 31) == 0) vb[0] = val;
-    head++;
-  }
-  if (T->n_pairs > 0) {
-    const double val = eval_self_warp(v, im, P, jb + head * qd);
-    if ((threadIdx.x & 31) == 0) vb[head] = val;
-  }
+  const int ext = T->n_prims > 0 ? 1 : 0, m = ext + (T->n_pairs > 0 ? 1 : 0);
+  const bool self = (threadIdx.x >> 5) & 1;
+  if (self ? T->n_pairs <= 0 : !ext) return;
+  const int row = self ? ext : 0;
+  double* g = jac + ((c0 + c) * m + row) * (int64_t)qd;
+  const double val = self ? eval_self_warp(v, im, P, g) : eval_ext_warp(v, im, P, g);
+  if ((threadIdx.x & 31) == 0) vals[(c0 + c) * m + row] = val;
 }
 
 // Per-sphere signed distances in two launches: the FP64 sphere centres (one thread per configuration:
@@ -848,8 +839,8 @@ cudaError_t launch_evaluate64(const PmTablesHdr* T, const PmTablesHdr& h, const 
   int n_sm = 0;
   const cudaError_t e = sm_count(&n_sm);
   if (e != cudaSuccess) return e;
-  if (B <= 4 * (int64_t)n_sm) return team_launch(k_evaluate64<1>, B, 1, 1, h, s, T, state, q, B, high_accuracy, vals, jac);
-  return team_launch(k_evaluate64<4>, (B + 3) / 4, 4, 1, h, s, T, state, q, B, high_accuracy, vals, jac);
+  if (B <= 4 * (int64_t)n_sm) return team_launch(k_evaluate64<1>, B, 1, 2, h, s, T, state, q, B, high_accuracy, vals, jac);
+  return team_launch(k_evaluate64<4>, (B + 3) / 4, 4, 2, h, s, T, state, q, B, high_accuracy, vals, jac);
 }
 cudaError_t launch_sphere_dist64(const PmTablesHdr* T, const PmTablesHdr& h, const double* state, const double* q, int64_t B,
                                  int high_accuracy, double* dist, double* centres, cudaStream_t s) {

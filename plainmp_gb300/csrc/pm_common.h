@@ -107,9 +107,10 @@ struct PmGridDev {
                            // distance between that record's box and the listing cell's box, in units of
                            // cell / PM_CL_UNITS, rounded down and capped at 255 (high 8 bits); a cell's list holds
                            // every occupied cell that can contain the nearest point of a query inside it
-  const int2* sb_rng;      // per non-empty super-block (PM_GRID_SB^3 blocks): [first, end) of its occupied blocks in sb_blk
-  const int32_t* sb_blk;   // occupied blocks, grouped by super-block
-  const float* sb_box;     // per non-empty super-block: box of its points (lo xyz, hi xyz)
+  const float4* sb_rec;    // per non-empty super-block (PM_GRID_SB^3 blocks): box of its points and its entries in
+                           // sb_blk, (lo xyz, first as int bits), (hi xyz, end)
+  const float4* sb_blk;    // occupied blocks, grouped by super-block: box and occupied-cell records, (lo xyz, first),
+                           // (hi xyz, end)
   int32_t n_sb;            // non-empty super-blocks
   int32_t pad_sb;
   // FP32 copies for the FP32 queries (no FP64 arithmetic on their path): origin, block edge and

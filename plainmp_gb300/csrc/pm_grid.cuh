@@ -89,12 +89,16 @@ __device__ inline bool list_nearest64(const PmGridDev& G, const D3& q, NNResult6
 // super-block whose box is closer than the best; inside one, its occupied blocks, their cells and
 // points, each skipped when its box is not closer than the best.
 __device__ inline void sb_nearest64(const PmGridDev& G, const D3& q, NNResult64& r) {
+  auto box2 = [&](const float4* rec) {  // a record's box
+    const float4 lo = __ldg(rec), hi = __ldg(rec + 1);
+    const double gx = gap64(q.x, (double)lo.x, (double)hi.x), gy = gap64(q.y, (double)lo.y, (double)hi.y), gz = gap64(q.z, (double)lo.z, (double)hi.z);
+    return gx * gx + (gy * gy + gz * gz);
+  };
   auto visit = [&](int j) {
-    const int2 br = __ldg(G.sb_rng + j);
-    for (int k = br.x; k < br.y; k++) {
-      const int b = __ldg(G.sb_blk + k);
-      if (box_d2_64(G.blk_box + 6 * (int64_t)b, q) >= r.d2) continue;
-      const int c0 = G.blk_occ[2 * b], c1 = G.blk_occ[2 * b + 1];
+    const int k1 = __float_as_int(__ldg(G.sb_rec + 2 * j + 1).w);
+    for (int k = __float_as_int(__ldg(G.sb_rec + 2 * j).w); k < k1; k++) {
+      if (box2(G.sb_blk + 2 * (int64_t)k) >= r.d2) continue;
+      const int c0 = __float_as_int(__ldg(G.sb_blk + 2 * (int64_t)k).w), c1 = __float_as_int(__ldg(G.sb_blk + 2 * (int64_t)k + 1).w);
       for (int c = c0; c < c1; c++) {
         if (box_d2_64(G.cell_box + 6 * (int64_t)c, q) >= r.d2) continue;
         const int p0 = G.cell_pts[2 * c], p1 = G.cell_pts[2 * c + 1];
@@ -112,7 +116,7 @@ __device__ inline void sb_nearest64(const PmGridDev& G, const D3& q, NNResult64&
   double lb_min = INFINITY;
   int j_min = -1;
   for (int j = 0; j < G.n_sb; j++) {
-    const double lb = box_d2_64(G.sb_box + 6 * (int64_t)j, q);
+    const double lb = box2(G.sb_rec + 2 * j);
     if (lb < lb_min) {
       lb_min = lb;
       j_min = j;
@@ -121,7 +125,7 @@ __device__ inline void sb_nearest64(const PmGridDev& G, const D3& q, NNResult64&
   if (j_min < 0 || !(lb_min < r.d2)) return;
   visit(j_min);
   for (int j = 0; j < G.n_sb; j++)
-    if (j != j_min && box_d2_64(G.sb_box + 6 * (int64_t)j, q) < r.d2) visit(j);
+    if (j != j_min && box2(G.sb_rec + 2 * j) < r.d2) visit(j);
 }
 
 // Exact FP64 nearest squared distance among the points with squared distance below maxd2

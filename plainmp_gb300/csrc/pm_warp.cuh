@@ -84,7 +84,13 @@ __device__ __forceinline__ FieldStart field_corner_candidate(const float4& rec, 
 // Where q's fine cell has a cell list, the list is scanned, nearest first, 32 entries at a time.
 // Elsewhere the super-block with the nearest box is searched first, then those within the threshold.
 // hint: a point index whose distance starts the search (e.g. the FP32 nearest point), or -1.
-__device__ inline NNResult64 warp_nearest64(const PmGridDev& G, const D3& q, double maxd2 = INFINITY, int hint = -1) {
+//
+// STEPS = 3: the squared distances of q + h e_x, q + h e_y, q + h e_z, h = 1e-6 (the forward differences of a
+// gradient), in one search: a point that FP32 rules out for q by 2h more is ruled out for all three, and the
+// points that are left get three FP64 distances.  d3 receives them; maxd2 must be INFINITY.
+constexpr double kStep = 1e-6;
+template <int STEPS = 0>
+__device__ inline NNResult64 warp_nearest64(const PmGridDev& G, const D3& q, double maxd2 = INFINITY, int hint = -1, double* d3 = nullptr) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   NNResult64 r{maxd2, -1};
@@ -95,9 +101,10 @@ __device__ inline NNResult64 warp_nearest64(const PmGridDev& G, const D3& q, dou
   const float mag = fabsf(qx) + fabsf(qy) + fabsf(qz) + pmax;
   if (!(mag < 1e15f)) {  // FP32 squares would overflow: the FP64 walk, one lane's result for all
     r = grid_nearest64(G, q, maxd2);
+    for (int i = 0; i < STEPS; i++) d3[i] = grid_nearest64(G, D3{i == 0 ? q.x + kStep : q.x, i == 1 ? q.y + kStep : q.y, i == 2 ? q.z + kStep : q.z}).d2;
     return r;
   }
-  const float tabs = 4e-7f * mag + 1e-12f;
+  const float tabs = 4e-7f * mag + (STEPS ? 1e-6f : 1e-12f);  // 2.5 tabs >= 2h
   auto thr = [&](float d2) {
     const float sb = sqrtf(d2) * (1.0f + 1e-5f) + 2.5f * tabs;
     return sb * sb * (1.0f + 1e-6f);
@@ -107,8 +114,17 @@ __device__ inline NNResult64 warp_nearest64(const PmGridDev& G, const D3& q, dou
   float c32 = INFINITY;  // the lane's unevaluated candidate
   int cand = -1;
   float t = thr((float)maxd2);
+  double b3[STEPS > 0 ? STEPS : 1];
+  for (int i = 0; i < STEPS; i++) b3[i] = INFINITY;
   auto exact = [&](int p) {
-    const D3 d{G.px[p] - q.x, G.py[p] - q.y, G.pz[p] - q.z};
+    const double px = G.px[p], py = G.py[p], pz = G.pz[p];
+    for (int i = 0; i < STEPS; i++) {
+      const D3 d{px - (i == 0 ? q.x + kStep : q.x), py - (i == 1 ? q.y + kStep : q.y), pz - (i == 2 ? q.z + kStep : q.z)};
+      const double d2 = d.x * d.x + (d.y * d.y + d.z * d.z);
+      if (d2 < b3[i]) b3[i] = d2;
+    }
+    if (STEPS > 0) return;
+    const D3 d{px - q.x, py - q.y, pz - q.z};
     const double d2 = d.x * d.x + (d.y * d.y + d.z * d.z);
     if (d2 < best || (d2 == best && bidx >= 0 && p < bidx)) {
       best = d2;
@@ -188,16 +204,15 @@ __device__ inline NNResult64 warp_nearest64(const PmGridDev& G, const D3& q, dou
     }
   } else {
     // one super-block: its occupied blocks nearest first, each block's cells over the lanes
-    auto visit = [&](int j) {
-      const int2 br = __ldg(G.sb_rng + j);
-      for (int base = br.x; base < br.y; base += 32) {  // warp-uniform
+    auto visit = [&](int b0, int b1) {
+      for (int base = b0; base < b1; base += 32) {  // warp-uniform
         const int k = base + lane;
         float lb = INFINITY;
         int2 occ = make_int2(0, 0);
-        if (k < br.y) {
-          const int b = __ldg(G.sb_blk + k);
-          occ = __ldg(reinterpret_cast<const int2*>(G.blk_occ) + b);
-          lb = box_d2_32(G.blk_box + 6 * (int64_t)b, qx, qy, qz);
+        if (k < b1) {
+          const float4 lo = __ldg(G.sb_blk + 2 * k), hi = __ldg(G.sb_blk + 2 * k + 1);
+          occ = make_int2(__float_as_int(lo.w), __float_as_int(hi.w));
+          lb = box2(lo, hi);
         }
         for (;;) {  // warp-uniform: the nearest block left
           const unsigned m = __reduce_min_sync(FULL, __float_as_uint(lb));
@@ -218,38 +233,55 @@ __device__ inline NNResult64 warp_nearest64(const PmGridDev& G, const D3& q, dou
     };
     float lb0 = INFINITY;
     int j0 = -1;
+    int2 r0 = make_int2(0, 0);
     for (int j = lane; j < G.n_sb; j += 32) {
-      const float lb = box_d2_32(G.sb_box + 6 * (int64_t)j, qx, qy, qz);
+      const float4 lo = __ldg(G.sb_rec + 2 * j), hi = __ldg(G.sb_rec + 2 * j + 1);
+      const float lb = box2(lo, hi);
       if (lb < lb0) {
         lb0 = lb;
         j0 = j;
+        r0 = make_int2(__float_as_int(lo.w), __float_as_int(hi.w));
       }
     }
     const unsigned m = __reduce_min_sync(FULL, __float_as_uint(lb0));
-    const unsigned who = __ballot_sync(FULL, __float_as_uint(lb0) == m);
-    j0 = __shfl_sync(FULL, j0, __ffs(who) - 1);
+    const int who = __ffs(__ballot_sync(FULL, __float_as_uint(lb0) == m)) - 1;
+    j0 = __shfl_sync(FULL, j0, who);
+    const int f0 = __shfl_sync(FULL, r0.x, who), f1 = __shfl_sync(FULL, r0.y, who);
     if (j0 >= 0 && __uint_as_float(m) <= t) {
-      visit(j0);
+      visit(f0, f1);
       for (int base = 0; base < G.n_sb; base += 32) {  // warp-uniform
         const int j = base + lane;
-        const float lb = j < G.n_sb && j != j0 ? box_d2_32(G.sb_box + 6 * (int64_t)j, qx, qy, qz) : INFINITY;
+        float lb = INFINITY;
+        int2 br = make_int2(0, 0);
+        if (j < G.n_sb && j != j0) {
+          const float4 lo = __ldg(G.sb_rec + 2 * j), hi = __ldg(G.sb_rec + 2 * j + 1);
+          lb = box2(lo, hi);
+          br = make_int2(__float_as_int(lo.w), __float_as_int(hi.w));
+        }
         for (unsigned bal = __ballot_sync(FULL, lb <= t && lb < INFINITY); bal != 0; bal &= bal - 1) {
           const int src = __ffs(bal) - 1;
           const float l = __shfl_sync(FULL, lb, src);
-          if (l <= t) visit(base + src);  // t is the warp's
+          const int b0 = __shfl_sync(FULL, br.x, src), b1 = __shfl_sync(FULL, br.y, src);
+          if (l <= t) visit(b0, b1);  // t is the warp's
         }
       }
     }
   }
   if (cand >= 0 && !(c32 > t)) exact(cand);
   __syncwarp();
-  // the warp's minimum of (best, index): best >= 0, so its words order like it
-  const unsigned hi = (unsigned)__double2hiint(best), lo = (unsigned)__double2loint(best);
-  const unsigned mh = __reduce_min_sync(FULL, hi);
-  const unsigned ml = __reduce_min_sync(FULL, hi == mh ? lo : 0xffffffffu);
-  const unsigned mi = __reduce_min_sync(FULL, hi == mh && lo == ml ? (unsigned)bidx : 0xffffffffu);
-  r.d2 = __hiloint2double((int)mh, (int)ml);
-  r.idx = (int)mi;
+  // the warp's minima: values >= 0, so their words order like them
+  auto least = [&](double d, unsigned& hi, unsigned& lo) {
+    hi = __reduce_min_sync(FULL, (unsigned)__double2hiint(d));
+    lo = __reduce_min_sync(FULL, (unsigned)__double2hiint(d) == hi ? (unsigned)__double2loint(d) : 0xffffffffu);
+    return __hiloint2double((int)hi, (int)lo);
+  };
+  unsigned mh, ml;
+  if (STEPS > 0) {
+    for (int i = 0; i < STEPS; i++) d3[i] = least(b3[i], mh, ml);
+    return r;
+  }
+  r.d2 = least(best, mh, ml);
+  r.idx = (int)__reduce_min_sync(FULL, (unsigned)__double2hiint(best) == mh && (unsigned)__double2loint(best) == ml ? (unsigned)bidx : 0xffffffffu);
   return r;
 }
 
