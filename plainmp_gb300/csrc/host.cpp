@@ -801,7 +801,7 @@ struct HostCst {
     std::vector<PmSphereF> sp(sr.size());
     for (size_t i = 0; i < sr.size(); i++) {
       const float v[3] = {(float)sx[i], (float)sy[i], (float)sz[i]};
-      sp[i] = PmSphereF{v[0], v[1], v[2], (float)sr[i], sgroup[i], sr[i] < 1e-6, norm_up(v)};
+      sp[i] = PmSphereF{v[0], v[1], v[2], (float)sr[i], sgroup[i], sr[i] < 1e-6, norm_up(v), 0};
     }
     std::vector<PmGroupF> gr(groups.size());
     for (size_t i = 0; i < groups.size(); i++) {
@@ -817,11 +817,7 @@ struct HostCst {
       f.aa = P.axis_aligned;
       f.za = P.z_axis_aligned;
       f.cloud = P.cloud;
-      for (int k = 0; k < 3; k++) {
-        f.lb[k] = (float)P.lb[k];
-        f.ub[k] = (float)P.ub[k];
-        f.pos[k] = (float)P.pos[k];
-      }
+      for (int k = 0; k < 3; k++) f.pos[k] = (float)P.pos[k];
       for (int k = 0; k < 9; k++) f.rot[k] = (float)P.rot[k];
       f.a = (float)P.a;
       f.b = (float)P.b;

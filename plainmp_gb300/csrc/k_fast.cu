@@ -2,7 +2,7 @@
 //
 // Per block of CPB configurations (k_fast_valid; k_fast_edges over the waypoints of edges):
 //   1. FK in FP32 into shared memory, with a running bound on each slot's error against the
-//      FP64 FK of the reference (see fk32); every later margin adds the bound of the spheres
+//      FP64 FK of the reference (see fk_local, fk_chain); every later margin adds the bound of the spheres
 //      involved.  A configuration with a non-finite coordinate goes to the exact FP64 check;
 //   2. group culling: the clearance of each sphere group's bounding sphere against each
 //      primitive (a point cloud: the lower bound of its nearest-point field);
@@ -39,11 +39,14 @@ using PrimF = PmPrimF;
 using SphereF = PmSphereF;
 using GroupF = PmGroupF;
 using SlotF = PmSlotF;
-// Per slot and configuration in shared memory: [0..8] R, [9..11] t, [12] et = bound on |t - t64|,
-// [13] eb = bound on |R - R64| as an operator (8 eq + 24 u), [14..17] world quaternion,
-// [18] eq = bound on |q - q64|_2.  A point s of the link frame then lies within et + eb |s| of
-// its FP64 position, plus the rounding of R s + t that margin32 covers.
-constexpr int kPoseF = 20;
+// Per slot and configuration in shared memory, 16 floats: the rows of (R, t) (xf), then [12] et = bound on
+// |t - t64|, [13] eb = bound on |R - R64| as an operator (8 eq + 24 u, eq = bound on the world quaternion's
+// error).  A point s of the link frame then lies within et + eb |s| of its FP64 position, plus the rounding of
+// R s + t that margin32 covers.  Poses and tables are read with 16-byte loads; a configuration's slots are
+// followed by 4 floats, so that the 4 or more configurations of a row of sphere tasks fall on different banks.
+// While the FK runs, a slot holds its local transform, then its world pose (fk_local, fk_chain, fk_matrix).
+constexpr int kPoseF = 16;
+__host__ __device__ inline int pose_stride(int n_slots) { return n_slots * kPoseF + 4; }
 
 enum { ST_PASS = 0, ST_FAIL = 1, ST_MAYBE = 2 };
 constexpr int FLAG_FAIL = 1;
@@ -107,107 +110,124 @@ __device__ __forceinline__ void approx_sin_cos32_q(double q, float qf, float& s,
   approx_sin_cos32(q * 0.5, s, c);
 }
 
-// FP32 FK of one configuration into P (n_slots x kPoseF) with error bounds against the FP64 FK
-// of the reference (update_kintree + get_link_pose; algorithm.cpp:88-210).  Bounds, u = 2^-24,
-// norms 2-norms, quaternions within 1e-3 of unit norm:
+// FP32 FK with error bounds against the FP64 FK of the reference (update_kintree + get_link_pose;
+// algorithm.cpp:88-210), in three steps: the local transforms of every (configuration, slot) side by side, the
+// serial chain of compositions by two threads per configuration, and the rotation matrices side by side
+// again.  With everything in the chain, its 150 instructions a slot kept one warp of eight busy for a quarter
+// of the block's time.  Bounds, u = 2^-24, norms 2-norms, quaternions within 1e-3 of unit norm:
 //   local rotation: joint quaternion from sin/cos (Taylor: 8u / 12u; sincosf: 2 ulp + the
 //     rounding of x) and an FP32 axis: 20u; times the FP32 origin quaternion: 32u;
 //   composition q = qp (x) lq: |dq| <= 1.001 (|dqp| + |dlq|) + 8.1u (4-term fused sums);
-//   rotation of a vector v by an FP32 matrix of qp: |d(Rv)| <= (8 |dqp| + 24u) |v| (the map
-//     q -> R(q)v has derivative norm <= 6.4 |v| at |q| <= 1.001; matrix and product rounding);
+//   rotation of a vector v by qp: |d(Rv)| <= (8 |dqp| + 24u) |v| (the map q -> R(q)v has derivative norm
+//     <= 6.4 |v| at |q| <= 1.001; the matrix's and the product's rounding, or fqrot's: two crosses of fused
+//     sums, 7u |v| in the first times 1.42, 6u and 2u in the second and the sums, 18u in all);
 //   translation t = tp + R lt: |dt| <= |dtp| + (8 |dqp| + 24u)|lt| + 1.01 u (|tp|_1 + |lt|_1).
 // The base pose adds the rounding of q's base entries (and of their half angles).
-// Field f of slot i is P[(i * kPoseF + f) * stride] (stride 1: a block's shared memory, one
-// configuration's slots in a row).
-// list: the slots to compute, in order (one phase of one thread of the two-thread FK), or null: all
-// nsl.  The two threads of a configuration walk their own lists in step, so a warp computes both
-// threads' k-th slots with one instruction stream.
-__device__ __forceinline__ void fk32(const SlotF* __restrict__ S, int nsl, const float* __restrict__ base8, int base_type, int n_ctrl,
-                                     const double* __restrict__ q, bool taylor, float* __restrict__ P, int64_t stride = 1,
-                                     const unsigned char* list = nullptr) {
-  for (int k = 0; k < nsl; k++) {
-    const int i = list ? list[k] : k;
-    const SlotF s = S[i];
-    float* o = P + (int64_t)i * kPoseF * stride;
+//
+// The local transform of a slot into o: [0..3] quaternion, [4..6] translation, [7] identity flag, [8] the
+// quaternion's error, [9] the translation's, [10] |t|_1, [11] |t| rounded up; a root's world pose as fk_chain
+// leaves it.  qv(col): a value of the configuration.
+template <class QV>
+__device__ __forceinline__ void fk_local(const SlotF& s, const float* __restrict__ base8, int base_type, int n_ctrl, const QV& qv, bool taylor,
+                                         float4* __restrict__ o) {
+  if (s.parent < 0) {
     FQ wq;
-    float wt[3], eq, et;
-    if (s.parent < 0) {
-      if (base_type == PM_BASE_PLANAR) {
-        const double hy = q[n_ctrl + 2] * 0.5;
-        float sy, cy;
-        sincosf((float)hy, &sy, &cy);
-        wq = FQ{0.f, 0.f, sy, cy};
-        wt[0] = (float)q[n_ctrl];
-        wt[1] = (float)q[n_ctrl + 1];
-        wt[2] = 0.f;
-        eq = kU * (8.0f + 2.0f * fabsf((float)hy));
-      } else if (base_type == PM_BASE_FLOATING) {
-        const double hr = q[n_ctrl + 3] * 0.5, hp = q[n_ctrl + 4] * 0.5, hy = q[n_ctrl + 5] * 0.5;
-        float sr, cr, sp, cp, sy, cy;
-        sincosf((float)hr, &sr, &cr);
-        sincosf((float)hp, &sp, &cp);
-        sincosf((float)hy, &sy, &cy);
-        wq = FQ{sr * cp * cy - cr * sp * sy, cr * sp * cy + sr * cp * sy, cr * cp * sy - sr * sp * cy, cr * cp * cy + sr * sp * sy};
-        for (int k = 0; k < 3; k++) wt[k] = (float)q[n_ctrl + k];
-        eq = kU * (40.0f + 4.0f * (fabsf((float)hr) + fabsf((float)hp) + fabsf((float)hy)));
-      } else {
-        wq = FQ{base8[0], base8[1], base8[2], base8[3]};
-        for (int k = 0; k < 3; k++) wt[k] = base8[4 + k];
-        eq = 2.0f * kU;
-      }
-      et = kU * (fabsf(wt[0]) + fabsf(wt[1]) + fabsf(wt[2]));
+    float wt[3], eq;
+    if (base_type == PM_BASE_PLANAR) {
+      const double hy = qv(n_ctrl + 2) * 0.5;
+      float sy, cy;
+      sincosf((float)hy, &sy, &cy);
+      wq = FQ{0.f, 0.f, sy, cy};
+      wt[0] = (float)qv(n_ctrl);
+      wt[1] = (float)qv(n_ctrl + 1);
+      wt[2] = 0.f;
+      eq = kU * (8.0f + 2.0f * fabsf((float)hy));
+    } else if (base_type == PM_BASE_FLOATING) {
+      const double hr = qv(n_ctrl + 3) * 0.5, hp = qv(n_ctrl + 4) * 0.5, hy = qv(n_ctrl + 5) * 0.5;
+      float sr, cr, sp, cp, sy, cy;
+      sincosf((float)hr, &sr, &cr);
+      sincosf((float)hp, &sp, &cp);
+      sincosf((float)hy, &sy, &cy);
+      wq = FQ{sr * cp * cy - cr * sp * sy, cr * sp * cy + sr * cp * sy, cr * cp * sy - sr * sp * cy, cr * cp * cy + sr * sp * sy};
+      for (int k = 0; k < 3; k++) wt[k] = (float)qv(n_ctrl + k);
+      eq = kU * (40.0f + 4.0f * (fabsf((float)hr) + fabsf((float)hp) + fabsf((float)hy)));
     } else {
-      const float* pp = P + (int64_t)s.parent * kPoseF * stride;
-      const FQ pq{pp[(14) * stride], pp[(15) * stride], pp[(16) * stride], pp[(17) * stride]};
-      FQ lq{0.f, 0.f, 0.f, 1.f};
-      float lt[3] = {s.lt[0], s.lt[1], s.lt[2]};
-      float el = 0.f, elt = kU * s.lt1, lt1 = s.lt1;
-      bool lid = s.lid != 0;
-      if (s.mode == PM_FK_STATE) {
-        lq = FQ{s.lq[0], s.lq[1], s.lq[2], s.lq[3]};
-        el = 2.0f * kU;
-      } else if (s.mode == PM_FK_PRIS) {
-        const float th = (float)q[s.qcol];
-        for (int k = 0; k < 3; k++) lt[k] = fmaf(s.axis[k], th, s.lt[k]);
-        lt1 = fabsf(lt[0]) + fabsf(lt[1]) + fabsf(lt[2]);
-        elt = 4.0f * kU * (s.lt1 + fabsf(th) * (fabsf(s.axis[0]) + fabsf(s.axis[1]) + fabsf(s.axis[2])));
-        lid = true;
-      } else {
-        const double qd = q[s.qcol];
-        const float qf = (float)qd, xf = qf * 0.5f;  // (float)(qd / 2), exactly
-        float sn, cs;
-        if (taylor) {
-          approx_sin_cos32_q(qd, qf, sn, cs);
-        } else {
-          sincosf(xf, &sn, &cs);
-        }
-        const FQ jq{sn * s.axis[0], sn * s.axis[1], sn * s.axis[2], cs};
-        lq = lid ? jq : fqmul(FQ{s.lq[0], s.lq[1], s.lq[2], s.lq[3]}, jq);
-        el = (lid ? 20.0f : 32.0f) * kU + (taylor ? 0.0f : 2.0f * kU * fabsf(xf));
-        lid = false;
-      }
-      wq = lid ? pq : fqmul(pq, lq);
-      for (int k = 0; k < 3; k++)
-        wt[k] = pp[(9 + k) * stride] + fmaf(pp[(3 * k) * stride], lt[0], fmaf(pp[(3 * k + 1) * stride], lt[1], pp[(3 * k + 2) * stride] * lt[2]));
-      const float peq = pp[(18) * stride];
-      eq = lid ? peq + el : 1.001f * (peq + el) + 8.1f * kU;
-      const float nlt = sqrtf(fmaf(lt[0], lt[0], fmaf(lt[1], lt[1], lt[2] * lt[2]))) * 1.001f;
-      et = pp[(12) * stride] + nlt * pp[(13) * stride] + 1.01f * kU * (fabsf(pp[(9) * stride]) + fabsf(pp[(10) * stride]) + fabsf(pp[(11) * stride]) + lt1) + elt;
+      wq = FQ{base8[0], base8[1], base8[2], base8[3]};
+      for (int k = 0; k < 3; k++) wt[k] = base8[4 + k];
+      eq = 2.0f * kU;
     }
-    float R[9];
-    fqmat(wq, R);
-    for (int k = 0; k < 9; k++) o[k * stride] = R[k];
-    o[9 * stride] = wt[0];
-    o[10 * stride] = wt[1];
-    o[11 * stride] = wt[2];
-    o[12 * stride] = et;
-    o[13 * stride] = 8.0f * eq + 24.0f * kU;
-    o[14 * stride] = wq.x;
-    o[15 * stride] = wq.y;
-    o[16 * stride] = wq.z;
-    o[17 * stride] = wq.w;
-    o[18 * stride] = eq;
+    o[0] = make_float4(wq.x, wq.y, wq.z, wq.w);
+    o[1] = make_float4(wt[0], wt[1], wt[2], kU * (fabsf(wt[0]) + fabsf(wt[1]) + fabsf(wt[2])));
+    o[2].x = eq;
+    return;
   }
+  FQ lq{0.f, 0.f, 0.f, 1.f};
+  float lt[3] = {s.lt[0], s.lt[1], s.lt[2]};
+  float el = 0.f, elt = kU * s.lt1, lt1 = s.lt1;
+  bool lid = s.lid != 0;
+  if (s.mode == PM_FK_STATE) {
+    lq = FQ{s.lq[0], s.lq[1], s.lq[2], s.lq[3]};
+    el = 2.0f * kU;
+  } else if (s.mode == PM_FK_PRIS) {
+    const float th = (float)qv(s.qcol);
+    for (int k = 0; k < 3; k++) lt[k] = fmaf(s.axis[k], th, s.lt[k]);
+    lt1 = fabsf(lt[0]) + fabsf(lt[1]) + fabsf(lt[2]);
+    elt = 4.0f * kU * (s.lt1 + fabsf(th) * (fabsf(s.axis[0]) + fabsf(s.axis[1]) + fabsf(s.axis[2])));
+    lid = true;
+  } else {
+    const double qd = qv(s.qcol);
+    const float qf = (float)qd, xf = qf * 0.5f;  // (float)(qd / 2), exactly
+    float sn, cs;
+    if (taylor) {
+      approx_sin_cos32_q(qd, qf, sn, cs);
+    } else {
+      sincosf(xf, &sn, &cs);
+    }
+    const FQ jq{sn * s.axis[0], sn * s.axis[1], sn * s.axis[2], cs};
+    lq = lid ? jq : fqmul(FQ{s.lq[0], s.lq[1], s.lq[2], s.lq[3]}, jq);
+    el = (lid ? 20.0f : 32.0f) * kU + (taylor ? 0.0f : 2.0f * kU * fabsf(xf));
+    lid = false;
+  }
+  o[0] = make_float4(lq.x, lq.y, lq.z, lq.w);
+  o[1] = make_float4(lt[0], lt[1], lt[2], lid ? 1.0f : 0.0f);
+  o[2] = make_float4(el, elt, lt1, sqrtf(fmaf(lt[0], lt[0], fmaf(lt[1], lt[1], lt[2] * lt[2]))) * 1.001f);
+}
+
+// The slots of `list` (n, parents first) of one configuration, composed onto their parents in place: world
+// quaternion [0..3], translation [4..6], et [7], eq [8].  The two threads of a configuration walk their own
+// lists in step, so a warp composes both threads' k-th slots with one instruction stream.
+__device__ __forceinline__ void fk_chain(const SlotF* __restrict__ S, int n, const unsigned char* list, float* __restrict__ P) {
+  for (int k = 0; k < n; k++) {
+    const int i = list[k], parent = S[i].parent;
+    if (parent < 0) continue;
+    float4* o = reinterpret_cast<float4*>(P + i * kPoseF);
+    const float4* pp = reinterpret_cast<const float4*>(P + parent * kPoseF);
+    const float4 p0 = pp[0], p1 = pp[1], l0 = o[0], l1 = o[1], l2 = o[2];
+    const float peq = pp[2].x;
+    const FQ pq{p0.x, p0.y, p0.z, p0.w};
+    const bool lid = l1.w != 0.f;
+    const float lt[3] = {l1.x, l1.y, l1.z};
+    float r[3];
+    fqrot(pq, lt, r);
+    const FQ wq = lid ? pq : fqmul(pq, FQ{l0.x, l0.y, l0.z, l0.w});
+    const float et = p1.w + l2.w * (8.0f * peq + 24.0f * kU) + 1.01f * kU * (fabsf(p1.x) + fabsf(p1.y) + fabsf(p1.z) + l2.z) + l2.y;
+    o[0] = make_float4(wq.x, wq.y, wq.z, wq.w);
+    o[1] = make_float4(p1.x + r[0], p1.y + r[1], p1.z + r[2], et);
+    o[2].x = lid ? peq + l2.x : 1.001f * (peq + l2.x) + 8.1f * kU;
+  }
+}
+
+// The slot's final form.
+__device__ __forceinline__ void fk_matrix(float* __restrict__ o) {
+  float4* p = reinterpret_cast<float4*>(o);
+  const float4 q = p[0], t = p[1];
+  const float eq = o[8];
+  float R[9];
+  fqmat(FQ{q.x, q.y, q.z, q.w}, R);
+  p[0] = make_float4(R[0], R[1], R[2], t.x);
+  p[1] = make_float4(R[3], R[4], R[5], t.y);
+  p[2] = make_float4(R[6], R[7], R[8], t.z);
+  p[3] = make_float4(t.w, 8.0f * eq + 24.0f * kU, 0.f, 0.f);
 }
 
 // Block offsets (dx, dy, dz) with max |d| <= kOffR, sorted by the minimum distance between two
@@ -587,14 +607,13 @@ __device__ __forceinline__ void push_item(const Scratch& s, const Src& src, int6
 }
 
 struct Smem {
-  double* qbuf;  // generated configurations (edges)
   int2* hq;      // hard cloud queries: (cfg << 16 | sphere, primitive)
   unsigned char* fkl;  // the two-thread FK's slot lists: [0, 64) phase 0, [64, 128) and [128, 192) the
                        // two threads of phase 1; fkn[0..2] their lengths
   int* fkn;
   int* hq_n;     // [0] pushed, [1] popped
   int* sdist;    // per (cfg, sphere): running minimum signed distance, order-preserving int
-  float* pose;   // [cfg][slot][kPoseF]
+  float* pose;   // [cfg][pose_stride]: [slot][kPoseF]
   SlotF* slot;
   float* base8;  // fixed base pose: q xyzw, t xyz
   SphereF* sph;
@@ -615,7 +634,7 @@ struct CfgSource {  // a batch of configurations q[B x q_dim]
   // one value of a configuration (locate: what a source needs to find out once per configuration)
   __device__ int locate(int64_t) const { return 0; }
   __device__ double value(const PmTablesHdr* T, int, int64_t i, int col) const { return q[i * T->q_dim + col]; }
-  __device__ bool pre_skip(int64_t) const { return false; }     // before the fast pass: nothing known
+  __device__ bool pre_skip(int64_t, int) const { return false; }  // before the fast pass: nothing known
   __device__ bool skip(int64_t i) const { return out[i] == 0; }  // after it: already invalid
   __device__ void fail(int64_t i) const { out[i] = 0; }
   __device__ void done(int64_t i, bool failed) const { out[i] = failed ? 0 : 1; }
@@ -677,7 +696,7 @@ struct EdgeSource {
     for (int i = 0; i < d; i++) buf[i] = a[i] + (b[i] - a[i]) * t;
     return buf;
   }
-  __device__ bool pre_skip(int64_t w) const { return valid[edge_of(w)] == 0; }
+  __device__ bool pre_skip(int64_t, const Where& p) const { return valid[p.e] == 0; }
   __device__ bool skip(int64_t w) const { return valid[edge_of(w)] == 0; }
   __device__ void fail(int64_t w) const { valid[edge_of(w)] = 0; }
   __device__ void done(int64_t w, bool failed) const {
@@ -693,51 +712,46 @@ struct EdgeSource {
   }
 };
 
-// Phases 1-3 for the configurations [c0, c0 + ncfg) of a source.  qbuf holds CPB * q_dim
-// doubles of shared memory for generated configurations.
+// Phases 1-3 for the configurations [c0, c0 + ncfg) of a source.  The block's flags are zero on entry and on
+// return.
 template <int CPB, class Src>
 __device__ void fast_block(const TView& v, const Smem& sm, const double* __restrict__ state, const Src& src, int64_t c0, int ncfg,
-                           float* __restrict__ dist32, float cutoff, const Scratch& scr, double* qbuf) {
+                           float* __restrict__ dist32, float cutoff, const Scratch& scr) {
   const PmTablesHdr* T = v.T;
-  const int ns = T->n_spheres, ng = T->n_groups, np = T->n_prims, npr = T->n_pairs, nsl = T->n_slots;
+  const int ns = T->n_spheres, ng = T->n_groups, np = T->n_prims, npr = T->n_pairs, nsl = T->n_slots, pst = pose_stride(nsl);
   const int tid = threadIdx.x;
-  // ---- 1. FK (FP32, with error bounds) -> shared memory, two threads per configuration (threads 2c
-  //         and 2c + 1): the trunk of the slot tree by the first, then one subtree set each (the
-  //         host's split); the configuration goes to qbuf so that both threads read it
+  // ---- 1. FK (FP32, with error bounds) -> shared memory: a task per (configuration, slot or value)
   {
-    const int fc = tid >> 1, fth = tid & 1;
-    const int qd = T->q_dim;
-    const bool taylor = T->base_type == PM_BASE_FIXED;
-    float* P = sm.pose + (size_t)fc * nsl * kPoseF;
-    if (fth == 0 && fc < CPB) {
-      int fl = 0;
-      if (fc < ncfg) {
-        if (src.pre_skip(c0 + fc)) {
-          fl = FLAG_FAIL | 2;  // already known invalid: no work
-        } else {
-          double* qb = qbuf + fc * qd;
-          const double* qc = src.cfg(T, c0 + fc, qb);
-          bool finite = true;
-          for (int i = 0; i < qd; i++) {
-            const double x = qc[i];
-            finite = finite && finite64(x);
-            qb[i] = x;
-          }
-          if (finite) {
-            fk32(sm.slot, sm.fkn[0], sm.base8, T->base_type, T->n_ctrl, qb, taylor, P, 1, sm.fkl);
-          } else {
-            // a NaN or infinite coordinate makes every FP32 bound NaN, and no decision would be taken:
-            // the exact FP64 check of the recheck kernel decides, as for an overflowing queue
-            fl = 2;
-            scr.overflow[src.overflow_slot(c0 + fc)] = 1;
-          }
+    const int qd = T->q_dim, width = max(nsl, qd);
+    for (int t = tid; t < CPB * width; t += blockDim.x) {  // the configuration fastest: their poses lie on different banks
+      const int c = t & (CPB - 1), j = t / CPB;
+      if (c >= ncfg) continue;
+      const auto where = src.locate(c0 + c);
+      if (j == 0 && src.pre_skip(c0 + c, where)) atomicOr(&sm.flags[c], FLAG_FAIL | 2);  // already known invalid: no work
+      if (j < qd && !finite64(src.value(T, where, c0 + c, j))) {
+        // a NaN or infinite coordinate makes every FP32 bound NaN, and no decision would be taken:
+        // the exact FP64 check of the recheck kernel decides, as for an overflowing queue
+        if (!src.pre_skip(c0 + c, where)) {
+          atomicOr(&sm.flags[c], 2);
+          scr.overflow[src.overflow_slot(c0 + c)] = 1;
         }
       }
-      sm.flags[fc] = fl;
+      if (j < nsl)
+        fk_local(sm.slot[j], sm.base8, T->base_type, T->n_ctrl, [&](int col) { return src.value(T, where, c0 + c, col); },
+                 T->base_type == PM_BASE_FIXED, reinterpret_cast<float4*>(sm.pose + c * pst + j * kPoseF));
     }
     __syncthreads();
-    if (fc < ncfg && !(sm.flags[fc] & 2))
-      fk32(sm.slot, sm.fkn[1 + fth], sm.base8, T->base_type, T->n_ctrl, qbuf + fc * qd, taylor, P, 1, sm.fkl + (1 + fth) * PM_MAX_SLOTS);
+    const int fc = tid >> 1, fth = tid & 1;  // threads 2c and 2c + 1 (the same warp): the trunk, then a subtree set each
+    if (tid < 2 * CPB) {  // whole warps
+      const bool on = fc < ncfg && !(sm.flags[fc] & 2);
+      float* P = sm.pose + fc * pst;
+      if (on && fth == 0) fk_chain(sm.slot, sm.fkn[0], sm.fkl, P);
+      __syncwarp();
+      if (on) fk_chain(sm.slot, sm.fkn[1 + fth], sm.fkl + (1 + fth) * PM_MAX_SLOTS, P);
+    }
+    __syncthreads();
+    for (int t = tid; t < CPB * nsl; t += blockDim.x)
+      if ((t & (CPB - 1)) < ncfg) fk_matrix(sm.pose + (t & (CPB - 1)) * pst + (t / CPB) * kPoseF);
   }
   __syncthreads();
   const bool want_dist = dist32 != nullptr;
@@ -749,8 +763,8 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
     const int c = t / nb, k = t - c * nb;
     if (sm.flags[c] & 2) continue;
     const PmPoseTerm& b = src.bnd.t[k];
-    const float* P = sm.pose + ((size_t)c * nsl + b.slot) * kPoseF;
-    const float x = P[9 + b.axis];
+    const float* P = sm.pose + c * pst + b.slot * kPoseF;
+    const float x = P[4 * b.axis + 3];
     const float lo = (float)b.lb, hi = (float)b.ub;
     // the FK error bound, plus the rounding of the bounds to FP32 and of the comparison
     const float m = P[12] + margin32(fabsf(x) + (b.has_lb ? fabsf(lo) : 0.f) + (b.has_ub ? fabsf(hi) : 0.f));
@@ -763,7 +777,7 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
     const int c = t / ng, gi = t - c * ng;
     if (sm.flags[c] & 2) continue;
     const GroupF& G = sm.grp[gi];
-    const float* P = sm.pose + ((size_t)c * nsl + G.slot) * kPoseF;
+    const float* P = sm.pose + c * pst + G.slot * kPoseF;
     float3 gc = xf(P, G.rel[0], G.rel[1], G.rel[2]);
     const float ekg = P[12] + P[13] * G.gn;  // FK error bound of the group centre
     unsigned mask = 0;
@@ -814,7 +828,7 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
       if (want_dist) sm.sdist[c * ns + si] = f2o(cutoff);
       return;
     }
-    const float* P = sm.pose + ((size_t)c * nsl + G.slot) * kPoseF;
+    const float* P = sm.pose + c * pst + G.slot * kPoseF;
     const float3 sc = xf(P, S.x, S.y, S.z);
     const float ek = P[12] + P[13] * S.sn;  // FK error bound of the sphere centre
     float sdmin = cutoff;
@@ -884,8 +898,8 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
         const int2 pr = sm.pairs[pi];
         const GroupF& G1 = sm.grp[pr.x];
         const GroupF& G2 = sm.grp[pr.y];
-        const float* P1 = sm.pose + ((size_t)c * nsl + G1.slot) * kPoseF;
-        const float* P2 = sm.pose + ((size_t)c * nsl + G2.slot) * kPoseF;
+        const float* P1 = sm.pose + c * pst + G1.slot * kPoseF;
+        const float* P2 = sm.pose + c * pst + G2.slot * kPoseF;
         const float3 a = xf(P1, G1.rel[0], G1.rel[1], G1.rel[2]);
         const float3 bb = xf(P2, G2.rel[0], G2.rel[1], G2.rel[2]);
         const float ddx = a.x - bb.x, ddy = a.y - bb.y, ddz = a.z - bb.z;
@@ -905,8 +919,8 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
       const int2 pr = sm.pairs[pi];
       const GroupF& G1 = sm.grp[pr.x];
       const GroupF& G2 = sm.grp[pr.y];
-      const float* P1 = sm.pose + ((size_t)c * nsl + G1.slot) * kPoseF;
-      const float* P2 = sm.pose + ((size_t)c * nsl + G2.slot) * kPoseF;
+      const float* P1 = sm.pose + c * pst + G1.slot * kPoseF;
+      const float* P2 = sm.pose + c * pst + G2.slot * kPoseF;
       int fail = 0;
       for (int jb = 0; jb < G2.count; jb += 8) {
         const int j = jb + (lane & 7);
@@ -954,7 +968,7 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
         const SphereF S = sm.sph[si];
         const GroupF& G = sm.grp[S.group];
         const PrimF& Pr = sm.prm[e.y];
-        const float* P = sm.pose + ((size_t)c * nsl + G.slot) * kPoseF;
+        const float* P = sm.pose + c * pst + G.slot * kPoseF;
         const float3 sc = xf(P, S.x, S.y, S.z);
         const float ek = P[12] + P[13] * S.sn;
         const float m = margin32(4.0f + fabsf(sc.x) + fabsf(sc.y) + fabsf(sc.z)) + ek;
@@ -976,7 +990,7 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
       const int2 e = sm.hq[k];
       const int c = e.x >> 16, si = e.x & 0xffff;
       const SphereF S = sm.sph[si];
-      const float* P = sm.pose + ((size_t)c * nsl + sm.grp[S.group].slot) * kPoseF;
+      const float* P = sm.pose + c * pst + sm.grp[S.group].slot * kPoseF;
       return xf(P, S.x, S.y, S.z);
     };
     int k = pop();
@@ -1001,7 +1015,7 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
       const int done_c = __shfl_sync(FULL, (!want_dist && (sm.flags[c] & FLAG_FAIL)) ? 1 : 0, 0);
       if (!done_c) {
         const PrimF& Pr = sm.prm[e.y];
-        const float* P = sm.pose + ((size_t)c * nsl + G.slot) * kPoseF;
+        const float* P = sm.pose + c * pst + G.slot * kPoseF;
         const float3 sc = xf(P, S.x, S.y, S.z);
         const float ek = P[12] + P[13] * S.sn;
         const float m = margin32(4.0f + fabsf(sc.x) + fabsf(sc.y) + fabsf(sc.z)) + ek;
@@ -1045,20 +1059,21 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
     }
   __syncthreads();
   if (tid < ncfg && !(sm.flags[tid] & 2)) src.done(c0 + tid, (sm.flags[tid] & FLAG_FAIL) != 0);
+  if (tid < CPB) sm.flags[tid] = 0;
   __syncthreads();
 }
 
 // Shared-memory layout of a fast block; every array starts on a 16-byte boundary.  slot .. pairs are the
 // tables' FP32 image in its own order, fkl its tail.
 struct SmemLayout {
-  size_t pose, slot, base8, sph, grp, prm, pairs, flags, cull, qbuf, fkl, hq_n, hq, sdist, total;
+  size_t pose, slot, base8, sph, grp, prm, pairs, flags, cull, fkl, hq_n, hq, sdist, total;
 };
 __host__ __device__ inline size_t a16(size_t x) { return (x + 15) & ~(size_t)15; }
 __host__ __device__ inline SmemLayout smem_layout(const PmTablesHdr& h, int cpb, bool want_dist) {
   SmemLayout L;
   size_t o = 0;
   L.pose = o;
-  o = a16(o + sizeof(float) * kPoseF * (size_t)cpb * h.n_slots);
+  o = a16(o + sizeof(float) * (size_t)cpb * pose_stride(h.n_slots));
   L.slot = o;
   o = a16(o + sizeof(SlotF) * h.n_slots);
   L.base8 = o;
@@ -1075,8 +1090,6 @@ __host__ __device__ inline SmemLayout smem_layout(const PmTablesHdr& h, int cpb,
   o = a16(o + sizeof(int) * cpb);
   L.cull = o;
   o = a16(o + sizeof(unsigned) * (size_t)cpb * h.n_groups);
-  L.qbuf = o;
-  o = a16(o + sizeof(double) * (size_t)cpb * h.q_dim);
   L.fkl = o;
   o = a16(o + PM_IMG_TAIL);
   L.hq_n = o;
@@ -1101,7 +1114,6 @@ __device__ Smem carve(unsigned char* p, const PmTablesHdr* T, int cpb) {
   sm.pairs = reinterpret_cast<int2*>(p + L.pairs);
   sm.flags = reinterpret_cast<int*>(p + L.flags);
   sm.cull = reinterpret_cast<unsigned*>(p + L.cull);
-  sm.qbuf = reinterpret_cast<double*>(p + L.qbuf);
   sm.fkl = p + L.fkl;
   sm.fkn = reinterpret_cast<int*>(p + L.fkl + 3 * PM_MAX_SLOTS);
   sm.hq_n = reinterpret_cast<int*>(p + L.hq_n);
@@ -1155,10 +1167,11 @@ __global__ void __launch_bounds__(NT, 65536 / (NT * 64)) k_fast_valid(const PmTa
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TView v(T);
   Smem sm = carve(smem_raw, T, CPB);
+  if (threadIdx.x < CPB) sm.flags[threadIdx.x] = 0;
   stage_tables(v, sm, state);
   CfgSource src{q, B, out, scr.bnd};
   const int64_t c0 = (int64_t)blockIdx.x * CPB;
-  fast_block<CPB>(v, sm, state, src, c0, (int)(B - c0 < CPB ? B - c0 : CPB), dist32, cutoff, scr, sm.qbuf);
+  fast_block<CPB>(v, sm, state, src, c0, (int)(B - c0 < CPB ? B - c0 : CPB), dist32, cutoff, scr);
 }
 
 // Persistent work-queue kernel over the flattened waypoints of all edges.
@@ -1170,6 +1183,7 @@ __global__ void __launch_bounds__(NT, 65536 / (NT * 64)) k_fast_edges(const PmTa
   __shared__ long long chunk;
   TView v(T);
   Smem sm = carve(smem_raw, T, CPB);
+  if (threadIdx.x < CPB) sm.flags[threadIdx.x] = 0;
   stage_tables(v, sm, state);
   const int64_t W = src.E > 0 ? src.off[src.E - 1] + src.n[src.E - 1] : 0;
   for (;;) {
@@ -1177,7 +1191,7 @@ __global__ void __launch_bounds__(NT, 65536 / (NT * 64)) k_fast_edges(const PmTa
     __syncthreads();
     const int64_t c0 = chunk;
     if (c0 >= W) break;
-    fast_block<CPB>(v, sm, state, src, c0, (int)(W - c0 < CPB ? W - c0 : CPB), nullptr, 0.f, scr, sm.qbuf);
+    fast_block<CPB>(v, sm, state, src, c0, (int)(W - c0 < CPB ? W - c0 : CPB), nullptr, 0.f, scr);
   }
 }
 

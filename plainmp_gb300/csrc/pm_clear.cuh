@@ -10,9 +10,12 @@ constexpr float kU = 5.9604645e-8f;  // 2^-24
 // gives about 52 units for the box, the largest case.
 __device__ __forceinline__ float margin32(float mag) { return 1e-6f + 64.0f * kU * (1.0f + mag); }
 
-__device__ __forceinline__ float3 xf(const float* P, float x, float y, float z) {  // R (row-major 9) * v + t (P[9..11])
-  return make_float3(fmaf(P[0], x, fmaf(P[1], y, fmaf(P[2], z, P[9]))), fmaf(P[3], x, fmaf(P[4], y, fmaf(P[5], z, P[10]))),
-                     fmaf(P[6], x, fmaf(P[7], y, fmaf(P[8], z, P[11]))));
+// A pose in FP32: the rows (R_i0 R_i1 R_i2 t_i) as float4 (P on a 16-byte boundary).
+__device__ __forceinline__ float3 xf(const float* P, float x, float y, float z) {  // R v + t
+  const float4* p = reinterpret_cast<const float4*>(P);
+  const float4 a = p[0], b = p[1], c = p[2];
+  return make_float3(fmaf(a.x, x, fmaf(a.y, y, fmaf(a.z, z, a.w))), fmaf(b.x, x, fmaf(b.y, y, fmaf(b.z, z, b.w))),
+                     fmaf(c.x, x, fmaf(c.y, y, fmaf(c.z, z, c.w))));
 }
 
 // Clearance g (the reference reports a collision iff g <= 0, up to its own rounding), the

@@ -158,22 +158,24 @@ struct PmSlotF {  // FK slot: the local transform's constant part (joint origin,
   float lt[3];
   float lt1;      // |lt|_1 (prismatic: of the origin part), rounded up
 };
-struct PmSphereF {
+// (16-byte alignment: a record is read with 16-byte loads)
+struct alignas(16) PmSphereF {
   float x, y, z, r;
   int32_t group, tiny;  // tiny: the FP64 radius is below 1e-6 (the reference's special cases)
   float sn;             // |offset in the link frame|, rounded up (for the FK error bound)
+  int32_t pad;
 };
-struct PmGroupF {
+struct alignas(16) PmGroupF {
   float rel[3], radius;
   int32_t slot, begin, count, only_self;
   int32_t tiny;
   float gn;  // |group centre in the link frame|, rounded up
   int32_t pad[2];
 };
-struct PmPrimF {
+struct alignas(16) PmPrimF {
   int32_t kind, aa, za, cloud;
-  float lb[3], ub[3], pos[3], rot[9];
-  float a, b, c, mag;
+  float pos[3], mag;
+  float rot[9], a, b, c;
 };
 // The image: slots, fixed base pose (8 floats), spheres, groups, primitives, pairs, each on a 16-byte
 // boundary, and a tail with the two-thread FK's slot lists [3][PM_MAX_SLOTS] (bytes) and their lengths [3].

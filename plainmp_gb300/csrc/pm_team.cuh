@@ -15,7 +15,7 @@
 namespace pmd {
 
 constexpr int kRec = 8;    // doubles per slot: quaternion x y z w, translation, identity flag of the local transform
-constexpr int kRec32 = 12; // floats per slot: R (row-major), t
+constexpr int kRec32 = 12; // floats per slot: the rows of (R, t)
 
 // Poses of one configuration (kRec / kRec32 per slot).
 struct TeamPose {
@@ -53,7 +53,7 @@ struct Image {
 // the quaternion (2u) moves R s by at most (8 * 2u + 24u) |s|, that of t by u |t|_1 (the rounding of R s + t
 // itself is part of margin32).
 __device__ __forceinline__ float cast_error(const float* P, float sn) {
-  return kU * (64.0f * sn + 4.0f * (fabsf(P[9]) + fabsf(P[10]) + fabsf(P[11]))) + 1e-9f;
+  return kU * (64.0f * sn + 4.0f * (fabsf(P[3]) + fabsf(P[7]) + fabsf(P[11]))) + 1e-9f;
 }
 
 // FK of configurations 0 .. ncfg - 1 by NT threads (a block, or a warp of one: WARP) into rec
@@ -146,18 +146,10 @@ __device__ void fk64_block(const TView& v, const double* __restrict__ state, con
     float* f = p32 + (size_t)t * kRec32;
     const float x = (float)r[0], y = (float)r[1], z = (float)r[2], w = (float)r[3];
     const float tx = 2.f * x, ty = 2.f * y, tz = 2.f * z;
-    f[0] = 1.f - (ty * y + tz * z);
-    f[1] = ty * x - tz * w;
-    f[2] = tz * x + ty * w;
-    f[3] = ty * x + tz * w;
-    f[4] = 1.f - (tx * x + tz * z);
-    f[5] = tz * y - tx * w;
-    f[6] = tz * x - ty * w;
-    f[7] = tz * y + tx * w;
-    f[8] = 1.f - (tx * x + ty * y);
-    f[9] = (float)r[4];
-    f[10] = (float)r[5];
-    f[11] = (float)r[6];
+    float4* row = reinterpret_cast<float4*>(f);
+    row[0] = make_float4(1.f - (ty * y + tz * z), ty * x - tz * w, tz * x + ty * w, (float)r[4]);
+    row[1] = make_float4(ty * x + tz * w, 1.f - (tx * x + tz * z), tz * y - tx * w, (float)r[5]);
+    row[2] = make_float4(tz * x - ty * w, tz * y + tx * w, 1.f - (tx * x + ty * y), (float)r[6]);
   }
   __syncthreads();
 }
