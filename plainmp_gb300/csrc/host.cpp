@@ -1023,9 +1023,11 @@ struct HostCst {
                  "control records upload");
   }
 
-  // Launch shape and tuning of a fast call of B configurations where the caller set none.  (16, 256) and
-  // tiles of 8 spheres while every block is resident at once (4 of 256 threads per SM): the block's serial
-  // parts then weigh most.  Beyond that, robots of up to 64 spheres run (16, 128), twice as many blocks in
+  // Launch shape and tuning of a fast call of B configurations where the caller set none.  Tiles of 8 spheres.
+  // (8, 256) while every such block is resident at once (4 of 256 threads per SM: 4,864 configurations), where
+  // the latency of one block is the kernel's; (16, 256) while those are.  Calls with distances at (16, 256) and
+  // (8, 256), us: 1,001 states of the chain x 20 primitives 49 -> 42, of the dual arm x primitives 45 -> 31, of
+  // the dual arm x cloud 50 -> 42; 4,096: 49 -> 47, 62 -> 54, 65 -> 61.  Beyond that, robots of up to 64 spheres run (16, 128), twice as many blocks in
   // flight; larger ones stay at (16, 256).  Measured against (32, 256) with the least tile, us:
   // dual arm (120 spheres) x cloud, 65,536 with distances 622 -> 510, 200,003 validity 630 -> 469; chain
   // (56) x 20 primitives, 4,096 with distances 81 -> 64, 65,536 273 -> 218; 16,384 at (16, 256) 97, at
@@ -1038,7 +1040,7 @@ struct HostCst {
     if (!shape_set && fast_smem_bytes(hdr, fast_cpb, want_dist) <= 200 * 1024) {  // what does not fit at (32, 256) is refused as it was
       int n_sm = 0;
       cuda_check(sm_count(&n_sm), "device attribute");
-      *cpb = 16;
+      *cpb = B <= 8 * 4 * (int64_t)n_sm ? 8 : 16;
       *nt = (B + 15) / 16 > 4 * (int64_t)n_sm && hdr.n_spheres <= 64 ? 128 : 256;
     }
     return t;

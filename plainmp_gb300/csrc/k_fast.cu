@@ -714,7 +714,10 @@ struct EdgeSource {
 
 // Phases 1-3 for the configurations [c0, c0 + ncfg) of a source.  The block's flags are zero on entry and on
 // return.
-template <int CPB, class Src>
+// LONE: the block's own latency counts (all blocks are resident at once, primitives to cull against): the cull
+// splits a group's primitives over lanes and the task rows come from a counter.  A block among many leaves both
+// out (1 % slower with them).
+template <int CPB, bool LONE, class Src>
 __device__ void fast_block(const TView& v, const Smem& sm, const double* __restrict__ state, const Src& src, int64_t c0, int ncfg,
                            float* __restrict__ dist32, float cutoff, const Scratch& scr) {
   const PmTablesHdr* T = v.T;
@@ -742,8 +745,8 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
     }
     __syncthreads();
     const int fc = tid >> 1, fth = tid & 1;  // threads 2c and 2c + 1 (the same warp): the trunk, then a subtree set each
-    if (tid < 2 * CPB) {  // whole warps
-      const bool on = fc < ncfg && !(sm.flags[fc] & 2);
+    if (tid < (CPB < 16 ? 32 : 2 * CPB)) {  // whole warps
+      const bool on = fc < ncfg && !(sm.flags[min(fc, CPB - 1)] & 2);
       float* P = sm.pose + fc * pst;
       if (on && fth == 0) fk_chain(sm.slot, sm.fkn[0], sm.fkl, P);
       __syncwarp();
@@ -772,29 +775,54 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
     if (fail) atomicOr(&sm.flags[c], FLAG_FAIL);
     else if ((b.has_lb && x - m <= lo) || (b.has_ub && x + m >= hi)) push_item(scr, src, c0 + c, -1 - k, 0, 0);
   }
-  // ---- 2. group culling against each primitive
-  for (int t = tid; t < ncfg * ng; t += blockDim.x) {
-    const int c = t / ng, gi = t - c * ng;
-    if (sm.flags[c] & 2) continue;
-    const GroupF& G = sm.grp[gi];
-    const float* P = sm.pose + c * pst + G.slot * kPoseF;
-    float3 gc = xf(P, G.rel[0], G.rel[1], G.rel[2]);
-    const float ekg = P[12] + P[13] * G.gn;  // FK error bound of the group centre
-    unsigned mask = 0;
-    const int npc = np < 32 ? np : 32;
-    for (int p = 0; p < npc; p++) {
-      float g, sd, mag;
-      const PrimF& P = sm.prm[p];
-      if (P.kind == PM_SDF_CLOUD) {  // the nearest-point field bounds the cloud from below
-        const float lb = grid_field_lb16(v.C[P.cloud], gc.x, gc.y, gc.z);
-        g = lb - P.a - G.radius;
-        mag = fabsf(gc.x) + fabsf(gc.y) + fabsf(gc.z) + lb;
-      } else {
-        clearance(P, v.C, gc.x, gc.y, gc.z, G.radius, G.tiny, 0.f, g, sd, mag);
-      }
-      if (g > margin32(mag) + ekg + (want_dist ? cutoff : 0.f)) mask |= 1u << p;
+  // ---- 2. group culling against each primitive, a task per (configuration, group).  LONE: the primitives are
+  //         split over 2^sl lanes while that many threads are free: a block of 16 chain configurations has 112
+  //         tasks, and each walked 20 primitives with half of the block idle.
+  const unsigned FULL = 0xffffffffu;
+  const int lane = tid & 31;
+  const int npc = np < 32 ? np : 32;
+  auto cleared = [&](const GroupF& G, const float* P, const float3& gc, int p) {
+    const PrimF& Q = sm.prm[p];
+    float g, sd, mag;
+    if (Q.kind == PM_SDF_CLOUD) {  // the nearest-point field bounds the cloud from below
+      const float lb = grid_field_lb16(v.C[Q.cloud], gc.x, gc.y, gc.z);
+      g = lb - Q.a - G.radius;
+      mag = fabsf(gc.x) + fabsf(gc.y) + fabsf(gc.z) + lb;
+    } else {
+      clearance(Q, v.C, gc.x, gc.y, gc.z, G.radius, G.tiny, 0.f, g, sd, mag);
     }
-    sm.cull[c * ng + gi] = mask;
+    // the FK error bound of the group centre is et + eb |centre|
+    return g > margin32(mag) + (P[12] + P[13] * G.gn) + (want_dist ? cutoff : 0.f);
+  };
+  if (LONE) {
+    int sl = 0;
+    while ((ncfg * ng << (sl + 1)) <= (int)blockDim.x && (2 << sl) <= min(npc, 8)) sl++;
+    const int n_cull = ncfg * ng << sl;
+    for (int t0 = tid & ~31; t0 < n_cull; t0 += blockDim.x) {  // warp-uniform
+      const int t = t0 + lane, cg = t >> sl;
+      const int c = cg / ng, gi = cg - c * ng;
+      const bool on = t < n_cull && !(sm.flags[min(c, CPB - 1)] & 2);
+      unsigned mask = 0;
+      if (on) {
+        const GroupF& G = sm.grp[gi];
+        const float* P = sm.pose + c * pst + G.slot * kPoseF;
+        const float3 gc = xf(P, G.rel[0], G.rel[1], G.rel[2]);
+        for (int p = t & ((1 << sl) - 1); p < npc; p += 1 << sl) mask |= cleared(G, P, gc, p) ? 1u << p : 0u;
+      }
+      for (int o = 1; o < 1 << sl; o <<= 1) mask |= __shfl_xor_sync(FULL, mask, o);
+      if (on) sm.cull[c * ng + gi] = mask;
+    }
+  } else {
+    for (int t = tid; t < ncfg * ng; t += blockDim.x) {
+      const int c = t / ng, gi = t - c * ng;
+      if (sm.flags[c] & 2) continue;
+      const GroupF& G = sm.grp[gi];
+      const float* P = sm.pose + c * pst + G.slot * kPoseF;
+      const float3 gc = xf(P, G.rel[0], G.rel[1], G.rel[2]);
+      unsigned mask = 0;
+      for (int p = 0; p < npc; p++) mask |= cleared(G, P, gc, p) ? 1u << p : 0u;
+      sm.cull[c * ng + gi] = mask;
+    }
   }
   __syncthreads();
   // ---- 3a. sphere tasks (primitives in-thread; cloud queries near the cloud are queued) and
@@ -802,6 +830,7 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
   if (tid == 0) {
     sm.hq_n[0] = 0;
     sm.hq_n[1] = 0;
+    sm.hq_n[3] = blockDim.x;  // the first row past the warps' first
   }
   __syncthreads();
   const int hq_cap = T->n_clouds > 0 ? CPB * ns : 0;
@@ -810,7 +839,7 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
   // tile puts the same sphere on neighbouring lanes (shared records); a large one keeps a
   // configuration's neighbouring spheres, and so their field cells, on one warp.  Pair tasks
   // follow, numbered with the configuration fastest.  CPB is a power of two: no division.
-  constexpr int cpb_l = CPB == 16 ? 4 : (CPB == 32 ? 5 : (CPB == 64 ? 6 : 7));
+  constexpr int cpb_l = CPB == 8 ? 3 : CPB == 16 ? 4 : (CPB == 32 ? 5 : (CPB == 64 ? 6 : 7));
   const int stl = max(min(scr.st_log2, 5), cpb_l >= 5 ? 0 : 5 - cpb_l);
   const int rl = 5 - stl, ncb_l = cpb_l - rl;  // configurations per row, rows per sphere tile (log2)
   const int n_sph_tasks = (((ns + (1 << stl) - 1) >> stl) << ncb_l) << 5;
@@ -881,9 +910,10 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
   // Self pairs: each lane tests its (configuration, group pair) by the group spheres; the warp then
   // takes the surviving pairs one at a time, 32 sphere pairs per step (rows of 8 x 4), so a rare
   // survivor does not hold 31 idle lanes for its whole sphere-pair loop.
-  const unsigned FULL = 0xffffffffu;
-  const int lane = tid & 31;
-  for (int t0 = tid & ~31; t0 < n_tasks; t0 += blockDim.x) {  // warp-uniform
+  // Rows of 32 tasks differ by an order of magnitude (cleared groups against several near primitives, pairs
+  // with survivors).  LONE: the warps take rows from a counter, so that none waits long for the others; else
+  // the SM's other blocks fill the wait, and the fixed share is cheaper.
+  for (int t0 = tid & ~31; t0 < n_tasks;) {  // warp-uniform
     const int t = t0 + lane;
     int hit_pi = -1, hit_c = 0;
     if (t < n_sph_tasks) {
@@ -942,6 +972,13 @@ __device__ void fast_block(const TView& v, const Smem& sm, const double* __restr
         if (__any_sync(FULL, fail)) break;
       }
       if (fail) atomicOr(&sm.flags[c], FLAG_FAIL);
+    }
+    if (LONE) {
+      int next = 0;
+      if (lane == 0) next = atomicAdd(&sm.hq_n[3], 32);
+      t0 = __shfl_sync(FULL, next, 0);
+    } else {
+      t0 += blockDim.x;
     }
   }
   __syncthreads();
@@ -1161,7 +1198,7 @@ __device__ void stage_tables(const TView& v, const Smem& sm, const double* __res
 // 64 registers a thread, stated as the occupancy target (NT threads x 65536 / (NT x 64) blocks
 // per SM): the same budget the compiler picks for NT alone, but its allocation under the explicit
 // target measured 4-8 % faster in both modes.
-template <int CPB, int NT>
+template <int CPB, int NT, bool LONE = false>
 __global__ void __launch_bounds__(NT, 65536 / (NT * 64)) k_fast_valid(const PmTablesHdr* __restrict__ T, const double* __restrict__ state, const double* __restrict__ q, int64_t B,
                                                     uint8_t* __restrict__ out, float* __restrict__ dist32, float cutoff, Scratch scr) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1171,7 +1208,7 @@ __global__ void __launch_bounds__(NT, 65536 / (NT * 64)) k_fast_valid(const PmTa
   stage_tables(v, sm, state);
   CfgSource src{q, B, out, scr.bnd};
   const int64_t c0 = (int64_t)blockIdx.x * CPB;
-  fast_block<CPB>(v, sm, state, src, c0, (int)(B - c0 < CPB ? B - c0 : CPB), dist32, cutoff, scr);
+  fast_block<CPB, LONE>(v, sm, state, src, c0, (int)(B - c0 < CPB ? B - c0 : CPB), dist32, cutoff, scr);
 }
 
 // Persistent work-queue kernel over the flattened waypoints of all edges.
@@ -1191,7 +1228,7 @@ __global__ void __launch_bounds__(NT, 65536 / (NT * 64)) k_fast_edges(const PmTa
     __syncthreads();
     const int64_t c0 = chunk;
     if (c0 >= W) break;
-    fast_block<CPB>(v, sm, state, src, c0, (int)(W - c0 < CPB ? W - c0 : CPB), nullptr, 0.f, scr);
+    fast_block<CPB, false>(v, sm, state, src, c0, (int)(W - c0 < CPB ? W - c0 : CPB), nullptr, 0.f, scr);
   }
 }
 
@@ -1573,6 +1610,12 @@ cudaError_t launch_fast_valid(const PmTablesHdr* T, const PmTablesHdr& h, const 
   if (sm > 200 * 1024) return cudaErrorInvalidConfiguration;
   unsigned grid = (unsigned)((B + cpb - 1) / cpb);
   cudaError_t e;
+  int n_sm = 0;
+  if ((e = sm_count(&n_sm)) != cudaSuccess) return e;
+  // 8 primitives or more and at most 4 blocks of 256 per SM: the latency of one block is the kernel's.  4,096
+  // chain states against 20 primitives with distances: 34.4 us without LONE, 25.4 with; 200,003 dual-arm states
+  // against the cloud: 407 us without, 411 with; against a cloud alone LONE gains nothing at (16, 256).
+  const bool lone = h.n_prims >= 8 && (int64_t)grid * nt <= 1024 * (int64_t)n_sm;
   prof_begin("k_fast_valid", s);
 #define PM_FAST_CASE(C, N)                                                                      \
   if (cpb == C && nt == N) {                                                                     \
@@ -1581,9 +1624,19 @@ cudaError_t launch_fast_valid(const PmTablesHdr* T, const PmTablesHdr& h, const 
     launched = true;                                                                             \
   }
   bool launched = false;
+  if (cpb == 8 && nt == 256) {
+    if ((e = prep(k_fast_valid<8, 256, true>, sm)) != cudaSuccess) return e;
+    k_fast_valid<8, 256, true><<<grid, 256, sm, s>>>(T, state, q, B, out, dist32, cutoff, scr);
+    launched = true;
+  }
+  if (lone && cpb == 16 && nt == 256) {
+    if ((e = prep(k_fast_valid<16, 256, true>, sm)) != cudaSuccess) return e;
+    k_fast_valid<16, 256, true><<<grid, 256, sm, s>>>(T, state, q, B, out, dist32, cutoff, scr);
+    launched = true;
+  } else
+  PM_FAST_CASE(16, 256)
   PM_FAST_CASE(16, 128)
   PM_FAST_CASE(32, 128)
-  PM_FAST_CASE(16, 256)
   PM_FAST_CASE(32, 256)
   PM_FAST_CASE(64, 256)
   PM_FAST_CASE(32, 512)
@@ -1594,8 +1647,6 @@ cudaError_t launch_fast_valid(const PmTablesHdr* T, const PmTablesHdr& h, const 
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   prof_end("k_fast_valid", s);
   CfgSource src{q, B, out, bnd};
-  int n_sm = 0;
-  if ((e = sm_count(&n_sm)) != cudaSuccess) return e;
   if (split) {
     prof_begin("k_hard_queries", s);
     const int bps = tune.hq_blocks_per_sm >= 1 && tune.hq_blocks_per_sm <= 8 ? tune.hq_blocks_per_sm : 4;
