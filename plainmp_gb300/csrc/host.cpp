@@ -175,6 +175,8 @@ static size_t up16(size_t x) { return (x + 15) & ~(size_t)15; }
 // that the kernel itself reads and writes: no copies on the stream.  A call of one state took 66 us with them,
 // 32 us without (update of the model state included).
 constexpr int64_t kZeroCopy = 64;
+// The same for validity-only calls of the fast path (with distances, the results are copied).
+constexpr int64_t kZeroCopyFast = 2048;
 
 // ---------------------------------------------------------------------------- host quaternion
 // construction-time helpers (setQuaternionFromRPY, transform.hpp:122-130)
@@ -683,7 +685,7 @@ struct HostCst {
   DevBuf d_ctrl_recs;
   // workspaces for host-memory calls
   DevBuf w_in, w_in2, w_out, w_out2, w_aux, w_seq, w_width;
-  DevBuf f_items, f_ctl, f_overflow;  // fast-path recheck queue, counters, per-config overflow flags
+  DevBuf f_items, f_ctl;  // fast-path recheck queue; counters and per-config (or per-edge) overflow flags
   DevBuf f_hq;                        // fast-path hard cloud queries (distances mode)
   PinBuf h_pin;                       // pinned staging of small host-memory calls
   DevBuf w_cen;                       // sphere centres of a device-memory distances call without centres
@@ -2110,12 +2112,11 @@ static int fast_valid_entry(pmgpu_cst* c, const double* q, int64_t B, uint8_t* o
     }
     const unsigned cap = (unsigned)std::min<int64_t>(std::max<int64_t>(4 * B, 1 << 16), (int64_t)1 << 28);
     int4* items = (int4*)C.f_items.ensure((size_t)cap * sizeof(int4));
-    char* ctl = (char*)C.f_ctl.ensure(64);
+    char* ctl = (char*)C.f_ctl.ensure(64 + (size_t)B);  // counters, then the overflow flags
     unsigned int* count = (unsigned int*)ctl;
     unsigned long long* dstats = (unsigned long long*)(ctl + 16);
-    uint8_t* ovf = (uint8_t*)C.f_overflow.ensure(std::max<size_t>((size_t)B, 16));
-    cuda_check(cudaMemsetAsync(ctl, 0, 64, s), "memset");
-    cuda_check(cudaMemsetAsync(ovf, 0, std::max<size_t>((size_t)B, 16), s), "memset");
+    uint8_t* ovf = (uint8_t*)ctl + 64;
+    cuda_check(cudaMemsetAsync(ctl, 0, 64 + (size_t)B, s), "memset");
     const double* dq = q;
     uint8_t* dout = out;
     float* dd = dist32;
@@ -2125,6 +2126,12 @@ static int fast_valid_entry(pmgpu_cst* c, const double* q, int64_t B, uint8_t* o
     if (mem == PMGPU_MEM_HOST) {
       pin = C.h_pin.ensure(up16(nq) + up16((size_t)B) + up16(nd) + 64);
       std::memcpy(pin, q, nq);
+    }
+    const bool zero_copy = mem == PMGPU_MEM_HOST && !dist32 && B <= kZeroCopyFast;
+    if (zero_copy) {
+      dq = (const double*)pin;
+      dout = (uint8_t*)pin + up16(nq);
+    } else if (mem == PMGPU_MEM_HOST) {
       double* dqw = (double*)C.w_in.ensure(std::max<size_t>(nq, 16));
       if (nq) cuda_check(cudaMemcpyAsync(dqw, pin, nq, cudaMemcpyHostToDevice, s), "H2D copy");
       dq = dqw;
@@ -2143,11 +2150,11 @@ static int fast_valid_entry(pmgpu_cst* c, const double* q, int64_t B, uint8_t* o
     unsigned long long local_ctl[6] = {0, 0, 0, 0, 0, 0};
     unsigned long long* h = pin ? reinterpret_cast<unsigned long long*>(pin_dist + up16(nd)) : local_ctl;
     if (mem == PMGPU_MEM_HOST) {
-      if (B) cuda_check(cudaMemcpyAsync(pin_out, dout, (size_t)B, cudaMemcpyDeviceToHost, s), "D2H copy");
+      if (B && !zero_copy) cuda_check(cudaMemcpyAsync(pin_out, dout, (size_t)B, cudaMemcpyDeviceToHost, s), "D2H copy");
       if (nd) cuda_check(cudaMemcpyAsync(pin_dist, dd, nd, cudaMemcpyDeviceToHost, s), "D2H copy");
     }
     if (stats || mem == PMGPU_MEM_HOST) {
-      cuda_check(cudaMemcpyAsync(h, ctl, 48, cudaMemcpyDeviceToHost, s), "D2H");
+      if (stats) cuda_check(cudaMemcpyAsync(h, ctl, 48, cudaMemcpyDeviceToHost, s), "D2H");
       cuda_check(cudaStreamSynchronize(s), "is_valid_fast");
       if (mem == PMGPU_MEM_HOST) {
         std::memcpy(out, pin_out, (size_t)B);
@@ -2266,11 +2273,8 @@ static int fast_edges_entry(pmgpu_cst* c, const double* s1, const double* s2, in
     }
     const double* dw = nullptr;
     if (box) {
-      dw = (const double*)C.w_width.ensure((size_t)d * 8 + 16);
-      if (mem == PMGPU_MEM_DEVICE)
-        cuda_check(cudaMemcpyAsync((void*)dw, width, nw, cudaMemcpyDeviceToDevice, s), "width");
-      else
-        cuda_check(cudaMemcpyAsync((void*)dw, pin + 2 * up16(ns_), nw, cudaMemcpyHostToDevice, s), "width");
+      // read in place by the setup kernel: the caller's device array, or page-locked staging
+      dw = mem == PMGPU_MEM_DEVICE ? width : (const double*)(pin + 2 * up16(ns_));
     }
     const size_t En = (size_t)std::max<int64_t>(E, 1);
     double* sr = (double*)C.e_sr.ensure(En * 8);
@@ -2278,13 +2282,12 @@ static int fast_edges_entry(pmgpu_cst* c, const double* s1, const double* s2, in
     int64_t* off = (int64_t*)C.e_off.ensure(En * 8);
     const unsigned cap = 1u << 18;
     int4* items = (int4*)C.f_items.ensure((size_t)cap * sizeof(int4));
-    char* ctl = (char*)C.f_ctl.ensure(64);
+    char* ctl = (char*)C.f_ctl.ensure(64 + En);  // counters, then the overflow flags
     unsigned int* count = (unsigned int*)ctl;
     unsigned long long* next = (unsigned long long*)(ctl + 8);
     unsigned long long* dstats = (unsigned long long*)(ctl + 16);
-    uint8_t* ovf = (uint8_t*)C.f_overflow.ensure(std::max<size_t>(En, 16));
-    cuda_check(cudaMemsetAsync(ctl, 0, 64, s), "memset");
-    cuda_check(cudaMemsetAsync(ovf, 0, std::max<size_t>(En, 16), s), "memset");
+    uint8_t* ovf = (uint8_t*)ctl + 64;
+    cuda_check(cudaMemsetAsync(ctl, 0, 64 + En, s), "memset");
     const double* d1 = s1;
     const double* d2 = s2;
     uint8_t* dout = out;

@@ -56,7 +56,7 @@ __device__ __forceinline__ float cast_error(const float* P, float sn) {
   return kU * (64.0f * sn + 4.0f * (fabsf(P[3]) + fabsf(P[7]) + fabsf(P[11]))) + 1e-9f;
 }
 
-// FK of configurations 0 .. ncfg - 1 by NT threads (a block, or a warp of one: WARP) into rec
+// FK of configurations 0 .. ncfg - 1 by NT threads (a block, or the one warp of a block: WARP) into rec
 // [ncfg][n_slots][kRec]; qf(c, col) gives a joint or base value.  The pose of a slot replaces its local
 // transform in place.  Poses are bit for bit those of fk64.
 template <int NT, bool WARP, class QF>
@@ -101,7 +101,9 @@ __device__ void fk64_levels(const TView& v, const double* __restrict__ state, co
     r[6] = p.t.z;
     r[7] = lid ? 1.0 : 0.0;
   }
-  const int32_t* lev = pm_at<int32_t>(T, T->off_lev);
+  // the levels (starts, then slot | parent << 16) in shared memory: two dependent loads a level otherwise
+  __shared__ int32_t lev[2 * PM_MAX_SLOTS + 1];
+  for (int i = tid; i < T->n_levels + 1 + nsl; i += NT) lev[i] = pm_at<int32_t>(T, T->off_lev)[i];
   const int32_t* order = lev + T->n_levels + 1;
   const int quad = tid >> 2, k = tid & 3, w0 = (tid >> 5) << 3;  // the lane's quad and component, the warp's first quad
   const int i1 = k == 0 ? 1 : (k == 1 ? 2 : 0), i2 = k == 0 ? 2 : (k == 1 ? 0 : 1);  // the cyclic next two of x y z
