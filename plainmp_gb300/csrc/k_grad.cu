@@ -140,16 +140,23 @@ __device__ void stage(const PmTablesHdr* T, const double* state, const Layout& L
     }
     sl[i] = g;
   }
-  if (threadIdx.x == 0) {  // spheres ordered by slot (stable): counting sort
-    for (int i = 0; i <= L.n_slots; i++) sb[i] = 0;
-    for (int k = 0; k < L.n_sph; k++) sb[G[sg[k]].slot + 1]++;
-    for (int i = 0; i < L.n_slots; i++) sb[i + 1] += sb[i];
+  // spheres ordered by slot (stable): counting sort, from the slots in the units' work area (free until the
+  // first unit; at least 6 floats per sphere).  Read from the tables instead, thread 0's counts chained two
+  // loads a sphere and held every other thread at the barrier.
+  int* slot_of = (int*)(smem + L.off_warp);
+  for (int k = threadIdx.x; k < L.n_sph; k += blockDim.x) slot_of[k] = G[sg[k]].slot;
+  for (int i = threadIdx.x; i <= L.n_slots; i += blockDim.x) sb[i] = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < L.n_slots; i += blockDim.x) {
+    int n = 0;  // spheres of slots up to i
+    for (int k = 0; k < L.n_sph; k++) n += slot_of[k] <= i;
+    sb[i + 1] = n;
   }
   __syncthreads();
   for (int k = threadIdx.x; k < L.n_sph; k += blockDim.x) {
-    const int slot = G[sg[k]].slot;
+    const int slot = slot_of[k];
     int pos = sb[slot];
-    for (int j = 0; j < k; j++) pos += G[sg[j]].slot == slot;
+    for (int j = 0; j < k; j++) pos += slot_of[j] == slot;
     sp[pos] = GSph{(float)sx[k], (float)sy[k], (float)sz[k], (float)sr[k], slot, !G[sg[k]].only_self};
   }
   for (int i = threadIdx.x; i < L.n_prims; i += blockDim.x) {
