@@ -223,12 +223,14 @@ __global__ void k_update_state(double* state, const PmSlot* recs, const double* 
   update_state_block(state, recs, q, n, accurate, base_type);
 }
 
-// NC configurations per block, WPC warps each; 128 registers a thread.
+// NC configurations per block, WPC warps each.  Batches run 4 configurations of a warp each at 64 registers:
+// 1,500, 4,096 and 16,384 chain states take 40, 62 and 191 us, with 8 at 128 registers 48, 70 and 207, with 4
+// at 128 registers 38, 69 and 208, with 2 at 64 registers 40, 77 and 232.  One configuration takes 4 warps at 128.
 // UPDATE (one configuration): a second block leaves the model in its state, as is_valid of the reference does.
 // The rows it writes (control joints' links, the base row unless the base is fixed) are not among those that
 // the check reads (links without a control joint, a fixed base).
 template <int NC, int WPC, bool UPDATE = false>
-__global__ void __launch_bounds__(NC * WPC * 32, 512 / (NC * WPC * 32))
+__global__ void __launch_bounds__(NC * WPC * 32, (NC > 1 ? 1024 : 512) / (NC * WPC * 32))
     k_is_valid64(const PmTablesHdr* __restrict__ T, double* state, const double* __restrict__ q, int64_t B, uint8_t* __restrict__ out,
                  const PmSlot* __restrict__ recs, int accurate) {
   extern __shared__ __align__(16) double team_mem[];
@@ -825,7 +827,7 @@ cudaError_t launch_is_valid64(const PmTablesHdr* T, const PmTablesHdr& h, const 
   if (B <= 4 * (int64_t)n_sm)
     e = team_launch(k_is_valid64<1, 4>, B, 1, 4, h, s, T, st, q, B, out, (const PmSlot*)nullptr, 0);
   else
-    e = team_launch(k_is_valid64<8, 1>, (B + 7) / 8, 8, 1, h, s, T, st, q, B, out, (const PmSlot*)nullptr, 0);
+    e = team_launch(k_is_valid64<4, 1>, (B + 3) / 4, 4, 1, h, s, T, st, q, B, out, (const PmSlot*)nullptr, 0);
   prof_end("k_is_valid64", s);
   return e;
 }

@@ -9,8 +9,7 @@ from plainmp_gb300 import workloads as W
 
 pytestmark = pytest.mark.gpu
 
-# (configurations per block, and the batch up to which a configuration gets a block of its own): 8 and
-# 4 x 152 SMs for validity, 4 and 4 x 152 for values
+# 4 configurations per block, up to 4 x 152 SMs one
 SIZES = [1, 3, 4, 5, 7, 8, 9, 607, 608, 609, 613]
 
 
