@@ -7,7 +7,7 @@ HBM): the 14-DOF dual arm (two 7-joint chains, 120 spheres, cross-arm self pairs
 identical to the reference plus the FP32 nearest-point signed distance of every sphere
 (clamped at the reference's 0.1 m cutoff).  metric = configurations checked per second.
 
-Reported beside it: the plain FP64 method (one thread per configuration, launch per batch)
+Reported beside it: the plain FP64 method (a warp per configuration, launch per batch)
 on the same batch, the validity-only fast path, the end-to-end rate through the public API
 with pinned host buffers (copies inside the timed region), the CPU restatement of the
 reference on all host cores, kernel timing and the dominant kernel's roofline, and the SM
@@ -1036,7 +1036,7 @@ def main():
                                                 "bytes_from": "ncu lts__t_sectors.sum x 32 B of one launch of each kernel"}},
         "clocks": clocks,
         "plain_fp64": {"value": B / (ms_plain / 1e3), "unit": "configs/s", "ms_per_batch": ms_plain,
-                       "what": "plain FP64 method, one thread per configuration, validity only"},
+                       "what": "plain FP64 method, a warp per configuration, validity only"},
         "fast_validity_only": {"value": B / (ms_valid / 1e3), "unit": "configs/s", "ms_per_batch": ms_valid,
                                "ms_per_batch_eager_call": ms_valid_eager,
                                "kernel_ms": {"k_fast_valid": kv_ms / max(kv_n, 1), "k_fast_recheck": kvr_ms / max(kvr_n, 1)},
