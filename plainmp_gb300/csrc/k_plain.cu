@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(NC * WPC * 32, (NC > 1 ? 1024 : 512) / (NC * W
   if (threadIdx.x < NC) failed[threadIdx.x] = 0;
   float* p32 = reinterpret_cast<float*>(team_mem + (size_t)NC * nsl * kRec);
   fk64_block<NC * WPC * 32>(v, state, [&](int c, int col) { return q[(c0 + c) * qd + col]; }, ncfg, T->base_type == PM_BASE_FIXED,
-                            team_mem, p32);
+                            kNorm2Valid, team_mem, p32);
   const int c = (threadIdx.x >> 5) / WPC, wi = (threadIdx.x >> 5) % WPC;
   if (c < ncfg) valid_team<WPC>(v, im, TeamPose{team_mem + (size_t)c * nsl * kRec, p32 + (size_t)c * nsl * kRec32}, wi, failed + c);
   __syncthreads();
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(NC * 32, 512 / (NC * 32)) k_check_motion64(con
       const double t = n + 1 < 129 ? (double)seq[n * 128 + (k + 1)] * sr : (double)k * sr;
       return a[col] + (b[col] - a[col]) * t;
     };
-    fk64_block<NC * 32>(v, state, qf, ncfg, T->base_type == PM_BASE_FIXED, team_mem, p32);
+    fk64_block<NC * 32>(v, state, qf, ncfg, T->base_type == PM_BASE_FIXED, kNorm2Valid, team_mem, p32);
     const int c = threadIdx.x >> 5;
     if (c < ncfg) valid_team<1>(v, im, TeamPose{team_mem + (size_t)c * nsl * kRec, p32 + (size_t)c * nsl * kRec32}, 0, failed + c);
     __syncthreads();
@@ -435,7 +435,7 @@ __device__ double eval_ext_warp(const TView& v, const Image& im, const TeamPose&
           // beyond the bound none of them is the least.  The ground's gate tests more than the distance
           // (g), and only the cutoff counts for it.  (g of a box or cylinder ends at -radius inside it.)
           const bool by_gate = Q.kind == PM_SDF_GROUND;
-          if (!((by_gate ? g : sd) > (by_gate ? (float)PM_CUTOFF : upper) + margin32(mag) + cast_error(R, G.gn))) n = G.count;
+          if (!((by_gate ? g : sd) > (by_gate ? (float)PM_CUTOFF : upper) + margin32(mag) + cast_error(R, G.gn) + kStretch * G.radius)) n = G.count;
         }
       }
       warp_spread(n, [&](int owner, int j, bool have) {
@@ -449,7 +449,7 @@ __device__ double eval_ext_warp(const TView& v, const Image& im, const TeamPose&
           const PmSphereF& S = im.sph[k];
           const float* R = P.at32(G.slot);
           const float3 c = xf(R, S.x, S.y, S.z);
-          const float ek = cast_error(R, S.sn);
+          const float ek = cast_error(R, S.sn) + kStretch * im.grp[g2].radius;
           if (Q.kind == PM_SDF_CLOUD) {
             const PmGridDev& Gd = v.C[Q.cloud];
             const float qmag = fabsf(c.x) + fabsf(c.y) + fabsf(c.z);
@@ -489,6 +489,7 @@ __device__ double eval_ext_warp(const TView& v, const Image& im, const TeamPose&
           const PmPrim& Qs = v.P[ps];
           const D3 cs = shfl_d3(c, src), gcs = shfl_d3(gc, src);
           const double rs = shfl_d(r, src), rg = shfl_d(G.radius, src);
+          const bool scales = isnan(P.at32(v.G[__shfl_sync(FULL, g2, src)].slot)[3]);  // the group sphere may not hold its spheres
           const unsigned long long os = __shfl_sync(FULL, order, src);
           // only a value up to the smallest so far matters: search slightly beyond its reach
           const double reach = ((double)upper + Qs.a + rs) * (1.0 + 1e-6) + 1e-6;
@@ -497,7 +498,7 @@ __device__ double eval_ext_warp(const TView& v, const Image& im, const TeamPose&
           if (nn.idx < 0) continue;
           const double val = sqrt(nn.d2) - Qs.a - rs;
           // below the cutoff the gate is open, but for rounding at the cutoff itself
-          if (val > PM_CUTOFF - 1e-7 && cloud_outside_warp(Qs, v.C, gcs, rg + PM_CUTOFF, nullptr)) continue;
+          if ((scales || val > PM_CUTOFF - 1e-7 - kStretch * rg) && cloud_outside_warp(Qs, v.C, gcs, rg + PM_CUTOFF, nullptr)) continue;
           if (val < PM_CUTOFF) best.take(val, os);  // the same on every lane
           upper = fminf(upper, (float)val + 1e-6f * (1.0f + fabsf((float)val)));
         }
@@ -560,7 +561,7 @@ __device__ double eval_self_warp(const TView& v, const Image& im, const TeamPose
         const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
         const float mag = fabsf(a.x) + fabsf(a.y) + fabsf(a.z) + fabsf(b.x) + fabsf(b.y) + fabsf(b.z);
         near = !(sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) - (G1.radius + G2.radius) >
-                 upper + 2.0f * margin32(mag) + cast_error(R1, G1.gn) + cast_error(R2, G2.gn));
+                 upper + 2.0f * margin32(mag) + cast_error(R1, G1.gn) + cast_error(R2, G2.gn) + kStretch * (G1.radius + G2.radius));
       }
       for (unsigned bal = __ballot_sync(FULL, near); bal != 0; bal &= bal - 1) {  // warp-uniform
         const int src = __ffs(bal) - 1;
@@ -575,7 +576,7 @@ __device__ double eval_self_warp(const TView& v, const Image& im, const TeamPose
           const float ex = ci.x - cj.x, ey = ci.y - cj.y, ez = ci.z - cj.z;
           const float mag = fabsf(ci.x) + fabsf(ci.y) + fabsf(ci.z) + fabsf(cj.x) + fabsf(cj.y) + fabsf(cj.z);
           const float d32 = sqrtf(fmaf(ex, ex, fmaf(ey, ey, ez * ez))) - (S1.r + S2.r);
-          const float m = 2.0f * margin32(mag) + cast_error(R1, S1.sn) + cast_error(R2, S2.sn);
+          const float m = 2.0f * margin32(mag) + cast_error(R1, S1.sn) + cast_error(R2, S2.sn) + kStretch * (im.grp[a].radius + im.grp[b].radius);
           if (pass == 0) {
             upper = fminf(upper, d32 + m);
             continue;
@@ -627,7 +628,7 @@ __global__ void __launch_bounds__(NC * 64, 512 / (NC * 64)) k_evaluate64(const P
   const int64_t c0 = (int64_t)blockIdx.x * NC;
   const int ncfg = (int)min((int64_t)NC, B - c0);
   float* p32 = reinterpret_cast<float*>(team_mem + (size_t)NC * nsl * kRec);
-  fk64_block<NC * 64>(v, state, [&](int c, int col) { return q[(c0 + c) * qd + col]; }, ncfg, !high_accuracy, team_mem, p32);
+  fk64_block<NC * 64>(v, state, [&](int c, int col) { return q[(c0 + c) * qd + col]; }, ncfg, !high_accuracy, kNorm2Eval, team_mem, p32);
   const int c = threadIdx.x >> 6;
   if (c >= ncfg) return;
   const TeamPose P{team_mem + (size_t)c * nsl * kRec, p32 + (size_t)c * nsl * kRec32};

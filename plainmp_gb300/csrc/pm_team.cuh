@@ -140,18 +140,29 @@ __device__ void fk64_levels(const TView& v, const double* __restrict__ state, co
 }
 
 // fk64_levels by a block of NT threads, and the poses in FP32 (p32 [ncfg][n_slots][kRec32]).
+// The FP32 bounds (cast_error, margin32) are those of rotations, and so is that a group's sphere holds its spheres.
+// A quaternion off unit norm (URDF axes and base poses are taken as they are given) scales: R stretches by up to
+// 1 + 2 (|q|^2 - 1), or shrinks where |q| < 1.  Where |q|^2 exceeds `norm2` the FP32 translation is NaN, so that every
+// FP32 comparison of the slot's spheres fails and FP64 decides.
+// Validity needs the bounds alone, which have 1 % to spare (the Taylor form is within 1e-5 of unit norm a joint);
+// evaluate also that the spheres leave the group's sphere by no more than kStretch of its radius.
+constexpr float kNorm2Valid = 1.01f;
+constexpr float kNorm2Eval = 1.000001f;
+constexpr float kStretch = 3e-6f;
 template <int NT, class QF>
-__device__ void fk64_block(const TView& v, const double* __restrict__ state, const QF& qf, int ncfg, bool taylor, double* rec, float* p32) {
+__device__ void fk64_block(const TView& v, const double* __restrict__ state, const QF& qf, int ncfg, bool taylor, float norm2, double* rec,
+                           float* p32) {
   fk64_levels<NT, false>(v, state, qf, ncfg, taylor, rec);
   for (int t = threadIdx.x; t < ncfg * v.T->n_slots; t += NT) {
     const double* r = rec + (size_t)t * kRec;
     float* f = p32 + (size_t)t * kRec32;
     const float x = (float)r[0], y = (float)r[1], z = (float)r[2], w = (float)r[3];
     const float tx = 2.f * x, ty = 2.f * y, tz = 2.f * z;
+    const bool scales = !(x * x + y * y + (z * z + w * w) <= norm2);
     float4* row = reinterpret_cast<float4*>(f);
-    row[0] = make_float4(1.f - (ty * y + tz * z), ty * x - tz * w, tz * x + ty * w, (float)r[4]);
-    row[1] = make_float4(ty * x + tz * w, 1.f - (tx * x + tz * z), tz * y - tx * w, (float)r[5]);
-    row[2] = make_float4(tz * x - ty * w, tz * y + tx * w, 1.f - (tx * x + ty * y), (float)r[6]);
+    row[0] = make_float4(1.f - (ty * y + tz * z), ty * x - tz * w, tz * x + ty * w, scales ? NAN : (float)r[4]);
+    row[1] = make_float4(ty * x + tz * w, 1.f - (tx * x + tz * z), tz * y - tx * w, scales ? NAN : (float)r[5]);
+    row[2] = make_float4(tz * x - ty * w, tz * y + tx * w, 1.f - (tx * x + ty * y), scales ? NAN : (float)r[6]);
   }
   __syncthreads();
 }
