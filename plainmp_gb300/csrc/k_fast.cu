@@ -1565,22 +1565,25 @@ cudaError_t upload_offsets() {
   return e;
 }
 
-// The offset table on the device and the kernel's dynamic shared-memory limit raised to sm bytes;
-// both once per device (the attribute again only for a larger size), so small calls pay for neither.
-template <class K>
-static cudaError_t prep(K kern, size_t sm) {
-  cudaError_t e = upload_offsets();
-  if (e != cudaSuccess) return e;
+cudaError_t raise_smem(const void* kern, size_t sm) {
   int dev = 0;
-  if ((e = current_device(&dev)) != cudaSuccess) return e;
+  cudaError_t e = current_device(&dev);
+  if (e != cudaSuccess) return e;
   static std::mutex mu;
   static std::map<std::pair<const void*, int>, size_t> raised;
   std::lock_guard<std::mutex> lk(mu);
-  size_t& have = raised[{reinterpret_cast<const void*>(kern), dev}];
+  size_t& have = raised[{kern, dev}];
   if (have >= sm) return cudaSuccess;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e == cudaSuccess) have = sm;
   return e;
+}
+
+// The offset table on the device, once, and raise_smem.
+template <class K>
+static cudaError_t prep(K kern, size_t sm) {
+  const cudaError_t e = upload_offsets();
+  return e != cudaSuccess ? e : raise_smem(reinterpret_cast<const void*>(kern), sm);
 }
 
 // Blocks of the recheck kernel: one warp per 8 configurations (or 2 edges), at most 16 per SM; its loops

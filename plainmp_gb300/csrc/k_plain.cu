@@ -794,11 +794,9 @@ inline unsigned grid_for(int64_t n, int bs) { return (unsigned)((n + bs - 1) / b
 // Launches a kernel of nc configurations per block, wpc warps each.
 template <class K, class... A>
 cudaError_t team_launch(K kern, int64_t blocks, int nc, int wpc, const PmTablesHdr& h, cudaStream_t s, A... args) {
-  const size_t sm = team_smem(h, nc);
-  if (sm > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-  }
+  const size_t sm = team_smem(h, nc);  // with the static part it may pass 48 KB long before it does alone
+  const cudaError_t e = pmg::raise_smem(reinterpret_cast<const void*>(kern), sm);
+  if (e != cudaSuccess) return e;
   kern<<<(unsigned)blocks, nc * wpc * 32, sm, s>>>(args...);
   return cudaGetLastError();
 }

@@ -48,6 +48,9 @@ bool fast_table_sizes_ok(const PmTablesHdr& h);
 // uploaded to the current device once.
 cudaError_t sm_count(int* n);
 cudaError_t upload_offsets();
+// The kernel's limit of dynamic shared memory on the current device, raised to sm bytes where it is below.  It is
+// never lowered: another thread may be about to launch with more.
+cudaError_t raise_smem(const void* kern, size_t sm);
 // Tuning of the fast kernels beyond the launch shape (the autotuner's other dimensions).
 struct FastTuning {
   int sphere_tile_log2 = -1;  // log2 of the spheres per warp row of sphere tasks (at least 32 / configurations per
