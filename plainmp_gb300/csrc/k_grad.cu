@@ -995,13 +995,7 @@ int grid_for(const void* fn, size_t smem, int64_t units, int per_block = kNW) {
 }
 
 template <class K>
-cudaError_t prep(K fn, size_t smem) {
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
-}
+cudaError_t prep(K fn, size_t smem) { return pmg::raise_smem(reinterpret_cast<const void*>(fn), smem); }
 
 }  // namespace
 

@@ -85,3 +85,32 @@ def two_threads():
 
 def test_threads_with_tables_of_different_sizes():
     _child("two_threads()")
+
+
+def two_threads_of_costs():
+    """The same with the differentiable costs."""
+    import torch
+
+    from plainmp_gb300 import diff
+
+    made = [chain(n)[1] for n in (60, 40, 50)]
+    q = torch.tensor(np.zeros((4, 7), np.float32), device="cuda")
+    errors = []
+
+    def work(cst):
+        try:
+            for _ in range(1500):
+                diff.ik_cost_grad(cst, q, None, None)
+        except Exception as e:
+            errors.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(c,)) for c in made]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not errors, errors
+
+
+def test_threads_of_costs_with_tables_of_different_sizes():
+    _child("two_threads_of_costs()")
