@@ -3,9 +3,9 @@
 The forward value and the gradient come from the library's FP32 kernels (include/pmgpu.h,
 "differentiable costs"); the gradient is a hand-written reverse-mode adjoint through the FK
 chain and the SDF, not autograd.  ``IKCost`` and ``TrajectoryCost`` wrap them as
-``torch.autograd.Function``s: where q needs a gradient, the forward pass runs the cost and its adjoint
-in one launch and keeps the gradient (one row per configuration, the size of q; no transforms), and the
-backward pass scales it.  Otherwise the forward pass evaluates the cost only.
+``torch.autograd.Function``s: where q needs a gradient and gradients are recorded, the forward pass
+runs the cost and its adjoint in one launch and keeps the gradient (one row per configuration, the size
+of q; no transforms), and the backward pass scales it.  Otherwise the forward pass evaluates the cost only.
 
 Terms (all FP32):
     d_s       min over primitives of SDF.evaluate(c_s) - r_s (the SphereCollisionCst ext-row
@@ -167,7 +167,10 @@ def _torch():
 
 
 class IKCost:
-    """torch.autograd.Function: cost (B,) of q (B, q_dim) against targets (B, 7)."""
+    """torch.autograd.Function: cost (B,) of q (B, q_dim) against targets (B, 7).
+
+    ``recorded``: whether gradients are recorded, read before the Function is entered (inside they never are, and
+    needs_input_grad says only whether q asks for one: true for a leaf under no_grad too)."""
 
     _fn = None
 
@@ -178,8 +181,8 @@ class IKCost:
 
             class _F(torch.autograd.Function):
                 @staticmethod
-                def forward(ctx, q, target, cst, pose_link, weights):
-                    if not ctx.needs_input_grad[0]:
+                def forward(ctx, q, target, cst, pose_link, weights, recorded):
+                    if not (recorded and ctx.needs_input_grad[0]):
                         return ik_cost_grad(cst, q, target, pose_link, want_grad=False, **weights)
                     cost, grad = ik_cost_grad(cst, q, target, pose_link, want_grad=True, **weights)
                     ctx.save_for_backward(q, target, grad)  # q and target: a change in place is an error
@@ -188,12 +191,12 @@ class IKCost:
                 @staticmethod
                 def backward(ctx, g):
                     if not ctx.needs_input_grad[0]:
-                        return None, None, None, None, None
+                        return None, None, None, None, None, None
                     q, _, grad = ctx.saved_tensors
-                    return (g[:, None] * grad).to(q.dtype), None, None, None, None
+                    return (g[:, None] * grad).to(q.dtype), None, None, None, None, None
 
             cls._fn = _F
-        return cls._fn.apply(q, target, cst, pose_link, weights)
+        return cls._fn.apply(q, target, cst, pose_link, weights, _torch().is_grad_enabled())
 
 
 class TrajectoryCost:
@@ -209,8 +212,8 @@ class TrajectoryCost:
 
             class _F(torch.autograd.Function):
                 @staticmethod
-                def forward(ctx, q, offsets, cst, weights):
-                    if not ctx.needs_input_grad[0]:
+                def forward(ctx, q, offsets, cst, weights, recorded):
+                    if not (recorded and ctx.needs_input_grad[0]):
                         return traj_cost_grad(cst, q, offsets, want_grad=False, **dict(weights))
                     cost, grad = traj_cost_grad(cst, q, offsets, want_grad=True, **dict(weights))
                     ctx.save_for_backward(q, offsets, grad)
@@ -219,15 +222,15 @@ class TrajectoryCost:
                 @staticmethod
                 def backward(ctx, g):
                     if not ctx.needs_input_grad[0]:
-                        return None, None, None, None
+                        return None, None, None, None, None
                     q, offsets, grad = ctx.saved_tensors
                     # d cost_i / d q_u for u in trajectory i: scale each waypoint row by g[i]
                     counts = offsets[1:] - offsets[:-1]
                     scale = torch.repeat_interleave(g, counts, output_size=q.shape[0])
-                    return (scale[:, None] * grad).to(q.dtype), None, None, None
+                    return (scale[:, None] * grad).to(q.dtype), None, None, None, None
 
             cls._fn = _F
-        return cls._fn.apply(q, offsets, cst, weights)
+        return cls._fn.apply(q, offsets, cst, weights, _torch().is_grad_enabled())
 
 
 def ik_cost(cst, q, target, pose_link, **weights):

@@ -59,3 +59,21 @@ def test_change_in_place_is_refused(setup):
             x += 1.0
         with pytest.raises(RuntimeError, match="modified by an inplace"):
             cost.sum().backward()
+
+
+@pytest.mark.parametrize("mode", [torch.no_grad, torch.inference_mode])
+def test_no_gradient_is_formed_where_none_is_recorded(setup, mode):
+    """A leaf that asks for gradients, in a call that records none: the cost alone, by the memory it takes."""
+    cst, q, t, off = setup
+    x = q.repeat(3000, 1).requires_grad_(True)  # its gradient: 5.9 MB; the cost 0.8 MB
+    tt = t.repeat(3000, 1)
+    offs = torch.arange(0, len(x) + 1, 70, device="cuda")
+    for call in (lambda: diff.ik_cost(cst, x, tt, "link7"), lambda: diff.trajectory_cost(cst, x, offs)):
+        with mode():
+            call()
+            torch.cuda.synchronize()
+            before = torch.cuda.memory_allocated()
+            torch.cuda.reset_peak_memory_stats()
+            cost = call()
+            assert torch.cuda.max_memory_allocated() - before < 4 * x.numel()
+            assert not cost.requires_grad
