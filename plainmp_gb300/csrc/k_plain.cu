@@ -642,7 +642,7 @@ __global__ void __launch_bounds__(NC * 64, 512 / (NC * 64)) k_evaluate64(const P
 }
 
 // Per-sphere signed distances in two launches: the FP64 sphere centres (one thread per configuration:
-// the FK), then the SDF of every (configuration, sphere) in its own thread, so the nearest-point
+// the FK), then the SDF of every (configuration, sphere) in its own thread or warp, so the nearest-point
 // searches of a batch run side by side instead of one configuration's 120 in a row.
 __global__ void k_sphere_centres64(const PmTablesHdr* __restrict__ T, const double* __restrict__ state, const double* __restrict__ q,
                                    int64_t B, int high_accuracy, double* __restrict__ centres) {
@@ -663,18 +663,43 @@ __global__ void k_sphere_centres64(const PmTablesHdr* __restrict__ T, const doub
     }
   }
 }
-// With a point cloud, a warp per sphere (CLOUD), for the cooperative search; else a thread.
+// f(primitive) for each point cloud among n primitives, on every lane of the warp; until f returns false.
+template <class F>
+__device__ __forceinline__ void each_cloud(const PmPrim* prims, int n, const F& f) {
+  for (int base = 0; base < n; base += 32) {
+    const int k = base + (threadIdx.x & 31);
+    // every lane loads: a branch around the load parts the lanes, and all that follows issues twice (k_sphere_sdf64
+    // over 4,096 chain states and the cloud 810 -> 1605 us)
+    const bool is_cloud = prims[min(k, n - 1)].kind == PM_SDF_CLOUD && k < n;
+    __syncwarp();
+    for (unsigned bal = __ballot_sync(0xffffffffu, is_cloud); bal != 0; bal &= bal - 1)
+      if (!f(prims[base + __ffs(bal) - 1])) return;
+  }
+}
+
+// The primitives by a thread per sphere, the point clouds by a warp per sphere (CLOUD), for the cooperative search;
+// `fold`: the other kernel has written the distances to the primitives.  (Both by the warp: every lane evaluated
+// every primitive, and 4,096 chain states against the cloud and 1,000 boxes took 621 ms, split in two 21.)
 template <bool CLOUD>
-__global__ void k_sphere_sdf64(const PmTablesHdr* __restrict__ T, const double* __restrict__ centres, int64_t n,
+__global__ void k_sphere_sdf64(const PmTablesHdr* __restrict__ T, const double* __restrict__ centres, int64_t n, bool fold,
                                double* __restrict__ dist) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (CLOUD) i >>= 5;
   if (i >= n) return;
   TView v(T);
-  const int k = (int)(i % T->n_spheres);
+  const double r = v.sr[(int)(i % T->n_spheres)];
   const D3 c{centres[3 * i], centres[3 * i + 1], centres[3 * i + 2]};
-  double d = INFINITY;
-  for (int pi = 0; pi < T->n_prims; pi++) d = fmin(d, (CLOUD ? prim_eval_warp(v.P[pi], v.C, c) : prim_eval(v.P[pi], v.C, c)) - v.sr[k]);
+  double d = fold ? dist[i] : INFINITY;
+  if (CLOUD) {
+    each_cloud(v.P, T->n_prims, [&](const PmPrim& P) {
+      d = fmin(d, cloud_eval_warp(P, v.C, c) - r);
+      return true;
+    });
+  } else {
+    for (int pi = 0; pi < T->n_prims; pi++)
+      if (v.P[pi].kind != PM_SDF_CLOUD) d = fmin(d, prim_eval(v.P[pi], v.C, c) - r);
+  }
+  __syncwarp();  // every lane has read dist[i]
   if (!CLOUD || (threadIdx.x & 31) == 0) dist[i] = d;
 }
 
@@ -750,9 +775,11 @@ __global__ void k_link_poses(const double* __restrict__ state, const int32_t* __
 }
 
 // ------------------------------------------------------------------ SDF utilities
-// A thread per point, or with point clouds (CLOUD) a warp, for the cooperative search.
+// The primitives by a thread per point, the point clouds by a warp per point (CLOUD), for the cooperative search;
+// `fold`: the other kernel has written the outcome of the primitives.  (Both by the warp: 100,000 points against a
+// cloud and 200 boxes took 53.5 ms, split in two 2.5.)
 template <bool CLOUD>
-__global__ void k_sdf_points(const PmPrim* __restrict__ prims, int n_prims, const PmGridDev* __restrict__ clouds, int is_union,
+__global__ void k_sdf_points(const PmPrim* __restrict__ prims, int n_prims, const PmGridDev* __restrict__ clouds, int is_union, bool fold,
                              const double* __restrict__ pts, const double* __restrict__ radii, int64_t n, double* eval_out,
                              uint8_t* outside_out) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -761,18 +788,30 @@ __global__ void k_sdf_points(const PmPrim* __restrict__ prims, int n_prims, cons
   const bool writer = !CLOUD || (threadIdx.x & 31) == 0;
   D3 p{pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]};
   if (eval_out) {
-    double v = is_union ? 1.7976931348623157e308 : 0.0;
-    for (int k = 0; k < (is_union ? n_prims : min(n_prims, 1)); k++) {
-      const double e = CLOUD ? prim_eval_warp(prims[k], clouds, p) : prim_eval(prims[k], clouds, p);
-      v = is_union ? fmin(v, e) : e;
+    double v = fold ? eval_out[i] : (is_union ? 1.7976931348623157e308 : 0.0);
+    auto take = [&](double e) { v = is_union ? fmin(v, e) : e; };
+    const int m = is_union ? n_prims : min(n_prims, 1);
+    if (CLOUD) {
+      each_cloud(prims, m, [&](const PmPrim& P) {
+        take(cloud_eval_warp(P, clouds, p));
+        return true;
+      });
+    } else {
+      for (int k = 0; k < m; k++)
+        if (prims[k].kind != PM_SDF_CLOUD) take(prim_eval(prims[k], clouds, p));
     }
+    __syncwarp();  // every lane has read eval_out[i]
     if (writer) eval_out[i] = v;
   }
   if (outside_out) {
-    bool o = true;
-    for (int k = 0; k < n_prims && o; k++)
-      o = CLOUD && prims[k].kind == PM_SDF_CLOUD ? cloud_outside_warp(prims[k], clouds, p, radii[i], nullptr)
-                                                 : prim_outside(prims[k], clouds, p, radii[i]);
+    bool o = !fold || outside_out[i] != 0;
+    if (CLOUD) {
+      if (o) each_cloud(prims, n_prims, [&](const PmPrim& P) { return o = cloud_outside_warp(P, clouds, p, radii[i], nullptr); });
+    } else {
+      for (int k = 0; k < n_prims && o; k++)
+        if (prims[k].kind != PM_SDF_CLOUD) o = prim_outside(prims[k], clouds, p, radii[i]);
+    }
+    __syncwarp();
     if (writer) outside_out[i] = o ? 1 : 0;
   }
 }
@@ -850,10 +889,9 @@ cudaError_t launch_sphere_dist64(const PmTablesHdr* T, const PmTablesHdr& h, con
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || !dist) return e;
   const int64_t n = B * h.n_spheres;
-  if (h.n_clouds > 0)
-    k_sphere_sdf64<true><<<grid_for(n, 8), 256, 0, s>>>(T, centres, n, dist);
-  else
-    k_sphere_sdf64<false><<<grid_for(n, 128), 128, 0, s>>>(T, centres, n, dist);
+  const bool prims = h.n_prims > h.n_clouds || h.n_clouds == 0;
+  if (prims) k_sphere_sdf64<false><<<grid_for(n, 128), 128, 0, s>>>(T, centres, n, false, dist);
+  if (h.n_clouds > 0) k_sphere_sdf64<true><<<grid_for(n, 8), 256, 0, s>>>(T, centres, n, prims, dist);
   return cudaGetLastError();
 }
 cudaError_t launch_spheres_of_state(const PmTablesHdr* T, const double* state, int groups, double* out4, cudaStream_t s) {
@@ -874,10 +912,9 @@ cudaError_t launch_check_motion64(const PmTablesHdr* T, const PmTablesHdr& h, co
 cudaError_t launch_sdf_points(const PmPrim* prims, int n_prims, const PmGridDev* clouds, int n_clouds, int is_union,
                               const double* pts, const double* radii, int64_t n, double* eval_out, uint8_t* outside_out, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  if (n_clouds > 0)
-    k_sdf_points<true><<<grid_for(n, 8), 256, 0, s>>>(prims, n_prims, clouds, is_union, pts, radii, n, eval_out, outside_out);
-  else
-    k_sdf_points<false><<<grid_for(n, 128), 128, 0, s>>>(prims, n_prims, clouds, is_union, pts, radii, n, eval_out, outside_out);
+  const bool others = n_prims > n_clouds || n_clouds == 0;
+  if (others) k_sdf_points<false><<<grid_for(n, 128), 128, 0, s>>>(prims, n_prims, clouds, is_union, false, pts, radii, n, eval_out, outside_out);
+  if (n_clouds > 0) k_sdf_points<true><<<grid_for(n, 8), 256, 0, s>>>(prims, n_prims, clouds, is_union, others, pts, radii, n, eval_out, outside_out);
   return cudaGetLastError();
 }
 cudaError_t launch_cloud_nearest(const PmGridDev* grid, const double* pts, int64_t n, double* sq, double* near3,

@@ -296,9 +296,8 @@ __device__ __forceinline__ bool cloud_outside_warp(const PmPrim& P, const PmGrid
   return sqrt(nn.d2) - P.a > r;
 }
 
-// prim_eval with the warp search for a point cloud.  Warp-uniform arguments; every lane gets the value.
-__device__ __forceinline__ double prim_eval_warp(const PmPrim& P, const PmGridDev* clouds, const D3& p) {
-  if (P.kind != PM_SDF_CLOUD) return prim_eval(P, clouds, p);
+// prim_eval of a point cloud with the warp search.  Warp-uniform arguments; every lane gets the value.
+__device__ __forceinline__ double cloud_eval_warp(const PmPrim& P, const PmGridDev* clouds, const D3& p) {
   return sqrt(warp_nearest64(clouds[P.cloud], p).d2) - P.a;
 }
 
