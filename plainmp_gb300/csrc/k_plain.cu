@@ -254,8 +254,46 @@ __global__ void __launch_bounds__(NC * WPC * 32, (NC > 1 ? 1024 : 512) / (NC * W
   if (threadIdx.x < ncfg) out[c0 + threadIdx.x] = failed[threadIdx.x] ? 0 : 1;
 }
 
-// CustomValidatorBase::checkMotion (motion_validator.cpp:17-79), a block per edge: its waypoints in the
-// reference's visiting order, NC at a time, a warp each; the first round with a collision ends it.
+// Step ratio of checkMotion on the edge a -> b (motion_validator.cpp:17-79).  inv: 1 / width, computed once a block
+// (FP64 divisions were most of the time of an edge without length).
+__device__ double edge_step(int type, const double* a, const double* b, const double* width, const double* inv, double resolution, int dim) {
+  if (type == 0) {  // BoxMotionValidator::determine_step_ratio (:89-111)
+    double diff_long = 0.0, max_diff = -INFINITY;
+    int li = 0;
+    for (int i = 0; i < dim; i++) {
+      const double diff = b[i] - a[i];
+      const double asd = fabs(diff) * inv[i];
+      if (asd > max_diff) {
+        max_diff = asd;
+        li = i;
+        diff_long = diff;
+      }
+    }
+    return fabs(diff_long) < 1e-6 ? INFINITY : width[li] / fabs(diff_long);
+  }
+  double dist = 0.0;  // EuclideanMotionValidator (:118-126)
+  for (int i = 0; i < dim; i++) {
+    const double d = a[i] - b[i];
+    dist += d * d;
+  }
+  return resolution / sqrt(dist);
+}
+// Waypoints to check, or 0 where the step ratio decides: `valid` is the answer then.  NaN / non-positive ratios,
+// and edges needing more than 2^26 waypoints, are reported invalid instead of looping (the reference has no bound
+// here).
+__device__ int edge_waypoints(double sr, bool& valid) {
+  valid = sr == INFINITY;
+  if (valid || !(sr > 0.0) || 1.0 / sr > 67108864.0) return 0;
+  return (int)(floor(1 / sr) + 1);
+}
+// Coordinate of waypoint k of n: b for k = 0, then the interior points in visiting order (:45-78).
+__device__ __forceinline__ double edge_value(double a, double b, double sr, int n, int k, const int16_t* __restrict__ seq) {
+  if (k == 0) return b;
+  return a + (b - a) * (n < 128 ? (double)seq[n * 128 + (k + 1)] * sr : (double)k * sr);
+}
+
+// CustomValidatorBase::checkMotion, a block per edge: its waypoints in the reference's visiting order, NC at a
+// time, a warp each; the first round with a collision ends it.
 // n_checked (a sum) and counts (per edge), each optional, count the waypoints up to and including the first
 // that collides, as the reference visits them.  The endpoints go to shared memory first: small calls pass them
 // in page-locked host memory.
@@ -267,9 +305,9 @@ __global__ void __launch_bounds__(NC * 32, 512 / (NC * 32)) k_check_motion64(con
                                                             unsigned long long* n_checked, unsigned long long* counts) {
   extern __shared__ __align__(16) double team_mem[];
   __shared__ int failed[NC];
-  __shared__ double ends[2][PM_MAX_DOF], wd[PM_MAX_DOF];
+  __shared__ double ends[2][PM_MAX_DOF], inv[PM_MAX_DOF];
   __shared__ double step;
-  __shared__ unsigned long long n_way;  // waypoints to check (0: decided already)
+  __shared__ int n_way;  // waypoints to check (0: decided already)
   const TView v(T);
   const Image im(T);
   const int64_t e = blockIdx.x;
@@ -278,62 +316,27 @@ __global__ void __launch_bounds__(NC * 32, 512 / (NC * 32)) k_check_motion64(con
   for (int i = threadIdx.x; i < dim; i += NC * 32) {
     ends[0][i] = s1[e * dim + i];
     ends[1][i] = s2[e * dim + i];
-    if (type == 0) wd[i] = width[i];
+    if (type == 0) inv[i] = 1.0 / width[i];
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    double sr;
-    if (type == 0) {  // BoxMotionValidator::determine_step_ratio (:89-111)
-      double diff_long = 0.0, max_diff = -INFINITY;
-      int li = 0;
-      for (int i = 0; i < dim; i++) {
-        double diff = b[i] - a[i];
-        double asd = fabs(diff) * (1.0 / wd[i]);
-        if (asd > max_diff) {
-          max_diff = asd;
-          li = i;
-          diff_long = diff;
-        }
-      }
-      sr = fabs(diff_long) < 1e-6 ? INFINITY : wd[li] / fabs(diff_long);
-    } else {  // EuclideanMotionValidator (:118-126)
-      double dist = 0.0;
-      for (int i = 0; i < dim; i++) {
-        double d = a[i] - b[i];
-        dist += d * d;
-      }
-      sr = resolution / sqrt(dist);
-    }
-    step = sr;
-    n_way = 0;
+    bool valid;
+    step = edge_step(type, a, b, width, inv, resolution, dim);
+    n_way = edge_waypoints(step, valid);
     if (counts) counts[e] = 0;
-    if (sr == INFINITY) {
-      out[e] = 1;
-    } else if (!(sr > 0.0) || 1.0 / sr > 67108864.0) {
-      // NaN / non-positive step ratios, and edges needing more than 2^26 waypoints, are reported
-      // invalid instead of looping (the reference has no bound here)
-      out[e] = 0;
-    } else {
-      n_way = (unsigned long long)(floor(1 / sr) + 1);
-    }
+    if (n_way == 0) out[e] = valid;
   }
   __syncthreads();
   const double sr = step;
-  const unsigned long long n = n_way;
+  const int n = n_way;
   if (n == 0) return;  // block-uniform
   float* p32 = reinterpret_cast<float*>(team_mem + (size_t)NC * nsl * kRec);
-  unsigned long long k0 = 0, checked = n;
+  int k0 = 0, checked = n;
   bool ok = true;
   for (; k0 < n && ok; k0 += NC) {  // block-uniform
-    const int ncfg = (int)min((unsigned long long)NC, n - k0);
+    const int ncfg = min(NC, n - k0);
     if (threadIdx.x < NC) failed[threadIdx.x] = 0;
-    // waypoint k: s2 for k = 0, then the interior points in visiting order (:45-78)
-    auto qf = [&](int c, int col) {
-      const unsigned long long k = k0 + c;
-      if (k == 0) return b[col];
-      const double t = n + 1 < 129 ? (double)seq[n * 128 + (k + 1)] * sr : (double)k * sr;
-      return a[col] + (b[col] - a[col]) * t;
-    };
+    auto qf = [&](int c, int col) { return edge_value(a[col], b[col], sr, n, k0 + c, seq); };
     fk64_block<NC * 32>(v, state, qf, ncfg, T->base_type == PM_BASE_FIXED, kNorm2Valid, team_mem, p32);
     const int c = threadIdx.x >> 5;
     if (c < ncfg) valid_team<1>(v, im, TeamPose{team_mem + (size_t)c * nsl * kRec, p32 + (size_t)c * nsl * kRec32}, 0, failed + c);
@@ -347,8 +350,93 @@ __global__ void __launch_bounds__(NC * 32, 512 / (NC * 32)) k_check_motion64(con
   }
   if (threadIdx.x == 0) {
     out[e] = ok ? 1 : 0;
-    if (n_checked) atomicAdd(n_checked, checked);
+    if (n_checked) atomicAdd(n_checked, (unsigned long long)checked);
     if (counts) counts[e] = checked;
+  }
+}
+
+// The same for more edges than SMs, G (up to 64) edges a block: the waypoints of its edges in a row, NC at a time,
+// leaving out those of an edge that has collided.  A block an edge, as above, has NC - 1 warps idle where edges are
+// of one waypoint, and starts a block for each edge without length: 100,000 chain edges of one waypoint took 7.4 ms,
+// 1.41 this way; of no length 1.01 ms, 0.10; 20,000 of three 1.66 ms, 0.84; 1,000 of twenty 0.24 ms either way.
+// (Up to 32 a block 1.34 and 0.13 ms for the first two, up to 128 1.50 and 0.10.)
+constexpr int kEdgesPerBlock = 64;
+static_assert(kEdgesPerBlock % 32 == 0, "whole warps");
+template <int NC>
+__global__ void __launch_bounds__(NC * 32, 512 / (NC * 32)) k_check_motions64(const PmTablesHdr* __restrict__ T, const double* __restrict__ state,
+                                                            const double* __restrict__ s1, const double* __restrict__ s2, int64_t E, int G,
+                                                            int type, const double* __restrict__ width, double resolution,
+                                                            const int16_t* __restrict__ seq, uint8_t* __restrict__ out,
+                                                            unsigned long long* n_checked, unsigned long long* counts) {
+  extern __shared__ __align__(16) double team_mem[];
+  __shared__ int failed[NC];
+  __shared__ double step[kEdgesPerBlock], inv[PM_MAX_DOF];
+  __shared__ int n_way[kEdgesPerBlock];   // waypoints of an edge (0: decided already)
+  __shared__ int checked[kEdgesPerBlock];  // up to its first collision (0: none yet)
+  __shared__ int task_e[NC], task_k[NC], n_task;
+  static_assert(kEdgesPerBlock <= NC * 32, "a thread an edge");
+  const TView v(T);
+  const Image im(T);
+  const int tid = threadIdx.x;
+  const int64_t e0 = (int64_t)blockIdx.x * G;
+  const int ge = (int)min((int64_t)G, E - e0);
+  const int dim = T->q_dim, nsl = T->n_slots;
+  if (type == 0)
+    for (int i = tid; i < dim; i += NC * 32) inv[i] = 1.0 / width[i];
+  __syncthreads();
+  if (tid < ge) {
+    const int64_t e = e0 + tid;
+    bool valid;
+    step[tid] = edge_step(type, s1 + e * dim, s2 + e * dim, width, inv, resolution, dim);
+    n_way[tid] = edge_waypoints(step[tid], valid);
+    checked[tid] = 0;
+    if (n_way[tid] == 0) out[e] = valid;
+  }
+  __syncthreads();
+  float* p32 = reinterpret_cast<float*>(team_mem + (size_t)NC * nsl * kRec);
+  int ce = 0, ck = 0;  // thread 0: the next edge and waypoint
+  for (;;) {  // block-uniform
+    if (tid == 0) {
+      int m = 0;
+      while (m < NC && ce < ge) {
+        if (ck >= n_way[ce] || checked[ce]) {
+          ce++;
+          ck = 0;
+        } else {
+          task_e[m] = ce;
+          task_k[m] = ck++;
+          failed[m++] = 0;
+        }
+      }
+      n_task = m;
+    }
+    __syncthreads();
+    const int ncfg = n_task;
+    if (ncfg == 0) break;
+    auto qf = [&](int c, int col) {
+      const int i = task_e[c];
+      const int64_t at = (e0 + i) * dim + col;
+      return edge_value(s1[at], s2[at], step[i], n_way[i], task_k[c], seq);
+    };
+    fk64_block<NC * 32>(v, state, qf, ncfg, T->base_type == PM_BASE_FIXED, kNorm2Valid, team_mem, p32);
+    const int c = tid >> 5;
+    if (c < ncfg) valid_team<1>(v, im, TeamPose{team_mem + (size_t)c * nsl * kRec, p32 + (size_t)c * nsl * kRec32}, 0, failed + c);
+    __syncthreads();
+    if (tid == 0)
+      for (int i = 0; i < ncfg; i++)
+        if (failed[i] && !checked[task_e[i]]) checked[task_e[i]] = task_k[i] + 1;
+  }
+  if (tid < kEdgesPerBlock) {  // whole warps
+    unsigned long long n = 0;
+    if (tid < ge) {
+      if (n_way[tid] > 0) {
+        n = checked[tid] ? checked[tid] : n_way[tid];
+        out[e0 + tid] = checked[tid] ? 0 : 1;
+      }
+      if (counts) counts[e0 + tid] = n;
+    }
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    if ((tid & 31) == 0 && n > 0 && n_checked) atomicAdd(n_checked, n);
   }
 }
 
@@ -907,7 +995,10 @@ cudaError_t launch_check_motion64(const PmTablesHdr* T, const PmTablesHdr& h, co
   if (e != cudaSuccess) return e;
   if (E <= n_sm)
     return team_launch(k_check_motion64<16>, E, 16, 1, h, s, T, state, s1, s2, type, width, resolution, seq, out, n_checked, counts);
-  return team_launch(k_check_motion64<8>, E, 8, 1, h, s, T, state, s1, s2, type, width, resolution, seq, out, n_checked, counts);
+  // more edges a block while 8 blocks per SM (4 rounds of resident ones) are left
+  const int G = (int)std::min<int64_t>(std::max<int64_t>(E / (8 * (int64_t)n_sm), 1), kEdgesPerBlock);
+  return team_launch(k_check_motions64<8>, (E + G - 1) / G, 8, 1, h, s, T, state, s1, s2, E, G, type, width, resolution, seq, out, n_checked,
+                     counts);
 }
 cudaError_t launch_sdf_points(const PmPrim* prims, int n_prims, const PmGridDev* clouds, int n_clouds, int is_union,
                               const double* pts, const double* radii, int64_t n, double* eval_out, uint8_t* outside_out, cudaStream_t s) {
