@@ -1026,14 +1026,21 @@ struct HostCst {
   }
 
   // Launch shape and tuning of a fast call of B configurations where the caller set none.  Tiles of 8 spheres.
-  // (8, 256) while every such block is resident at once (4 of 256 threads per SM: 4,864 configurations), where
-  // the latency of one block is the kernel's; (16, 256) while those are.  Calls with distances at (16, 256) and
-  // (8, 256), us: 1,001 states of the chain x 20 primitives 49 -> 42, of the dual arm x primitives 45 -> 31, of
-  // the dual arm x cloud 50 -> 42; 4,096: 49 -> 47, 62 -> 54, 65 -> 61.  Beyond that, robots of up to 64 spheres run (16, 128), twice as many blocks in
-  // flight; larger ones stay at (16, 256).  Measured against (32, 256) with the least tile, us:
-  // dual arm (120 spheres) x cloud, 65,536 with distances 622 -> 510, 200,003 validity 630 -> 469; chain
-  // (56) x 20 primitives, 4,096 with distances 81 -> 64, 65,536 273 -> 218; 16,384 at (16, 256) 97, at
-  // (16, 128) 89; the same chain at 4,096 and (16, 128) 76.
+  // resident(c): blocks of c configurations and 256 threads that run at once (4 per SM, fewer where the tables leave
+  // no room for 4).
+  // (8, 256) while every such block is resident, where the latency of one block is the kernel's; (16, 256) while
+  // those are.  Calls with distances at (16, 256) and (8, 256), us: 1,001 states of the chain (56 spheres) x 20
+  // primitives 49 -> 42, of the dual arm (120) x primitives 45 -> 31, of the dual arm x cloud 50 -> 42; 4,096: 49 ->
+  // 47, 62 -> 54, 65 -> 61.  Blocks that are not all resident only stage the tables more often: 4,096 chain states
+  // x the cloud and 1,000 boxes, two blocks an SM, 455 at (16, 256), 775 at (8, 256).
+  // Beyond that (16, 128) where eight of its blocks fit an SM (28,160 bytes each; seven for up to 64 spheres), else
+  // (16, 256): 65,536 states at (16, 256) and (16, 128), us, validity: chain x 20 primitives 178 -> 137, 60 to 120
+  // spheres on the dual arm x 20 (24.8 to 26.7 KB) 217 -> 199 to 236 -> 219, 350 on the chain (23.0 KB) 862 -> 660;
+  // dual arm x cloud (40.5 KB) 171 -> 190; distances: chain 223 -> 195, 60 spheres (28.6 KB) 259 -> 254, 120
+  // (34.4 KB) 305 -> 353.
+  // (32, 256) for the validity of robots of more than 256 spheres against up to 32 primitives: fewer warps a
+  // configuration find its collision before the others have started.  9,000 states of the chain with 350 spheres x 8
+  // primitives 312 us at (16, 256), 241 at (32, 256); 65,536 with 1,400 spheres 9,129 -> 8,338.
   FastTuning fast_shape(int64_t B, bool want_dist, int* cpb, int* nt) const {
     *cpb = fast_cpb;
     *nt = fast_nt;
@@ -1042,8 +1049,19 @@ struct HostCst {
     if (!shape_set && fast_smem_bytes(hdr, fast_cpb, want_dist) <= 200 * 1024) {  // what does not fit at (32, 256) is refused as it was
       int n_sm = 0;
       cuda_check(sm_count(&n_sm), "device attribute");
-      *cpb = B <= 8 * 4 * (int64_t)n_sm ? 8 : 16;
-      *nt = (B + 15) / 16 > 4 * (int64_t)n_sm && hdr.n_spheres <= 64 ? 128 : 256;
+      auto resident = [&](int c) {  // 228 KB an SM, 1 KB of it a block's own
+        return n_sm * std::min<int64_t>(4, 228 * 1024 / (int64_t)(fast_smem_bytes(hdr, c, want_dist) + 1024));
+      };
+      const size_t sm16 = fast_smem_bytes(hdr, 16, want_dist);
+      *cpb = 16;
+      *nt = 256;
+      if ((B + 7) / 8 <= resident(8)) {
+        *cpb = 8;
+      } else if ((B + 15) / 16 > resident(16) && sm16 <= 228 * 1024 / (hdr.n_spheres <= 64 ? 7 : 8) - 1024) {
+        *nt = 128;
+      } else if (!want_dist && hdr.n_spheres > 256 && hdr.n_prims <= 32 && hdr.n_clouds == 0) {
+        *cpb = 32;
+      }
     }
     return t;
   }
