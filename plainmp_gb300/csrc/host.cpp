@@ -178,6 +178,13 @@ constexpr int64_t kZeroCopy = 64;
 // The same for validity-only calls of the fast path (with distances, the results are copied).
 constexpr int64_t kZeroCopyFast = 2048;
 
+// |v|^2 above 1 by more than rounding (a quaternion or axis that is none of a rotation), or not finite
+static bool above_unit(const double* v, int n) {
+  double s = 0.0;
+  for (int k = 0; k < n; k++) s += v[k] * v[k];
+  return !(s <= 1.0 + 1e-7);
+}
+
 // ---------------------------------------------------------------------------- host quaternion
 // construction-time helpers (setQuaternionFromRPY, transform.hpp:122-130)
 static void quat_from_rpy(double r, double p, double y, double q[4]) {
@@ -211,7 +218,7 @@ struct HostModel {
   std::vector<double> state_init;  // rows of PM_STATE_STRIDE doubles (row 0 = base)
   std::vector<double> angles;
   double base7[7] = {0, 0, 0, 0, 0, 0, 1};
-  uint64_t version = 1;  // bumped when the link set changes
+  uint64_t version = 1;  // bumped when the link set changes, or the base pose leaves or regains unit norm
   // device
   DevBuf d_state;
   DevBuf d_parents;
@@ -771,12 +778,28 @@ struct HostCst {
     }
   }
 
+  // Whether a rotation of the constraint's links may be off unit norm: URDF axes, fixed transforms and base poses are
+  // taken as they are given.  The fast kernels' error bounds, and that a colliding sphere lies in its group's sphere,
+  // hold for rotations (to 1e-3 and more), so such a constraint's configurations and edges are all decided by the
+  // exact check of the recheck kernel, as those whose terms overflow the queue, and its groups are never culled (FP32
+  // radius kNoCull), which leaves the fast kernels the distances.
+  static constexpr float kNoCull = 1e6f;
+  bool off_unit() const {
+    const HostModel& m = *kin;
+    if (base_type == PM_BASE_FIXED && above_unit(m.base7 + 3, 4)) return true;
+    for (const HostJoint& j : m.joints)
+      if (slot_of_link[j.child] >= 0 && j.type != UJ_PRISMATIC && above_unit(j.axis, 3)) return true;
+    for (int l = 0; l < m.n_link(); l++)
+      if (slot_of_link[l] >= 0 && above_unit(&m.state_init[(size_t)PM_STATE_LINK_ROW(l) * PM_STATE_STRIDE], 4)) return true;
+    return false;
+  }
+
   // The FP32 image of the tables: the records of the fast kernels as a block keeps them.  Slots
   // without a control joint and the base pose are filled in by the block from the model state.
   static std::vector<char> fast_image(const std::vector<PmSlot>& slots, const std::vector<PmGroup>& groups, const std::vector<double>& sx,
                                       const std::vector<double>& sy, const std::vector<double>& sz, const std::vector<double>& sr,
                                       const std::vector<int32_t>& sgroup, const std::vector<int32_t>& pairs,
-                                      const std::vector<PmPrim>& prims) {
+                                      const std::vector<PmPrim>& prims, bool off_unit) {
     std::vector<char> img;
     auto add = [&](const void* p, size_t bytes) {
       const size_t off = img.size();
@@ -809,7 +832,7 @@ struct HostCst {
     for (size_t i = 0; i < groups.size(); i++) {
       const PmGroup& G = groups[i];
       const float v[3] = {(float)G.rel[0], (float)G.rel[1], (float)G.rel[2]};
-      gr[i] = PmGroupF{{v[0], v[1], v[2]}, (float)G.radius, G.slot, G.begin, G.count, G.only_self, G.radius < 1e-6, norm_up(v), {0, 0}};
+      gr[i] = PmGroupF{{v[0], v[1], v[2]}, off_unit ? kNoCull : (float)G.radius, G.slot, G.begin, G.count, G.only_self, G.radius < 1e-6, norm_up(v), {0, 0}};
     }
     std::vector<PmPrimF> pr(prims.size());
     for (size_t i = 0; i < prims.size(); i++) {
@@ -956,6 +979,7 @@ struct HostCst {
     h.q_dim = q_dim();
     h.base_type = base_type;
     h.root_slot = slot_of_link[m.root];
+    h.off_unit = off_unit();
     h.n_clouds = (int)clouds.size();
     std::vector<char> buf;
     auto align = [&]() {
@@ -995,7 +1019,7 @@ struct HostCst {
     lev.insert(lev.end(), by_depth.begin(), by_depth.end());
     h.n_levels = n_levels;
     h.off_lev = put(lev.data(), lev.size() * 4);
-    const std::vector<char> img = fast_image(slots, grec, sx, sy, sz, sr, sgroup, prs, prims);
+    const std::vector<char> img = fast_image(slots, grec, sx, sy, sz, sr, sgroup, prs, prims, h.off_unit != 0);
     h.img_bytes = (int64_t)img.size();
     h.off_img = put(img.data(), img.size());
     align();
@@ -1375,6 +1399,7 @@ int pmgpu_model_set_base_pose(pmgpu_model* m, const double* pose7) {
   return guarded([&] {
     check_ptr(m, "model");
     HostModel& M = *m->m;
+    if (above_unit(M.base7 + 3, 4) != above_unit(pose7 + 3, 4)) M.version++;  // the constraints' tables depend on it
     std::memcpy(M.base7, pose7, sizeof(M.base7));
     const double q[4] = {pose7[3], pose7[4], pose7[5], pose7[6]}, t[3] = {pose7[0], pose7[1], pose7[2]};
     set_row(M.state_init, PM_STATE_BASE_ROW, q, t, false);
@@ -2077,7 +2102,7 @@ static void fast_host_pipelined(HostCst& C, const PmTablesHdr* T, const double* 
     items[k] = (int4*)P.items[k].ensure((size_t)cap * sizeof(int4));
   }
   cuda_check(cudaMemsetAsync(ctl, 0, (size_t)n_chunks * 64, s), "memset");
-  cuda_check(cudaMemsetAsync(ovf, 0, std::max<size_t>((size_t)B, 16), s), "memset");
+  cuda_check(cudaMemsetAsync(ovf, C.hdr.off_unit, std::max<size_t>((size_t)B, 16), s), "memset");
   cuda_check(cudaEventRecord(P.ev_in, s), "event");  // the second stream starts after the caller's prior work
   cuda_check(cudaStreamWaitEvent(P.aux, P.ev_in, 0), "event");
   for (int64_t i = 0; i < n_chunks; i++) {
@@ -2135,6 +2160,7 @@ static int fast_valid_entry(pmgpu_cst* c, const double* q, int64_t B, uint8_t* o
     unsigned long long* dstats = (unsigned long long*)(ctl + 16);
     uint8_t* ovf = (uint8_t*)ctl + 64;
     cuda_check(cudaMemsetAsync(ctl, 0, 64 + (size_t)B, s), "memset");
+    if (C.hdr.off_unit && B) cuda_check(cudaMemsetAsync(ovf, 1, (size_t)B, s), "memset");
     const double* dq = q;
     uint8_t* dout = out;
     float* dd = dist32;
@@ -2306,6 +2332,7 @@ static int fast_edges_entry(pmgpu_cst* c, const double* s1, const double* s2, in
     unsigned long long* dstats = (unsigned long long*)(ctl + 16);
     uint8_t* ovf = (uint8_t*)ctl + 64;
     cuda_check(cudaMemsetAsync(ctl, 0, 64 + En, s), "memset");
+    if (C.hdr.off_unit) cuda_check(cudaMemsetAsync(ovf, 1, En, s), "memset");
     const double* d1 = s1;
     const double* d2 = s2;
     uint8_t* dout = out;

@@ -712,7 +712,7 @@ struct EdgeSource {
   __device__ void full_check(const TView& v, const double* state, int64_t e, double* buf) const {
     bool ok = true;
     for (int64_t w = off[e]; w < off[e] + n[e] && ok; w++) ok = is_valid_cfg(v, state, cfg(v.T, w, buf), bnd);
-    if (!ok) valid[e] = 0;
+    if (n[e] > 0) valid[e] = ok;
   }
 };
 

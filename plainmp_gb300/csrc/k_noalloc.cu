@@ -95,7 +95,7 @@ extern "C" int pmgpu_cst_is_valid_fast_noalloc(pmgpu_cst* c, const double* q, in
   int4* items = reinterpret_cast<int4*>(base + kCtlBytes);
   uint8_t* overflow = base + kCtlBytes + kQueueBytes;
   cudaError_t e = cudaMemsetAsync(base, 0, kCtlBytes, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(overflow, 0, (size_t)B, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(overflow, hdr.off_unit, (size_t)B, s);
   if (e == cudaSuccess)
     e = pmg::launch_fast_valid(T, hdr, state, q, B, out, dist32, 0.1f, items, count, kQueueItems, overflow, stats, cpb, nt, s);
   if (e != cudaSuccess) {

@@ -45,14 +45,15 @@ def pair(request, oracle):
         pose[3:] *= scale
         kin.set_base_pose(pose)
         m.set_base_pose(pose)
-    return cst, oc
+    # a bound of |q|^2 along the chain: the even joints' axes, the base
+    return cst, oc, max(1.0, scale ** 2) ** (4 if what == "axes" else 1)
 
 
 N = 20000  # enough that an error bound short by a few orders meets a decision or a least term
 
 
 def test_fp64_method_decides(pair):
-    cst, oc = pair
+    cst, oc, n2 = pair
     Q = W.chain7_configs(N, seed=31)
     ref = oc.is_valid(Q, threads=8)
     assert 0 < ref.sum() < N
@@ -64,7 +65,7 @@ def test_fp64_method_decides(pair):
 def test_fp64_values(pair):
     """The least value is the reference's: same term, so the same bits up to sin and cos (2 units in the last place of
     each joint, carried by transforms of up to 1e3: 1e-9; a wrong term is off by more than its FP32 bound, 1e-6)."""
-    cst, oc = pair
+    cst, oc, n2 = pair
     Q = W.chain7_configs(N, seed=33)
     rv, _ = oc.evaluate(Q, threads=8)
     v, _ = cst.evaluate_batch(Q)
@@ -72,9 +73,29 @@ def test_fp64_values(pair):
 
 
 def test_fast_path_decides(pair):
-    cst, oc = pair
+    cst, oc, n2 = pair
     Q = W.chain7_configs(N, seed=35)
     ref = oc.is_valid(Q, threads=8)
     assert np.array_equal(cst.is_valid_fast(Q), ref)
     s1, s2 = Q[:200], Q[:200] + np.linspace(-0.2, 0.2, 7)
     assert np.array_equal(BoxMotionValidator(cst, [0.05] * 7).check_motion_fast(s1, s2), oc.check_motion(s1, s2, 0, width=[0.05] * 7)[0])
+
+
+def test_fast_path_agrees_on_many_states(pair):
+    """Two million states, against the FP64 method: decisions inside a bound that is too small are few."""
+    import torch
+
+    cst, _, n2 = pair
+    for k in range(10):
+        Q = torch.from_numpy(W.chain7_configs(200_000, seed=100 + k)).cuda()
+        assert torch.equal(cst.is_valid_fast(Q), cst.is_valid_batch(Q))
+
+
+def test_fast_distances(pair):
+    """The FP32 distance bound of unit rotations (1e-6 + 64 units of roundoff of magnitudes below 20 m) times n2, which
+    every error of a rotated vector is proportional to at most."""
+    cst, oc, n2 = pair
+    Q = W.chain7_configs(2000, seed=37)
+    _, d = cst.is_valid_fast(Q, distances=True)
+    ref = np.minimum(oc.sphere_distances(Q, threads=8), 0.1)
+    assert np.abs(d.astype(np.float64) - ref).max() < (1e-6 + 64 * 2.0 ** -24 * 21) * n2
