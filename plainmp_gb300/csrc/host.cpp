@@ -1070,7 +1070,7 @@ struct HostCst {
     *nt = fast_nt;
     FastTuning t = tune;
     if (t.sphere_tile_log2 < 0) t.sphere_tile_log2 = 3;
-    if (!shape_set && fast_smem_bytes(hdr, fast_cpb, want_dist) <= 200 * 1024) {  // what does not fit at (32, 256) is refused as it was
+    if (!shape_set) {
       int n_sm = 0;
       cuda_check(sm_count(&n_sm), "device attribute");
       auto resident = [&](int c) {  // 228 KB an SM, 1 KB of it a block's own
@@ -1086,6 +1086,10 @@ struct HostCst {
       } else if (!want_dist && hdr.n_spheres > 256 && hdr.n_prims <= 32 && hdr.n_clouds == 0) {
         *cpb = 32;
       }
+      while (*cpb > 8 && fast_smem_bytes(hdr, *cpb, want_dist) > kFastSmemMax) {  // large tables
+        *cpb /= 2;
+        *nt = 256;
+      }
     }
     return t;
   }
@@ -1099,7 +1103,7 @@ struct HostCst {
     *nt = edge_nt;
     FastTuning t = tune;
     if (t.sphere_tile_log2 < 0) t.sphere_tile_log2 = 3;
-    if (!tune_set && fast_smem_bytes(hdr, edge_cpb, false) <= 200 * 1024) *cpb = 16;  // what does not fit at (32, 128) is refused as it was
+    if (!tune_set) *cpb = 16;
     return t;
   }
 

@@ -1629,7 +1629,7 @@ cudaError_t launch_fast_valid(const PmTablesHdr* T, const PmTablesHdr& h, const 
   Scratch scr{items, count, cap, overflow, stats, split ? static_cast<HardQuery*>(hq) : nullptr, split ? hq_count : nullptr,
               split ? hq_cap : 0u, tune.sphere_tile_log2, bnd};
   size_t sm = fast_smem_bytes(h, cpb, dist32 != nullptr);
-  if (sm > 200 * 1024) return cudaErrorInvalidConfiguration;
+  if (sm > kFastSmemMax) return cudaErrorInvalidConfiguration;
   unsigned grid = (unsigned)((B + cpb - 1) / cpb);
   cudaError_t e;
   int n_sm = 0;
@@ -1699,7 +1699,7 @@ cudaError_t launch_fast_edges(const PmTablesHdr* T, const PmTablesHdr& h, const 
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   EdgeSource src{s1, s2, off, n, sr, seq, E, out, bnd};
   size_t sm = fast_smem_bytes(h, cpb, false);
-  if (sm > 200 * 1024) return cudaErrorInvalidConfiguration;
+  if (sm > kFastSmemMax) return cudaErrorInvalidConfiguration;
   bool launched = false;
   // persistent blocks, at most 4 per edge (a few chunks of waypoints each): a small call stages the
   // tables in few blocks

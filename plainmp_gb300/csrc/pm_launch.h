@@ -42,6 +42,8 @@ cudaError_t launch_check_motion64(const PmTablesHdr* T, const PmTablesHdr& h, co
 
 // ---- fast path (k_fast.cu): FP32 decisions + FP64 recheck of uncertain terms.
 size_t fast_smem_bytes(const PmTablesHdr& h, int cpb, bool want_dist);
+// The most a launch may ask for: 227 KB a block, less the edge kernel's static part; larger tables are refused.
+constexpr size_t kFastSmemMax = 225 * 1024;
 // The fast kernels' queue records hold at most 65,535 spheres and 32,767 primitives.
 bool fast_table_sizes_ok(const PmTablesHdr& h);
 // SM count of the current device (cached per device); the offset table of the warp searches,

@@ -114,3 +114,36 @@ def two_threads_of_costs():
 
 def test_threads_of_costs_with_tables_of_different_sizes():
     _child("two_threads_of_costs()")
+
+
+def test_largest_tables_of_the_fast_calls():
+    """A chain of 6,357 spheres against 20 primitives, about the most that a block's shared memory holds: validity,
+    edges and the call that allocates nothing, against the FP64 method."""
+    import ctypes as C
+
+    import torch
+
+    from plainmp_gb300._lib import lib
+
+    from plainmp_gb300 import BoxMotionValidator, scenes
+    from plainmp_gb300 import workloads as W
+
+    r, rng, specs = W.chain7_robot(), np.random.default_rng(1), []
+    for k, s in enumerate(r.spheres):
+        lo, hi = s.relative_positions.min(1, keepdims=True), s.relative_positions.max(1, keepdims=True)
+        n = 908 + (k == 0)
+        specs.append(W.SphereSpec(s.parent_link_name, lo + (hi - lo) * rng.uniform(size=(3, n)), rng.uniform(0.001, 0.01, n)))
+    many = W.Robot(r.urdf, r.control_joints, r.end_link, specs, [])
+    _, cst, _ = scenes.make_constraint(many, W.chain7_scene(), reorder=False)
+    assert cst.n_spheres == 6357
+    Q = torch.from_numpy(W.chain7_configs(300, seed=8)).cuda()
+    ref = cst.is_valid_batch(Q)
+    assert 0 < int(ref.sum()) < len(ref)
+    assert torch.equal(cst.is_valid_fast(Q), ref)
+    v = BoxMotionValidator(cst, [0.05] * 7)
+    assert torch.equal(v.check_motion_fast(Q, Q + 0.07), v.check_motion_batch(Q, Q + 0.07))
+    out = torch.full_like(ref, 7)
+    torch.cuda.synchronize()
+    assert lib.pmgpu_cst_is_valid_fast_noalloc(cst._h, C.c_void_p(Q.data_ptr()), C.c_int64(len(Q)), C.c_void_p(out.data_ptr()), None, None) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(out, ref)
