@@ -188,18 +188,19 @@ int pmgpu_cst_is_valid_fast(pmgpu_cst* c, const double* q, int64_t B, uint8_t* o
                             int mem, void* stream);
 
 /* Launch shape of the fast kernel: configurations per block and threads per block, one of
- * (16,128) (32,128) (16,256) (32,256) (64,256) (32,512) (64,512) (128,512); chosen per workload by the
- * autotuner (plainmp_gb300/autotune.py).  Until it is set, each call chooses by the batch and sphere
- * counts, and the getter gives (32,256).  No counterpart in the reference. */
+ * (8,256) (16,128) (32,128) (16,256) (32,256) (64,256) (32,512) (64,512) (128,512); chosen per workload by the
+ * autotuner (plainmp_gb300/autotune.py).  (32,256), the default, leaves the choice to each call, by its batch,
+ * the tables' size and the robot's spheres.  No counterpart in the reference. */
 int pmgpu_cst_set_fast_launch(pmgpu_cst* c, int configs_per_block, int threads_per_block);
 int pmgpu_cst_get_fast_launch(const pmgpu_cst* c, int* configs_per_block, int* threads_per_block);
 /* The fast kernels' other tuning parameters, chosen per workload by the autotuner.  No counterpart
  * in the reference.  sphere_tile: spheres of one configuration per warp row of sphere tasks (0 or a
- * power of two up to 32; at least 32 / configurations-per-block are used; 0: 8);
- * hq_blocks_per_sm: blocks of 256 threads per SM of the hard cloud-query kernel (1..8);
+ * power of two up to 32; at least 32 / configurations-per-block are used; 0, the default, leaves the choice to
+ * the call: 8);
+ * hq_blocks_per_sm: blocks of 256 threads per SM of the hard cloud-query kernel (1..8; default 4);
  * edge_configs_per_block, edge_threads: the edge kernel's waypoints and threads per block, one of
- * (16,128) (32,128) (32,256) (64,256).  Defaults: 0, 4, and an edge shape of the call's choice, which the
- * getter gives as 32, 128. */
+ * (16,128) (32,128) (32,256) (64,256).  (32,128), the default, leaves the choice to the call: (16,128).
+ * Setting what the getters gave restores the state they found. */
 int pmgpu_cst_set_fast_tuning(pmgpu_cst* c, int sphere_tile, int hq_blocks_per_sm, int edge_configs_per_block, int edge_threads);
 int pmgpu_cst_get_fast_tuning(const pmgpu_cst* c, int* sphere_tile, int* hq_blocks_per_sm, int* edge_configs_per_block,
                               int* edge_threads);

@@ -202,8 +202,9 @@ class SphereCollisionCst(IneqConstraintBase):
     def set_fast_tuning(self, sphere_tile: int = 0, hq_blocks_per_sm: int = 4, edge_configs_per_block: int = 32,
                         edge_threads: int = 128) -> None:
         """The fast kernels' other tuning parameters (see plainmp_gb300.autotune): spheres of one
-        configuration per warp row of sphere tasks (0: 8), blocks per SM of the hard
-        cloud-query kernel, and the edge kernel's waypoints and threads per block."""
+        configuration per warp row of sphere tasks (0: the call's choice, 8), blocks per SM of the hard
+        cloud-query kernel, and the edge kernel's waypoints and threads per block (32, 128: the
+        call's choice)."""
         check(lib.pmgpu_cst_set_fast_tuning(self._h, int(sphere_tile), int(hq_blocks_per_sm), int(edge_configs_per_block),
                                              int(edge_threads)))
 

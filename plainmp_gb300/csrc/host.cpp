@@ -686,7 +686,7 @@ struct HostCst {
   int fast_nt = 256;  // threads per block of the fast kernel
   FastTuning tune;    // the fast kernels' other autotuned parameters
   int edge_cpb = 32, edge_nt = 128;  // waypoints and threads per block of the edge kernel
-  bool shape_set = false, tune_set = false;  // set by the caller (the autotuner); else chosen per call
+  bool shape_set = false, edge_set = false;  // set by the caller (the autotuner); else chosen per call
   std::vector<int> slot_of_link;
   std::vector<PmSlot> ctrl_recs;  // per control joint (child link, REV/PRIS) for state updates
   DevBuf d_ctrl_recs;
@@ -1103,7 +1103,7 @@ struct HostCst {
     *nt = edge_nt;
     FastTuning t = tune;
     if (t.sphere_tile_log2 < 0) t.sphere_tile_log2 = 3;
-    if (!tune_set) *cpb = 16;
+    if (!edge_set) *cpb = 16;
     return t;
   }
 
@@ -2024,13 +2024,13 @@ extern "C" {
 int pmgpu_cst_set_fast_launch(pmgpu_cst* c, int configs_per_block, int threads_per_block) {
   return guarded([&] {
     check_ptr(c, "cst");
-    static const int ok[][2] = {{16, 128}, {32, 128}, {16, 256}, {32, 256}, {64, 256}, {32, 512}, {64, 512}, {128, 512}};
+    static const int ok[][2] = {{8, 256}, {16, 128}, {32, 128}, {16, 256}, {32, 256}, {64, 256}, {32, 512}, {64, 512}, {128, 512}};
     bool found = false;
     for (auto& p : ok) found = found || (p[0] == configs_per_block && p[1] == threads_per_block);
     if (!found) throw std::invalid_argument("unsupported (configs_per_block, threads_per_block) pair");
     c->c.fast_cpb = configs_per_block;
     c->c.fast_nt = threads_per_block;
-    c->c.shape_set = true;
+    c->c.shape_set = configs_per_block != 32 || threads_per_block != 256;  // what the getter gives where none is set
   });
 }
 int pmgpu_cst_set_fast_tuning(pmgpu_cst* c, int sphere_tile, int hq_blocks_per_sm, int edge_configs_per_block, int edge_threads) {
@@ -2049,14 +2049,14 @@ int pmgpu_cst_set_fast_tuning(pmgpu_cst* c, int sphere_tile, int hq_blocks_per_s
     c->c.tune.hq_blocks_per_sm = hq_blocks_per_sm;
     c->c.edge_cpb = edge_configs_per_block;
     c->c.edge_nt = edge_threads;
-    c->c.tune_set = true;
+    c->c.edge_set = edge_configs_per_block != 32 || edge_threads != 128;
   });
 }
 int pmgpu_cst_get_fast_tuning(const pmgpu_cst* c, int* sphere_tile, int* hq_blocks_per_sm, int* edge_configs_per_block,
                               int* edge_threads) {
   return guarded([&] {
     check_ptr(c, "cst");
-    if (sphere_tile) *sphere_tile = c->c.tune.sphere_tile_log2 <= 0 ? 0 : (1 << c->c.tune.sphere_tile_log2);
+    if (sphere_tile) *sphere_tile = c->c.tune.sphere_tile_log2 < 0 ? 0 : (1 << c->c.tune.sphere_tile_log2);
     if (hq_blocks_per_sm) *hq_blocks_per_sm = c->c.tune.hq_blocks_per_sm;
     if (edge_configs_per_block) *edge_configs_per_block = c->c.edge_cpb;
     if (edge_threads) *edge_threads = c->c.edge_nt;

@@ -1715,7 +1715,6 @@ cudaError_t launch_fast_edges(const PmTablesHdr* T, const PmTablesHdr& h, const 
     launched = true;                                                                                                     \
   }
   PM_EDGE_CASE(16, 128)
-  PM_EDGE_CASE(32, 128)
   PM_EDGE_CASE(32, 256)
   PM_EDGE_CASE(64, 256)
 #undef PM_EDGE_CASE
