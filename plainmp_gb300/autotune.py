@@ -2,7 +2,8 @@
 
 Dimensions: the fast kernel's launch shape (configurations per block, threads per block) and its
 sphere tile (spheres of one configuration per warp row of sphere tasks), the hard cloud-query
-kernel's blocks per SM (distances only), and the edge kernel's launch shape.  The best values
+kernel's blocks per SM (distances only), and the edge kernel's launch shape; the first candidate of
+each is what a call picks where nothing is set, so tuned is not slower than untuned.  The best values
 depend on the robot (FK slots, spheres, self pairs), the scene (primitives vs a point cloud),
 whether per-sphere distances are requested and the batch size.  ``autotune`` and
 ``autotune_edges`` time the candidates on the caller's batch with CUDA events and keep the
@@ -16,7 +17,8 @@ import os
 from pathlib import Path
 from typing import List, Optional, Tuple
 
-SHAPES = [(16, 128), (32, 128), (16, 256), (32, 256), (64, 256), (32, 512), (64, 512), (128, 512)]
+# (32, 256) and, of the edge kernel, (32, 128) are the defaults: the call's own choice
+SHAPES = [(32, 256), (8, 256), (16, 128), (32, 128), (16, 256), (64, 256), (32, 512), (64, 512), (128, 512)]
 
 
 def cache_path() -> Path:
@@ -26,6 +28,9 @@ def cache_path() -> Path:
     return Path(os.path.expanduser("~")) / ".cache" / "plainmp_gb300" / "autotune.json"
 
 
+KERNELS = 2  # raised whenever choices stored for the kernels of before no longer fit: other shapes, tiles or defaults
+
+
 def signature(cst, batch: int, distances: bool) -> str:
     import torch
 
@@ -33,7 +38,7 @@ def signature(cst, batch: int, distances: bool) -> str:
     sdf = cst.get_sdf()
     scene = type(sdf).__name__ if sdf is not None else "none"
     return (f"{torch.cuda.get_device_name()}|q{cst.q_dim()}|s{cst.n_spheres}|g{cst.n_groups}|sg{int(g['only_self'].sum())}|"
-            f"c{cst.cst_dim()}|{scene}|B{batch}|d{int(distances)}")
+            f"c{cst.cst_dim()}|{scene}|B{batch}|d{int(distances)}|k{KERNELS}")
 
 
 def _load() -> dict:
@@ -53,9 +58,9 @@ def _save(d: dict) -> None:
 
 
 def sphere_tiles(cpb: int) -> List[int]:
-    """The sphere tiles worth trying at a shape: 0 (the least, 32 / cpb) and every larger power of two."""
+    """The sphere tiles worth trying at a shape: the least, 32 / cpb, and every larger power of two."""
     least = max(1, 32 // cpb)
-    return [0] + [t for t in (2, 4, 8, 16, 32) if t > least]
+    return [t for t in (1, 2, 4, 8, 16, 32) if t >= least]
 
 
 def _time(fn, reps: int) -> float:
@@ -92,7 +97,7 @@ def autotune(cst, Q, distances: bool = False, reps: int = 5, use_cache: bool = T
     best, best_ms = None, float("inf")
     for cpb, nt in SHAPES:
         cst.set_fast_launch(cpb, nt)
-        for st in sphere_tiles(cpb):
+        for st in [0] if (cpb, nt) == SHAPES[0] else sphere_tiles(cpb):
             cst.set_fast_tuning(st, 4, ecpb, ent)
             try:
                 ms = _time(lambda: cst.is_valid_fast(Q, distances=distances), reps)
@@ -122,7 +127,7 @@ def autotune(cst, Q, distances: bool = False, reps: int = 5, use_cache: bool = T
     return (cpb, nt), times
 
 
-EDGE_SHAPES = [(16, 128), (32, 128), (32, 256), (64, 256)]
+EDGE_SHAPES = [(32, 128), (16, 128), (32, 256), (64, 256)]
 
 
 def autotune_edges(validator, S1, S2, reps: int = 5, use_cache: bool = True, verbose: bool = False
