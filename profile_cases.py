@@ -3,8 +3,9 @@ configurations against the 200k-point box-surface cloud, validity only (``valid`
 per-sphere distances (``dist``), three launches each; one fused IK descent (8192 problems x 50
 steps, ``ik``); one trajectory cost + gradient (512 trajectories, ``traj``); three fast edge
 pipelines over 1024 chain edges (``edges``); two plain FP64 batches of 8192 dual-arm configurations
-(``plain``).
-python profile_cases.py [valid|dist|ik|traj|edges|plain|all]"""
+(``plain``); two evaluations of 601 planar-base chain configurations against the cloud (``evaluate``);
+two nearest-point batches of 100,000 queries (``nearest``).
+python profile_cases.py [valid|dist|ik|traj|edges|plain|evaluate|nearest|all]"""
 import sys
 from pathlib import Path
 
@@ -58,6 +59,38 @@ def plain(n: int = 8192, launches: int = 2):
     torch.cuda.synchronize()
 
 
+def evaluate(n: int = 601, launches: int = 2):
+    """Constraint values and Jacobians (k_evaluate64) of the planar-base chain against the 200k-point cloud."""
+    import torch
+
+    from plainmp_gb300 import scenes
+    from plainmp_gb300 import workloads as W
+
+    _, cst, _ = scenes.make_constraint(W.planar_chain7_robot(), W.Scene(cloud=W.box_surface_cloud(), cloud_radius=0.0))
+    rng = np.random.default_rng(0)
+    q = rng.uniform(-np.pi, np.pi, size=(n, cst.q_dim()))
+    q[:, 7:9] = rng.uniform(-1.0, 1.0, size=(n, 2))
+    Q = torch.tensor(q, device="cuda")
+    for _ in range(launches):
+        cst.evaluate_batch(Q)
+    torch.cuda.synchronize()
+
+
+def nearest(n: int = 100_000, launches: int = 2):
+    """Exact nearest points (k_cloud_nearest) of queries in a 2.5 m cube around the 200k-point cloud."""
+    import torch
+
+    from plainmp_gb300 import CloudSDF
+    from plainmp_gb300 import workloads as W
+
+    sdf = CloudSDF(W.box_surface_cloud().astype(np.float64), 0.0)
+    pts = np.array([0.6, 0.0, 0.8]) + np.random.default_rng(0).uniform(-1.25, 1.25, size=(n, 3))
+    Q = torch.tensor(pts, device="cuda")
+    for _ in range(launches):
+        sdf.nearest(Q)
+    torch.cuda.synchronize()
+
+
 def ik(steps: int = 50):
     import torch
 
@@ -104,3 +137,7 @@ if __name__ == "__main__":
         edges()
     if which in ("plain", "all"):
         plain()
+    if which in ("evaluate", "all"):
+        evaluate()
+    if which in ("nearest", "all"):
+        nearest()
