@@ -1,8 +1,8 @@
 // OMPL adapter of the C ABI: the state-validity callback and the box motion validator that
 // CollisionAwareSpaceInformation installs (ompl/ompl_thin_wrap.hpp:114-120, 181-182;
 // ompl/motion_validator.hpp:29-34), each call a batch of one through include/pmgpu.h's fast entry
-// points (FP32 with the FP64 recheck: the reference's booleans, at a fraction of the plain FP64
-// method's per-call latency).
+// points (FP32 with the FP64 recheck: the reference's booleans).  Per call they are the faster ones for
+// states and for long edges; pmgpu_check_motion is for edges of up to about 32 waypoints.
 // Header-only: it includes the two OMPL headers it needs and the C ABI's header.
 #pragma once
 #include <stdexcept>

@@ -48,7 +48,6 @@ using SlotF = PmSlotF;
 constexpr int kPoseF = 16;
 __host__ __device__ inline int pose_stride(int n_slots) { return n_slots * kPoseF + 4; }
 
-enum { ST_PASS = 0, ST_FAIL = 1, ST_MAYBE = 2 };
 constexpr int FLAG_FAIL = 1;
 
 // A hard cloud query handed from k_fast_valid to k_hard_queries (distances mode): the sphere centre
@@ -1634,7 +1633,9 @@ cudaError_t launch_fast_valid(const PmTablesHdr* T, const PmTablesHdr& h, const 
   cudaError_t e;
   int n_sm = 0;
   if ((e = sm_count(&n_sm)) != cudaSuccess) return e;
-  // 8 primitives or more and at most 4 blocks of 256 per SM: the latency of one block is the kernel's.  4,096
+  // 8 primitives or more and at most 4 blocks of 256 per SM: the latency of one block is the kernel's.  Calls of 9,000
+  // states at (16, 256) without and with LONE, us: chain x 2 primitives 44.4, 46.7, x 7 48.4, 50.0, x 8 48.2, 48.5, x 20
+  // with distances 60.8, 56.7; dual arm x 4 54.3, 52.5, x 8 41.9, 39.8, x 20 with distances 79.1, 73.1.  4,096
   // chain states against 20 primitives with distances: 34.4 us without LONE, 25.4 with; 200,003 dual-arm states
   // against the cloud: 407 us without, 411 with; against a cloud alone LONE gains nothing at (16, 256).
   const bool lone = h.n_prims >= 8 && (int64_t)grid * nt <= 1024 * (int64_t)n_sm;

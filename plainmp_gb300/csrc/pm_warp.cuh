@@ -79,7 +79,7 @@ __device__ __forceinline__ FieldStart field_corner_candidate(const float4& rec, 
 // final threshold leaves are evaluated together at the end.  One FP64 distance per query then remains,
 // against every box and point of the walk: 100,000 uniform queries in a 2.5 m cube around the 200k-point
 // cloud took 26.1 ms with one thread per query in FP64 (the FP64 pipe 82 % busy with 3.3 of 32 lanes),
-// and take 0.387 ms this way.
+// and take 0.36 ms this way.
 //
 // Where q's fine cell has a cell list, the list is scanned, nearest first, 32 entries at a time.
 // Elsewhere the super-block with the nearest box is searched first, then those within the threshold.

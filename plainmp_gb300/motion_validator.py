@@ -53,7 +53,7 @@ class _ValidatorBase:
         return b1, b2
 
     def check_motion_batch(self, S1, S2, return_count: bool = False):
-        """Plain FP64 method, one device thread per edge: (E,) uint8."""
+        """Plain FP64 method, a block per edge or several edges per block: (E,) uint8."""
         if self._parts is not None:
             raise TypeError("the plain edge method takes a SphereCollisionCst; a composite goes through check_motion_fast")
         b1, b2 = self._edges(S1, S2)
