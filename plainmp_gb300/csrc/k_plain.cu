@@ -995,8 +995,11 @@ cudaError_t launch_check_motion64(const PmTablesHdr* T, const PmTablesHdr& h, co
   if (e != cudaSuccess) return e;
   if (E <= n_sm)
     return team_launch(k_check_motion64<16>, E, 16, 1, h, s, T, state, s1, s2, type, width, resolution, seq, out, n_checked, counts);
-  // more edges a block while 8 blocks per SM (4 rounds of resident ones) are left
+  // more edges a block while 8 blocks per SM (4 rounds of resident ones) are left; below two, the block an edge that
+  // keeps its endpoints in shared memory (1,024 chain edges of 1 to 120 waypoints: 417 us, 432 with the other kernel)
   const int G = (int)std::min<int64_t>(std::max<int64_t>(E / (8 * (int64_t)n_sm), 1), kEdgesPerBlock);
+  if (G == 1)
+    return team_launch(k_check_motion64<8>, E, 8, 1, h, s, T, state, s1, s2, type, width, resolution, seq, out, n_checked, counts);
   return team_launch(k_check_motions64<8>, (E + G - 1) / G, 8, 1, h, s, T, state, s1, s2, E, G, type, width, resolution, seq, out, n_checked,
                      counts);
 }
