@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(NC * 32, 512 / (NC * 32)) k_check_motion64(con
   }
 }
 
-// The same for more edges than SMs, G (up to 64) edges a block: the waypoints of its edges in a row, NC at a time,
+// The same for 16 edges per SM and more, G (2 to 64) edges a block: the waypoints of its edges in a row, NC at a time,
 // leaving out those of an edge that has collided.  A block an edge, as above, has NC - 1 warps idle where edges are
 // of one waypoint, and starts a block for each edge without length: 100,000 chain edges of one waypoint took 7.4 ms,
 // 1.41 this way; of no length 1.01 ms, 0.10; 20,000 of three 1.66 ms, 0.84; 1,000 of twenty 0.24 ms either way.
