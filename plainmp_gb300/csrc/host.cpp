@@ -181,11 +181,17 @@ constexpr int64_t kZeroCopy = 64;
 // 16,384 nothing.)
 constexpr int64_t kZeroCopyFast = 2048;
 
-// |v|^2 above 1 by more than rounding (a quaternion or axis that is none of a rotation), or not finite
-static bool above_unit(const double* v, int n) {
+// |v|^2 - 1 of a quaternion or axis that is longer than a rotation's (infinite where it is not finite), else 0.
+static double excess_of(const double* v, int n) {
   double s = 0.0;
   for (int k = 0; k < n; k++) s += v[k] * v[k];
-  return !(s <= 1.0 + 1e-7);
+  return s <= 1.0 ? 0.0 : (s < 1e300 ? s - 1.0 : std::numeric_limits<double>::infinity());
+}
+// The base pose's, with what rounding to FP32 leaves counted as none (a group of 1 m then loses a sphere by 0.6 um at
+// most, and every margin is 1 um and more).
+static double base_excess(const double* base7) {
+  const double e = excess_of(base7 + 3, 4);
+  return e <= 3e-7 ? 0.0 : e;
 }
 
 // ---------------------------------------------------------------------------- host quaternion
@@ -221,7 +227,7 @@ struct HostModel {
   std::vector<double> state_init;  // rows of PM_STATE_STRIDE doubles (row 0 = base)
   std::vector<double> angles;
   double base7[7] = {0, 0, 0, 0, 0, 0, 1};
-  uint64_t version = 1;  // bumped when the link set changes, or the base pose leaves or regains unit norm
+  uint64_t version = 1;  // bumped when the link set changes, or how far the base pose is off unit norm
   // device
   DevBuf d_state;
   DevBuf d_parents;
@@ -781,20 +787,22 @@ struct HostCst {
     }
   }
 
-  // Whether a rotation of the constraint's links may be off unit norm: URDF axes, fixed transforms and base poses are
-  // taken as they are given.  The fast kernels' error bounds, and that a colliding sphere lies in its group's sphere,
-  // hold for rotations (to 1e-3 and more), so such a constraint's configurations and edges are all decided by the
-  // exact check of the recheck kernel, as those whose terms overflow the queue, and its groups are never culled (FP32
-  // radius kNoCull), which leaves the fast kernels the distances.
+  // How far |q|^2 of the constraint's links may exceed 1: URDF axes, fixed transforms and base poses are taken as they
+  // are given.  The fast kernels' error bounds, and that a colliding sphere lies in its group's sphere, hold for
+  // rotations.  Up to kExcess (axes of four digits) the bounds have room, and every link's error is raised by what the
+  // stretch moves a sphere out of its group (the root's slack in the image).  Above it (off_unit) all configurations
+  // and edges are decided by the exact check of the recheck kernel, as those whose terms overflow the queue, and groups
+  // are never culled (FP32 radius kNoCull), which leaves the fast kernels the distances.
+  static constexpr double kExcess = 1e-3;
   static constexpr float kNoCull = 1e6f;
-  bool off_unit() const {
+  double unit_excess() const {
     const HostModel& m = *kin;
-    if (base_type == PM_BASE_FIXED && above_unit(m.base7 + 3, 4)) return true;
+    double x = base_type == PM_BASE_FIXED ? base_excess(m.base7) : 0.0;
     for (const HostJoint& j : m.joints)
-      if (slot_of_link[j.child] >= 0 && j.type != UJ_PRISMATIC && above_unit(j.axis, 3)) return true;
+      if (slot_of_link[j.child] >= 0 && j.type != UJ_PRISMATIC) x += excess_of(j.axis, 3);
     for (int l = 0; l < m.n_link(); l++)
-      if (slot_of_link[l] >= 0 && above_unit(&m.state_init[(size_t)PM_STATE_LINK_ROW(l) * PM_STATE_STRIDE], 4)) return true;
-    return false;
+      if (slot_of_link[l] >= 0) x += excess_of(&m.state_init[(size_t)PM_STATE_LINK_ROW(l) * PM_STATE_STRIDE], 4);
+    return x < 1e-9 ? 0.0 : x;
   }
 
   // The FP32 image of the tables: the records of the fast kernels as a block keeps them.  Slots
@@ -802,7 +810,7 @@ struct HostCst {
   static std::vector<char> fast_image(const std::vector<PmSlot>& slots, const std::vector<PmGroup>& groups, const std::vector<double>& sx,
                                       const std::vector<double>& sy, const std::vector<double>& sz, const std::vector<double>& sr,
                                       const std::vector<int32_t>& sgroup, const std::vector<int32_t>& pairs,
-                                      const std::vector<PmPrim>& prims, bool off_unit) {
+                                      const std::vector<PmPrim>& prims, bool off_unit, float stretch) {
     std::vector<char> img;
     auto add = [&](const void* p, size_t bytes) {
       const size_t off = img.size();
@@ -865,7 +873,9 @@ struct HostCst {
       tail[l * PM_MAX_SLOTS + n[l]++] = (char)i;
     }
     std::memcpy(tail + 3 * PM_MAX_SLOTS, n, sizeof(n));
-    const float base8[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    float reach = 0.0f;
+    for (auto& G : groups) reach = std::max(reach, (float)G.radius);
+    const float base8[8] = {0, 0, 0, 0, 0, 0, 0, stretch * reach};
     add(sl.data(), sl.size() * sizeof(PmSlotF));
     add(base8, sizeof(base8));
     add(sp.data(), sp.size() * sizeof(PmSphereF));
@@ -982,7 +992,9 @@ struct HostCst {
     h.q_dim = q_dim();
     h.base_type = base_type;
     h.root_slot = slot_of_link[m.root];
-    h.off_unit = off_unit();
+    const double x = unit_excess();
+    h.off_unit = !(x <= kExcess);
+    h.stretch = (float)(2.1 * std::min(x, 1.2 * kExcess));  // |R| <= 1 + 2 (|q|^2 - 1)
     h.n_clouds = (int)clouds.size();
     std::vector<char> buf;
     auto align = [&]() {
@@ -1022,7 +1034,7 @@ struct HostCst {
     lev.insert(lev.end(), by_depth.begin(), by_depth.end());
     h.n_levels = n_levels;
     h.off_lev = put(lev.data(), lev.size() * 4);
-    const std::vector<char> img = fast_image(slots, grec, sx, sy, sz, sr, sgroup, prs, prims, h.off_unit != 0);
+    const std::vector<char> img = fast_image(slots, grec, sx, sy, sz, sr, sgroup, prs, prims, h.off_unit != 0, h.stretch);
     h.img_bytes = (int64_t)img.size();
     h.off_img = put(img.data(), img.size());
     align();
@@ -1407,7 +1419,7 @@ int pmgpu_model_set_base_pose(pmgpu_model* m, const double* pose7) {
   return guarded([&] {
     check_ptr(m, "model");
     HostModel& M = *m->m;
-    if (above_unit(M.base7 + 3, 4) != above_unit(pose7 + 3, 4)) M.version++;  // the constraints' tables depend on it
+    if (base_excess(M.base7) != base_excess(pose7)) M.version++;  // the constraints' tables depend on it
     std::memcpy(M.base7, pose7, sizeof(M.base7));
     const double q[4] = {pose7[3], pose7[4], pose7[5], pose7[6]}, t[3] = {pose7[0], pose7[1], pose7[2]};
     set_row(M.state_init, PM_STATE_BASE_ROW, q, t, false);

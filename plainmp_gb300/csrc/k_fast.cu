@@ -121,7 +121,8 @@ __device__ __forceinline__ void approx_sin_cos32_q(double q, float qf, float& s,
 //     <= 6.4 |v| at |q| <= 1.001; the matrix's and the product's rounding, or fqrot's: two crosses of fused
 //     sums, 7u |v| in the first times 1.42, 6u and 2u in the second and the sums, 18u in all);
 //   translation t = tp + R lt: |dt| <= |dtp| + (8 |dqp| + 24u)|lt| + 1.01 u (|tp|_1 + |lt|_1).
-// The base pose adds the rounding of q's base entries (and of their half angles).
+// The base pose adds the rounding of q's base entries (and of their half angles), and the image's slack for rotations
+// off unit norm (0 for none).
 //
 // The local transform of a slot into o: [0..3] quaternion, [4..6] translation, [7] identity flag, [8] the
 // quaternion's error, [9] the translation's, [10] |t|_1, [11] |t| rounded up; a root's world pose as fk_chain
@@ -156,7 +157,7 @@ __device__ __forceinline__ void fk_local(const SlotF& s, const float* __restrict
       eq = 2.0f * kU;
     }
     o[0] = make_float4(wq.x, wq.y, wq.z, wq.w);
-    o[1] = make_float4(wt[0], wt[1], wt[2], kU * (fabsf(wt[0]) + fabsf(wt[1]) + fabsf(wt[2])));
+    o[1] = make_float4(wt[0], wt[1], wt[2], kU * (fabsf(wt[0]) + fabsf(wt[1]) + fabsf(wt[2])) + base8[7]);
     o[2].x = eq;
     return;
   }
@@ -614,7 +615,7 @@ struct Smem {
   int* sdist;    // per (cfg, sphere): running minimum signed distance, order-preserving int
   float* pose;   // [cfg][pose_stride]: [slot][kPoseF]
   SlotF* slot;
-  float* base8;  // fixed base pose: q xyzw, t xyz
+  float* base8;  // fixed base pose: q xyzw, t xyz; the image's slack
   SphereF* sph;
   GroupF* grp;
   PrimF* prm;
@@ -1208,7 +1209,7 @@ __device__ void stage_tables(const TView& v, const Smem& sm, const double* __res
     f.lid = signbit(row[7]);
     f.lt1 = fabsf(row[7]);
   } else if (mine == -1) {
-    for (int k = 0; k < 8; k++) sm.base8[k] = k < 7 ? row[k] : 0.0f;
+    for (int k = 0; k < 7; k++) sm.base8[k] = row[k];
   }
   __syncthreads();
 }

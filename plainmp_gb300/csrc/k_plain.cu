@@ -498,6 +498,7 @@ __device__ double eval_ext_warp(const TView& v, const Image& im, const TeamPose&
   const PmTablesHdr* T = v.T;
   const int lane = threadIdx.x & 31;
   const int ng = T->n_groups, np = T->n_prims, dof = T->q_dim;
+  const float stretch = T->stretch;
   Least best{PM_CUTOFF, kNoTerm};
   float upper = (float)PM_CUTOFF;  // no term above it can be the least
   for (int pass = 0; pass < 2; pass++) {  // 0: the bound; 1: the values
@@ -523,7 +524,7 @@ __device__ double eval_ext_warp(const TView& v, const Image& im, const TeamPose&
           // beyond the bound none of them is the least.  The ground's gate tests more than the distance
           // (g), and only the cutoff counts for it.  (g of a box or cylinder ends at -radius inside it.)
           const bool by_gate = Q.kind == PM_SDF_GROUND;
-          if (!((by_gate ? g : sd) > (by_gate ? (float)PM_CUTOFF : upper) + margin32(mag) + cast_error(R, G.gn) + kStretch * G.radius)) n = G.count;
+          if (!((by_gate ? g : sd) > (by_gate ? (float)PM_CUTOFF : upper) + margin32(mag) + cast_error(R, G.gn) + stretch * G.radius)) n = G.count;
         }
       }
       warp_spread(n, [&](int owner, int j, bool have) {
@@ -537,7 +538,7 @@ __device__ double eval_ext_warp(const TView& v, const Image& im, const TeamPose&
           const PmSphereF& S = im.sph[k];
           const float* R = P.at32(G.slot);
           const float3 c = xf(R, S.x, S.y, S.z);
-          const float ek = cast_error(R, S.sn) + kStretch * im.grp[g2].radius;
+          const float ek = cast_error(R, S.sn) + stretch * im.grp[g2].radius;
           if (Q.kind == PM_SDF_CLOUD) {
             const PmGridDev& Gd = v.C[Q.cloud];
             const float qmag = fabsf(c.x) + fabsf(c.y) + fabsf(c.z);
@@ -586,7 +587,7 @@ __device__ double eval_ext_warp(const TView& v, const Image& im, const TeamPose&
           if (nn.idx < 0) continue;
           const double val = sqrt(nn.d2) - Qs.a - rs;
           // below the cutoff the gate is open, but for rounding at the cutoff itself
-          if ((scales || val > PM_CUTOFF - 1e-7 - kStretch * rg) && cloud_outside_warp(Qs, v.C, gcs, rg + PM_CUTOFF, nullptr)) continue;
+          if ((scales || val > PM_CUTOFF - 1e-6 - stretch * rg) && cloud_outside_warp(Qs, v.C, gcs, rg + PM_CUTOFF, nullptr)) continue;
           if (val < PM_CUTOFF) best.take(val, os);  // the same on every lane
           upper = fminf(upper, (float)val + 1e-6f * (1.0f + fabsf((float)val)));
         }
@@ -633,6 +634,7 @@ __device__ double eval_self_warp(const TView& v, const Image& im, const TeamPose
   const PmTablesHdr* T = v.T;
   const int lane = threadIdx.x & 31;
   const int dof = T->q_dim;
+  const float stretch = T->stretch;
   Least best{PM_CUTOFF, kNoTerm};
   float upper = (float)PM_CUTOFF;
   for (int pass = 0; pass < 2; pass++) {
@@ -649,7 +651,7 @@ __device__ double eval_self_warp(const TView& v, const Image& im, const TeamPose
         const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
         const float mag = fabsf(a.x) + fabsf(a.y) + fabsf(a.z) + fabsf(b.x) + fabsf(b.y) + fabsf(b.z);
         near = !(sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) - (G1.radius + G2.radius) >
-                 upper + 2.0f * margin32(mag) + cast_error(R1, G1.gn) + cast_error(R2, G2.gn) + kStretch * (G1.radius + G2.radius));
+                 upper + 2.0f * margin32(mag) + cast_error(R1, G1.gn) + cast_error(R2, G2.gn) + stretch * (G1.radius + G2.radius));
       }
       for (unsigned bal = __ballot_sync(FULL, near); bal != 0; bal &= bal - 1) {  // warp-uniform
         const int src = __ffs(bal) - 1;
@@ -664,7 +666,7 @@ __device__ double eval_self_warp(const TView& v, const Image& im, const TeamPose
           const float ex = ci.x - cj.x, ey = ci.y - cj.y, ez = ci.z - cj.z;
           const float mag = fabsf(ci.x) + fabsf(ci.y) + fabsf(ci.z) + fabsf(cj.x) + fabsf(cj.y) + fabsf(cj.z);
           const float d32 = sqrtf(fmaf(ex, ex, fmaf(ey, ey, ez * ez))) - (S1.r + S2.r);
-          const float m = 2.0f * margin32(mag) + cast_error(R1, S1.sn) + cast_error(R2, S2.sn) + kStretch * (im.grp[a].radius + im.grp[b].radius);
+          const float m = 2.0f * margin32(mag) + cast_error(R1, S1.sn) + cast_error(R2, S2.sn) + stretch * (im.grp[a].radius + im.grp[b].radius);
           if (pass == 0) {
             upper = fminf(upper, d32 + m);
             continue;

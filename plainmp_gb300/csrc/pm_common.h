@@ -185,7 +185,8 @@ struct PmTablesHdr {
   int32_t n_slots, n_ctrl, n_groups, n_spheres;
   int32_t n_pairs, n_prims, q_dim, base_type;
   int32_t root_slot, n_clouds, n_levels;
-  int32_t off_unit;  // some rotation of the slots may be off unit norm (HostCst::off_unit)
+  int32_t off_unit;  // rotations of the slots are off unit norm by more than the FP32 bounds allow (HostCst::unit_excess)
+  float stretch;     // a slot's R scales by at most 1 + this (off_unit: where its |q|^2 is below kNorm2Eval)
   int64_t off_slots, off_joints, off_groups, off_sx, off_sy, off_sz, off_sr, off_sgroup, off_pairs, off_prims, off_clouds;
   int64_t off_img, img_bytes;  // the FP32 image
   int64_t off_lev;  // slots by depth: the n_levels + 1 starts, then slot | parent << 16 (int32)

@@ -145,10 +145,9 @@ __device__ void fk64_levels(const TView& v, const double* __restrict__ state, co
 // 1 + 2 (|q|^2 - 1), or shrinks where |q| < 1.  Where |q|^2 exceeds `norm2` the FP32 translation is NaN, so that every
 // FP32 comparison of the slot's spheres fails and FP64 decides.
 // Validity needs the bounds alone, which have 1 % to spare (the Taylor form is within 1e-5 of unit norm a joint);
-// evaluate also that the spheres leave the group's sphere by no more than kStretch of its radius.
+// evaluate also that the spheres leave the group's sphere by no more than the tables' stretch of its radius.
 constexpr float kNorm2Valid = 1.01f;
-constexpr float kNorm2Eval = 1.000001f;
-constexpr float kStretch = 3e-6f;
+constexpr float kNorm2Eval = 1.0011f;
 template <int NT, class QF>
 __device__ void fk64_block(const TView& v, const double* __restrict__ state, const QF& qf, int ncfg, bool taylor, float norm2, double* rec,
                            float* p32) {

@@ -26,7 +26,7 @@ def _robot(scale, base="FIXED"):
     return W.Robot(re.sub(r'<axis xyz="([^"]*)"/>', axis, r.urdf), r.control_joints, r.end_link, r.spheres, r.self_pairs, base_type=base)
 
 
-CASES = [("axes", 3.0), ("axes", 1.05), ("axes", 1.0 + 2e-5), ("base", 1.7), ("base", 1.0 + 1e-4), ("base", 0.4)]
+CASES = [("axes", 3.0), ("axes", 1.05), ("axes", 1.0001), ("axes", 1.0 + 2e-5), ("base", 1.7), ("base", 1.0 + 1e-4), ("base", 0.4)]
 
 
 @pytest.fixture(scope="module", params=CASES, ids=lambda c: f"{c[0]}-{c[1]:g}")
@@ -99,3 +99,11 @@ def test_fast_distances(pair):
     _, d = cst.is_valid_fast(Q, distances=True)
     ref = np.minimum(oc.sphere_distances(Q, threads=8), 0.1)
     assert np.abs(d.astype(np.float64) - ref).max() < (1e-6 + 64 * 2.0 ** -24 * 21) * n2
+
+
+def test_rounded_axes_keep_the_fast_path(pair):
+    """Up to 1e-3 of excess in all, as axes of four digits have, the bounds are widened; above it everything is checked
+    exactly."""
+    cst, oc, n2 = pair
+    _, st = cst.is_valid_fast(W.chain7_configs(3000, seed=39), stats=True)
+    assert st["rechecked_configs"] == (0 if n2 < 1.001 else 3000)
